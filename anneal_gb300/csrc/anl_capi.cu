@@ -242,7 +242,7 @@ static void free_ctx(anl_ctx* c) {
     f(c->oc_gw);
     f(c->oc_state);
     f(c->ainv_lo);
-    f(c->flag_d);
+    f(c->coarse_dmax);
     f(c->restart_d);
     f(c->p);
     f(c->q);
@@ -373,7 +373,7 @@ static int create(anl_ctx** out, int nx, int ny, int nz, double h, double nu, in
             ALLOC(c->ainv_lo, (size_t)c->nc * c->nc * sizeof(float));
         }
     }
-    ALLOC(c->flag_d, 4 * sizeof(int));
+    ALLOC(c->coarse_dmax, sizeof(double));
     ALLOC(c->restart_d, R * sizeof(int));
     ALLOC(c->cheb_d, c->lev.size() * kChebStride * sizeof(double));
     ALLOC(c->ke_d, 576 * sizeof(double));
@@ -461,8 +461,7 @@ static int create(anl_ctx** out, int nx, int ny, int nz, double h, double nu, in
     }
     if (cudaMemset(c->counter, 0, (16 + R) * sizeof(unsigned)) != cudaSuccess ||
         cudaMemset(c->restart_d, 0, R * sizeof(int)) != cudaSuccess ||
-        upload_cheb(c) != cudaSuccess ||
-        cudaMemset(c->flag_d, 0, 4 * sizeof(int)) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+        upload_cheb(c) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
         set_error("context initialisation failed: %s", cudaGetErrorString(cudaGetLastError()));
         free_ctx(c);
         return ANL_ERR_CUDA;

@@ -123,13 +123,13 @@ struct anl_ctx {
     // smoothing kernels from device memory
     double* cheb_d = nullptr;
 
-    // coarsest level: dense factor (FP64) or a Chebyshev fallback when too large
+    // coarsest level: dense inverse or a Chebyshev fallback when too large
     int nc = 0;
     bool dense_coarse = false;
     bool coarse_ready = false;
-    double* A = nullptr;     // nc x nc, lower Cholesky factor after setup
+    double* A = nullptr;     // nc x nc, scratch of the inversion
     double* Ainv = nullptr;  // nc x nc inverse
-    int* flag_d = nullptr;
+    double* coarse_dmax = nullptr;  // largest diagonal entry of the coarsest matrix
 
     // CG vectors (precision T) and FP64 solution / right-hand side
     void* p = nullptr;

@@ -173,7 +173,6 @@ struct TailArgs {
 size_t tail_smem_bytes(const TailLevel* lev, int nlev);
 int vtail_prepare();
 int launch_vtail(const TailArgs& a, cudaStream_t s);
-int launch_ainv_split(const double* ainv, int n, float* hi, float* lo, cudaStream_t s);
 
 // ------------------------------------------------------------------ tensor-core K u (fine grid)
 

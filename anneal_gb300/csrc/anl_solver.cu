@@ -1551,9 +1551,11 @@ static int pcg_one(anl_ctx* c, const double* f, double* x, double rtol, int maxi
             status = ANL_ERR_MAXITER;
             break;
         }
-        // not converged: the replaced residual carries on; restart the directions after a
-        // breakdown
-        if (h.done == 4) {
+        // not converged: the replaced residual carries on. The directions restart after a
+        // breakdown and after a failed certification: there the recurrence residual had become far
+        // smaller than the true one, so the replaced residual is not orthogonal to the last
+        // direction and beta, scaled by the old r.z, would be noise (a 3 x 3 x 1 solve diverged)
+        if (h.done == 1 || h.done == 4) {
             const int one_r = 1;
             ANL_CUDA(cudaMemcpyAsync(restart, &one_r, sizeof(int), cudaMemcpyHostToDevice, s));
         }
@@ -1754,7 +1756,8 @@ static int pcg_batch(anl_ctx* c, int R, const double* f, double* x, double rtol,
                 ANL_TRY(finish(r, ANL_ERR_MAXITER));
                 continue;
             }
-            if (h.done == 4) ANL_CUDA(cudaMemcpyAsync(c->restart_d + r, &one, sizeof(int), cudaMemcpyHostToDevice, s));
+            if (h.done == 1 || h.done == 4)  // as in pcg_one
+                ANL_CUDA(cudaMemcpyAsync(c->restart_d + r, &one, sizeof(int), cudaMemcpyHostToDevice, s));
         }
     }
     ANL_CUDA(cudaMemcpyAsync(c->sc_h, c->sc_base, R * sizeof(PcgScalars), cudaMemcpyDeviceToHost, s));

@@ -421,15 +421,6 @@ __global__ void __launch_bounds__(TT, 1) k_vtail(TailArgs a) {
     for (int q = tid; q < 3 * nn; q += TT) x0[q] = t.X(0)[q];
 }
 
-__global__ void k_ainv_split(const double* ainv, int64_t n2, float* hi, float* lo) {
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n2; q += (int64_t)gridDim.x * blockDim.x) {
-        float h, l;
-        split_double(ainv[q], h, l);
-        hi[q] = h;
-        lo[q] = l;
-    }
-}
-
 }  // namespace
 
 size_t tail_smem_bytes(const TailLevel* lev, int nlev) { return sizeof(float) * (size_t)tail_layout(lev, nlev).words; }
@@ -452,13 +443,6 @@ int launch_vtail(const TailArgs& a, cudaStream_t s) {
         return ANL_ERR_BADARG;
     }
     k_vtail<<<std::max(1, a.nrhs), TT, bytes, s>>>(a);
-    ANL_LAUNCH_CHECK();
-    return ANL_OK;
-}
-
-int launch_ainv_split(const double* ainv, int n, float* hi, float* lo, cudaStream_t s) {
-    const int64_t n2 = (int64_t)n * n;
-    k_ainv_split<<<(int)std::min<int64_t>(1024, (n2 + 255) / 256), 256, 0, s>>>(ainv, n2, hi, lo);
     ANL_LAUNCH_CHECK();
     return ANL_OK;
 }
