@@ -8,8 +8,8 @@
 //    trilinear prolongation P and restriction P^T, Chebyshev smoothing on D^-1 K below the
 //    element bound lambda_max(Ke) / Ke_00 (an upper bound of the spectrum for every design):
 //    2 steps over [0.03, 1] x bound on levels 0-1, 8 steps over [0.002, 1] x bound on the
-//    latency-bound levels below; a dense FP64 Cholesky solve on the coarsest grid, refactored
-//    every solve (a high-degree Chebyshev sweep if that grid is too large for a dense factor);
+//    latency-bound levels below; a dense inverse on the coarsest grid, formed
+//    anew every solve (a high-degree Chebyshev sweep if that grid is too large for a dense factor);
 //  * the CG iterate x and right-hand side stay in FP64; the CG scalars come from FP64
 //    reductions (compensated FP32 partials); the residual is replaced by the true residual
 //    b - K x of the FP64 operator (in double-float arithmetic) periodically and before
@@ -389,11 +389,14 @@ __global__ void k_cheb_first(int64_t nn, const T* b, const float* dinv, const ui
     }
 }
 
-// ------------------------------------------------------------------ coarsest grid (FP64)
+// ------------------------------------------------------------------ coarsest grid
 
 // Dense K of the coarsest level, one thread per entry (deterministic: each entry sums
-// the elements shared by its two nodes in a fixed order). Non-free rows/cols -> identity.
-__global__ void k_assemble_dense(Dims d, const float* E, const uint8_t* nmask, const double* ke, int n, double* A) {
+// the elements shared by its two nodes in a fixed order, in FP64). Non-free rows/cols -> identity.
+// *dmax (zeroed) receives the largest diagonal entry: positive doubles order like their bits.
+template <class T>
+__global__ void k_assemble_dense(Dims d, const float* E, const uint8_t* nmask, const double* ke, int n, T* A,
+                                 unsigned long long* dmax) {
     const int64_t total = (int64_t)n * n;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int row = (int)(t / n), col = (int)(t % n);
@@ -401,7 +404,8 @@ __global__ void k_assemble_dense(Dims d, const float* E, const uint8_t* nmask, c
         const int ci = row % 3, cj = col % 3;
         const bool fr = (nmask[N] >> ci) & 1, fc = (nmask[M] >> cj) & 1;
         if (!fr || !fc) {
-            A[t] = row == col ? 1.0 : 0.0;
+            A[t] = T(row == col ? 1 : 0);
+            if (row == col) atomicMax(dmax, (unsigned long long)__double_as_longlong(1.0));
             continue;
         }
         const int Ni = (int)(N % (d.nx + 1)), Nj = (int)((N / (d.nx + 1)) % (d.ny + 1)),
@@ -422,228 +426,123 @@ __global__ void k_assemble_dense(Dims d, const float* E, const uint8_t* nmask, c
                 s += (double)E[d.elem(ei, ej, ek)] * ke[(3 * la + ci) * 24 + 3 * lb + cj];
             }
         }
-        A[t] = s;
+        A[t] = T(s);
+        if (row == col && s > 0.0) atomicMax(dmax, (unsigned long long)__double_as_longlong(s));
     }
 }
 
-// In-place lower Cholesky factor of the n x n SPD matrix A (one CTA, right-looking).
-__global__ void __launch_bounds__(1024) k_cholesky(double* A, int n, int* flag) {
-    __shared__ double piv, dmax;
-    if (threadIdx.x == 0) {
-        double m = 0.0;
-        for (int j = 0; j < n; ++j) m = fmax(m, A[(int64_t)j * n + j]);
-        dmax = m;
-    }
-    __syncthreads();
-    for (int j = 0; j < n; ++j) {
-        if (threadIdx.x == 0) {
-            const double a = A[(int64_t)j * n + j];
-            // A pivot this small relative to the largest diagonal comes from near-void coarse
-            // elements (E_min 1e-9 of a design) or from a floating piece. The factor only
-            // preconditions, so it is regularised to stay positive definite; a part that
-            // cannot carry its load shows up as a CG that does not converge.
-            if (!(a > 1e-12 * dmax)) {
-                *flag += 1;
-                piv = sqrt(1e-12 * dmax);
-            } else {
-                piv = sqrt(a);
-            }
-            A[(int64_t)j * n + j] = piv;
-        }
-        __syncthreads();
-        const double p = piv;
-        for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) A[(int64_t)i * n + j] /= p;
-        __syncthreads();
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-        for (int gi = j + 1 + warp; gi < n; gi += nw) {
-            const double lij = A[(int64_t)gi * n + j];
-            for (int gk = j + 1 + lane; gk <= gi; gk += 32) A[(int64_t)gi * n + gk] -= lij * A[(int64_t)gk * n + j];
-        }
-        __syncthreads();
-    }
+// A^-1 of the dense n x n coarsest-grid matrix by block Gauss-Jordan elimination without
+// pivoting (the matrix is positive definite), one launch per block column of GJ_B. Step k, with
+// K the k-th block: P = A_KK^-1; A_ij -= A_iK P A_Kj; A_Kj = P A_Kj; A_iK = -A_iK P; A_KK = P.
+// After the last step the array holds the inverse. Every CTA of a step owns one GJ_T x GJ_T tile
+// of the result, reads the previous step's array and writes the other one, so no CTA waits on
+// another; each forms P and its strip of P A_Kj itself.
+//
+// A step does n^2 GJ_B multiply-adds on all SMs and is bound by the chain of its CTAs (the GJ_B
+// pivots of P, one barrier each, then the two products), a few microseconds, so an inversion
+// costs about n / 16 of these. It replaces a factor on one SM: a global-memory FP64 Cholesky
+// above 160 DOFs (4.7 ms + 1.3 ms for the inverse at 336 DOFs, a third of a SIMP step on grids
+// whose coarsest level has 161-400) and shared-memory factors below (193 + 61 us in float pairs,
+// 331 + 85 us in FP64, at 135).
+//
+// Pivots (Schur complements' diagonal entries, as in a Cholesky factor) of at most 1e-12 of the
+// largest diagonal entry come from near-void coarse elements (E_min 1e-9 of a design) or from a
+// floating piece. The inverse only preconditions, so they are set to that bound, which keeps it
+// positive definite; a part that cannot carry its load shows up as a CG that does not converge.
+constexpr int GJ_B = 16, GJ_T = 32, GJ_NT = 256;
+
+__device__ __forceinline__ double gj_recip(double a) {
+    // the FP32 reciprocal refined by two Newton steps (each doubles the correct bits): a chain of
+    // four FP64 operations, where a division is several times longer on this part's FP64 pipe
+    const float r0 = 1.f / (float)a;
+    if (!(r0 > 0.f && r0 < INFINITY)) return 1.0 / a;
+    double r = r0;
+    r = fma(r, fma(-a, r, 1.0), r);
+    return fma(r, fma(-a, r, 1.0), r);
 }
+__device__ __forceinline__ DF gj_recip(DF a) { return df_recip(a); }
+__device__ __forceinline__ double gj_lead(double a) { return a; }
+__device__ __forceinline__ float gj_lead(DF a) { return a.hi; }
+__device__ __forceinline__ double gj_value(double a) { return a; }
+__device__ __forceinline__ double gj_value(DF a) { return a.value(); }
 
-// Column c of A^-1 from the Cholesky factor L (lower triangle of A): one CTA per column.
-__global__ void __launch_bounds__(128) k_chol_inverse(const double* L, double* Ainv, int n) {
-    extern __shared__ double xs[];
-    const int c = blockIdx.x;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) xs[i] = i == c ? 1.0 : 0.0;
-    __syncthreads();
-    for (int j = 0; j < n; ++j) {  // L y = e_c
-        const double yj = xs[j] / L[(int64_t)j * n + j];
-        __syncthreads();
-        if (threadIdx.x == 0) xs[j] = yj;
-        for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) xs[i] -= L[(int64_t)i * n + j] * yj;
-        __syncthreads();
-    }
-    for (int j = n - 1; j >= 0; --j) {  // L^T x = y
-        const double xj = xs[j] / L[(int64_t)j * n + j];
-        __syncthreads();
-        if (threadIdx.x == 0) xs[j] = xj;
-        for (int i = threadIdx.x; i < j; i += blockDim.x) xs[i] -= L[(int64_t)j * n + i] * xj;
-        __syncthreads();
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) Ainv[(int64_t)i * n + c] = xs[i];
-}
-
-// The same factorisation and inverse with the matrix in shared memory, for n <= kCholSmemN
-// (n^2 doubles within the 227 KB a CTA may hold): no global round trip per column step, and
-// the inverse multiplies by precomputed reciprocal pivots.
-constexpr int kCholSmemN = 160;
-
-__global__ void __launch_bounds__(1024) k_cholesky_smem(double* A, int n, int* flag) {
-    extern __shared__ double S[];
-    __shared__ double piv, dmax;
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) S[t] = A[t];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double m = 0.0;
-        for (int j = 0; j < n; ++j) m = fmax(m, S[j * n + j]);
-        dmax = m;
-    }
-    __syncthreads();
-    for (int j = 0; j < n; ++j) {
-        if (threadIdx.x == 0) {
-            const double a = S[j * n + j];
-            // tiny pivots are regularised as in k_cholesky
-            if (!(a > 1e-12 * dmax)) {
-                *flag += 1;
-                piv = sqrt(1e-12 * dmax);
-            } else {
-                piv = sqrt(a);
-            }
-            S[j * n + j] = piv;
-        }
-        __syncthreads();
-        const double rp = 1.0 / piv;
-        for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) S[i * n + j] *= rp;
-        __syncthreads();
-        // trailing update of the lower triangle: one thread per (i, k), k <= i
-        const int m = n - j - 1;
-        for (int t = threadIdx.x; t < m * m; t += blockDim.x) {
-            const int i = j + 1 + t / m, k = j + 1 + t % m;
-            if (k <= i) S[i * n + k] -= S[i * n + j] * S[k * n + j];
-        }
-        __syncthreads();
-    }
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) A[t] = S[t];
-}
-
-__global__ void __launch_bounds__(256) k_chol_inverse_smem(const double* L, double* Ainv, int n) {
-    extern __shared__ double S[];  // L (n * n), reciprocal pivots (n), the column (n)
-    double* rd = S + n * n;
-    double* xs = rd + n;
-    const int c = blockIdx.x;
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) S[t] = L[t];
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        rd[i] = 1.0 / S[i * n + i];
-        xs[i] = i == c ? 1.0 : 0.0;
-    }
-    __syncthreads();
-    for (int j = c; j < n; ++j) {  // L y = e_c (y_j = 0 for j < c)
-        const double yj = xs[j] * rd[j];
-        for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) xs[i] -= S[i * n + j] * yj;
-        __syncthreads();
-        if (threadIdx.x == 0) xs[j] = yj;
-        __syncthreads();
-    }
-    for (int j = n - 1; j >= 0; --j) {  // L^T x = y
-        const double xj = xs[j] * rd[j];
-        for (int i = threadIdx.x; i < j; i += blockDim.x) xs[i] -= S[j * n + i] * xj;
-        __syncthreads();
-        if (threadIdx.x == 0) xs[j] = xj;
-        __syncthreads();
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) Ainv[(int64_t)i * n + c] = xs[i];
-}
-
-// The FP32 solver's coarsest grid in double-float arithmetic (about 48 bits, on the FP32 pipes:
-// FP64 arithmetic on this part runs at a small fraction of FP32, and the factor's trailing
-// updates are ~n^3/6 multiply-adds on one SM): A = L D L^T, no square roots. The matrix comes in
-// as FP64 and is split into float pairs without FP64 arithmetic (split_double). Each column
-// step is two phases with a barrier after each: the column of L (and an unscaled copy), then
-// the trailing update of the lower triangle, one warp per row. Every thread forms the pivot's
-// reciprocal itself, so the pivot needs no phase of its own. Tiny pivots are regularised as in
-// k_cholesky (to 1e-12 of the largest diagonal entry). On exit A holds L strictly below the
-// diagonal (unit diagonal implied) and D on it.
-__global__ void __launch_bounds__(1024) k_ldlt_df(double* A, int n, int* flag) {
-    extern __shared__ DF SD[];  // the matrix (n * n), then the unscaled column (n)
-    DF* ucol = SD + n * n;
-    __shared__ float dmax;
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
-        float h, l;
-        split_double(A[t], h, l);
-        SD[t] = DF(h, l);
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        float m = 0.f;
-        for (int j = threadIdx.x; j < n; j += 32) m = fmaxf(m, SD[j * n + j].hi);
+// inv, hi, lo: on the last step the inverse as FP64 (dst is then not written) and, where hi is not
+// null, as float pairs
+template <class T>
+__global__ void __launch_bounds__(GJ_NT) k_gj_step(const T* __restrict__ src, T* __restrict__ dst, int n, int kb,
+                                                   const double* dmax, double* inv, float* hi, float* lo) {
+    __shared__ T D[2][GJ_B][GJ_B + 1];    // A_KK, inverted in place (ping-pong)
+    __shared__ T C[GJ_T][GJ_B + 1];       // A_iK of the tile's rows
+    __shared__ T R[GJ_B][GJ_T + 1];       // A_Kj of the tile's columns
+    __shared__ T W[GJ_B][GJ_T + 1];       // P A_Kj (P itself where column j lies in K)
+    __shared__ T rp;
+    const int tid = threadIdx.x, k0 = kb * GJ_B, i0 = blockIdx.y * GJ_T, j0 = blockIdx.x * GJ_T;
+    auto at = [&](int i, int j) { return i < n && j < n ? src[(int64_t)i * n + j] : T(i == j ? 1 : 0); };
+    const int pi = tid / GJ_B, pj = tid % GJ_B;
+    const int tx = tid % GJ_T, ty = tid / GJ_T;
+    constexpr int ROWS = GJ_NT / GJ_T, TPT = GJ_T / ROWS;
+    T acc[TPT];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (threadIdx.x == 0) dmax = m;
+    for (int r = 0; r < TPT; ++r) acc[r] = at(i0 + ty + r * ROWS, j0 + tx);
+    D[0][pi][pj] = at(k0 + pi, k0 + pj);
+    for (int t = tid; t < GJ_T * GJ_B; t += GJ_NT) {
+        C[t / GJ_B][t % GJ_B] = at(i0 + t / GJ_B, k0 + t % GJ_B);
+        R[t / GJ_T][t % GJ_T] = at(k0 + t / GJ_T, j0 + t % GJ_T);
     }
     __syncthreads();
-    const float floor_ = 1e-12f * dmax;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int j = 0; j < n; ++j) {
-        DF a = SD[j * n + j];
-        if (!(a.hi > floor_)) {  // every thread takes the same branch (the value is idempotent)
-            a = DF(floor_);
-            if (threadIdx.x == 0) {
-                SD[j * n + j] = a;
-                *flag += 1;
+    const double least = 1e-12 * *dmax;
+    for (int p = 0; p < GJ_B; ++p) {
+        T(&S)[GJ_B][GJ_B + 1] = D[p & 1];
+        if (tid < 32) {  // one warp: FP64 instructions are issued per warp at a low rate
+            const T a = S[p][p];
+            const T q = gj_recip(gj_lead(a) > least ? a : T(least));
+            if (tid == 0) rp = q;
+        }
+        __syncthreads();
+        const T row = pj == p ? rp : S[p][pj] * rp;  // the scaled pivot row
+        T v;
+        if (pi == p) v = row;
+        else if (pj == p) v = T(0) - S[pi][p] * row;
+        else v = S[pi][pj] - S[pi][p] * row;
+        D[(p + 1) & 1][pi][pj] = v;
+        __syncthreads();
+    }
+    T(&P)[GJ_B][GJ_B + 1] = D[GJ_B & 1];
+    for (int t = tid; t < GJ_B * GJ_T; t += GJ_NT) {
+        const int m = t / GJ_T, c = t % GJ_T, jk = j0 + c - k0;
+        T w = T(0);
+        if (jk >= 0 && jk < GJ_B) {
+            w = P[m][jk];
+        } else {
+#pragma unroll
+            for (int q = 0; q < GJ_B; ++q) w = w + P[m][q] * R[q][c];
+        }
+        W[m][c] = w;
+    }
+    __syncthreads();
+    const int j = j0 + tx;
+    const bool col_in = j >= k0 && j < k0 + GJ_B;
+#pragma unroll
+    for (int r = 0; r < TPT; ++r) {
+        const int li = ty + r * ROWS, i = i0 + li;
+        T v = col_in ? T(0) : acc[r];
+        if (i >= k0 && i < k0 + GJ_B) {
+            v = W[i - k0][tx];
+        } else {
+#pragma unroll
+            for (int q = 0; q < GJ_B; ++q) v = v - C[li][q] * W[q][tx];
+        }
+        if (i < n && j < n) {
+            const int64_t e = (int64_t)i * n + j;
+            if (inv == nullptr) {
+                dst[e] = v;
+            } else {
+                const double d = gj_value(v);
+                inv[e] = d;
+                if (hi != nullptr) split_double(d, hi[e], lo[e]);
             }
         }
-        const DF ia = df_recip(a);
-        for (int k = j + 1 + threadIdx.x; k < n; k += blockDim.x) {
-            const DF u = SD[k * n + j];
-            ucol[k] = u;
-            SD[k * n + j] = u * ia;
-        }
-        __syncthreads();
-        for (int i = j + 1 + warp; i < n; i += nw) {
-            const DF lij = SD[i * n + j];
-            for (int k = j + 1 + lane; k <= i; k += 32) SD[i * n + k] = SD[i * n + k] - lij * ucol[k];
-        }
-        __syncthreads();
     }
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) A[t] = SD[t].value();
-}
-
-// Column c of A^-1 from L D L^T (k_ldlt_df), one CTA per column: L y = e_c, z = D^-1 y,
-// L^T x = z, one barrier per step (each thread reads the settled entry of the step and
-// updates the others).
-__global__ void __launch_bounds__(256) k_ldlt_inverse_df(const double* LD, double* Ainv, int n) {
-    extern __shared__ DF SD[];  // L (n * n), 1 / D (n), the column (n)
-    DF* rd = SD + n * n;
-    DF* xs = rd + n;
-    const int c = blockIdx.x;
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
-        float h, l;
-        split_double(LD[t], h, l);
-        SD[t] = DF(h, l);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        rd[i] = df_recip(SD[i * n + i]);
-        xs[i] = DF(i == c ? 1.f : 0.f);
-    }
-    __syncthreads();
-    for (int j = c; j < n - 1; ++j) {  // L y = e_c (y_j = 0 for j < c)
-        const DF yj = xs[j];
-        for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) xs[i] = xs[i] - SD[i * n + j] * yj;
-        __syncthreads();
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) xs[i] = xs[i] * rd[i];
-    __syncthreads();
-    for (int j = n - 1; j > 0; --j) {  // L^T x = z
-        const DF xj = xs[j];
-        for (int i = threadIdx.x; i < j; i += blockDim.x) xs[i] = xs[i] - SD[j * n + i] * xj;
-        __syncthreads();
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) Ainv[(int64_t)i * n + c] = xs[i].value();
 }
 
 // x = A^-1 b on the coarsest grid (FP64), one warp per row.
@@ -1068,47 +967,36 @@ void cheb_coefficients(double bound, double lo_frac, int degree, double* out) {
     }
 }
 
-static int coarse_factor(anl_ctx* c, cudaStream_t s) {
-    Level& L = c->lev.back();
-    const int n = c->nc;
+// The inverse of the coarsest grid's matrix into c->Ainv (and its float pairs for the tail): the
+// steps alternate between c->A and c->Ainv, starting where the last one ends in c->Ainv.
+template <class T>
+static int coarse_invert(anl_ctx* c, cudaStream_t s) {
+    const Level& L = c->lev.back();
+    const int n = c->nc, steps = (n + GJ_B - 1) / GJ_B, tiles = (n + GJ_T - 1) / GJ_T;
+    static_assert(sizeof(T) == sizeof(double), "both arrays hold either form");
+    T* buf[2] = {reinterpret_cast<T*>(c->A), reinterpret_cast<T*>(c->Ainv)};
+    int cur = (steps + 1) & 1;
+    ANL_CUDA(cudaMemsetAsync(c->coarse_dmax, 0, sizeof(double), s));
     const int64_t total = (int64_t)n * n;
-    k_assemble_dense<<<(int)std::min<int64_t>(4096, (total + 255) / 256), 256, 0, s>>>(L.d, L.E, L.nmask, c->ke_d, n, c->A);
+    k_assemble_dense<T><<<(int)std::min<int64_t>(4096, (total + 255) / 256), 256, 0, s>>>(
+        L.d, L.E, L.nmask, c->ke_d, n, buf[cur], reinterpret_cast<unsigned long long*>(c->coarse_dmax));
     ANL_LAUNCH_CHECK();
-    ANL_CUDA(cudaMemsetAsync(c->flag_d, 0, sizeof(int), s));
-    if (n <= kCholSmemN) {
-        const int fb = n * n * (int)sizeof(double), ib = (n * n + 2 * n) * (int)sizeof(double);
-        static bool attr = false;
-        if (!attr) {
-            ANL_CUDA(cudaFuncSetAttribute(k_cholesky_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          kCholSmemN * kCholSmemN * (int)sizeof(double)));
-            ANL_CUDA(cudaFuncSetAttribute(k_chol_inverse_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (kCholSmemN * kCholSmemN + 2 * kCholSmemN) * (int)sizeof(double)));
-            ANL_CUDA(cudaFuncSetAttribute(k_ldlt_df, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (kCholSmemN * kCholSmemN + kCholSmemN) * (int)sizeof(DF)));
-            ANL_CUDA(cudaFuncSetAttribute(k_ldlt_inverse_df, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (kCholSmemN * kCholSmemN + 2 * kCholSmemN) * (int)sizeof(DF)));
-            attr = true;
-        }
-        if (c->fp64) {
-            k_cholesky_smem<<<1, 1024, fb, s>>>(c->A, n, c->flag_d);
-            ANL_LAUNCH_CHECK();
-            k_chol_inverse_smem<<<n, 256, ib, s>>>(c->A, c->Ainv, n);
-            ANL_LAUNCH_CHECK();
-        } else {  // the FP32 solver's preconditioner: double-float factor and inverse
-            k_ldlt_df<<<1, 1024, (n * n + n) * (int)sizeof(DF), s>>>(c->A, n, c->flag_d);
-            ANL_LAUNCH_CHECK();
-            k_ldlt_inverse_df<<<n, 256, (n * n + 2 * n) * (int)sizeof(DF), s>>>(c->A, c->Ainv, n);
-            ANL_LAUNCH_CHECK();
-        }
-    } else {
-        k_cholesky<<<1, 1024, 0, s>>>(c->A, n, c->flag_d);
-        ANL_LAUNCH_CHECK();
-        k_chol_inverse<<<n, 128, n * sizeof(double), s>>>(c->A, c->Ainv, n);
+    for (int k = 0; k < steps; ++k, cur ^= 1) {
+        const bool last = k + 1 == steps;
+        k_gj_step<T><<<dim3(tiles, tiles), GJ_NT, 0, s>>>(buf[cur], buf[cur ^ 1], n, k, c->coarse_dmax,
+                                                          last ? c->Ainv : nullptr, last ? c->ainv_hi : nullptr,
+                                                          c->ainv_lo);
         ANL_LAUNCH_CHECK();
     }
-    if (c->tail_from >= 0) ANL_TRY(launch_ainv_split(c->Ainv, n, c->ainv_hi, c->ainv_lo, s));
     c->coarse_ready = true;
     return ANL_OK;
+}
+
+// FP32 contexts invert in double-float arithmetic up to GJ_DF_N unknowns and in FP64 above, FP64
+// contexts always in FP64.
+constexpr int GJ_DF_N = 160;
+static int coarse_factor(anl_ctx* c, cudaStream_t s) {
+    return c->fp64 || c->nc > GJ_DF_N ? coarse_invert<double>(c, s) : coarse_invert<DF>(c, s);
 }
 
 // Refresh the hierarchy's element scales from the level-0 scales; with `rebuild` also
