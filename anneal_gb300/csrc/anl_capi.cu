@@ -259,7 +259,6 @@ static void free_ctx(anl_ctx* c) {
     f(c->partials);
     f(c->counter);
     f(c->red_out);
-    f(c->filt.w);
     f(c->filt.Hs);
     f(c->ftmp);
     f(c->ftmp2);

@@ -27,15 +27,21 @@ struct Level {
     int64_t vs = 0;
 };
 
+constexpr int kMaxFilterR = 5;
+// the taps of a filter layer by (|dx|, |dy|) in either order
+constexpr int kFilterClasses = (kMaxFilterR + 1) * (kMaxFilterR + 2) / 2;
+__host__ __device__ constexpr int filter_class(int a, int b) {
+    return a >= b ? a * (a + 1) / 2 + b : b * (b + 1) / 2 + a;
+}
+
 struct FilterState {
     bool ready = false;
     int R = 0;
     double r = 0.0;
-    float* w = nullptr;   // (2R+1)^3 cone weights, device
-    float* Hs = nullptr;  // conv(active), zeros replaced by 1
+    float wc[kMaxFilterR + 1][kFilterClasses];  // cone weights by |dz| and class
+    float* Hs = nullptr;                        // conv(active), zeros replaced by 1
 };
 
-constexpr int kMaxFilterR = 5;
 constexpr int kChebMax = 32;
 constexpr int kChebStride = 1 + 2 * kChebMax;
 

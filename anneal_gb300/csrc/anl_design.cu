@@ -6,7 +6,7 @@
 #include <algorithm>
 #include <cstddef>
 #include <cmath>
-#include <vector>
+#include <cstring>
 
 #include "anl_ctx.cuh"
 
@@ -17,19 +17,31 @@ static inline int dgrid(int64_t n) { return (int)std::max<int64_t>(1, std::min<i
 
 // ------------------------------------------------------------------ density filter
 
-// Filter (optimize.py:24-47). One CTA of 32x8 threads owns a 32x8 column of elements over
-// FT_ZC layers and marches up z: a ring of 2R + 2 element planes (each with an R-element halo
-// in x and y) in shared memory, one new plane staged per layer, one barrier per layer (the ring
-// has one slot more than the stencil reads, so the next plane never lands in a slot in use).
-// The taps are summed in (dz, dy, dx) order.
+// Filter (optimize.py:24-47). One CTA of 32x8 threads owns a 32x8 column of elements and marches
+// up z, one staged plane (with an R-element halo in x and y) per layer, double-buffered with one
+// barrier. The cone's weight depends on (|dx|, |dy|, |dz|) alone and not on the order of |dx| and
+// |dy|, so a thread sums its plane's (2R+1)^2 values once by class (|dx|, |dy|), weighs the class
+// sums for each |dz| and adds these R + 1 partial results to the 2R + 1 output layers they belong
+// to, kept in registers. Against a ring of 2R + 2 planes re-read for every layer this takes a
+// (2R+1)-th of the shared-memory loads and, at R = 2, 42 instead of 125 multiply-adds: the kernel
+// was bound by them at R >= 2 and by its latency chain at R = 1. Forward with projection and
+// backward at 128x64x64, r = 2.6: 166 -> 23 us together (memory floor 2 us).
 enum { F_HS = 0, F_FWD = 1, F_BWD = 2, F_PHYS = 3, F_OCVOL = 4 };
 
 constexpr int FT_X = 32, FT_Y = 8, FT_ZC = 16, FT_N = FT_X * FT_Y;
+// Layers per CTA. A chunk stages 2R layers more than it writes, and a layer is a chain of memory
+// latencies, so a grid of few columns is cut into shorter chunks until it has about three CTAs
+// per SM (4 layers at least; with 16 at 128x64x64 a third of the SMs had one CTA and the others
+// none).
+static inline int filter_chunk(const Dims& d) {
+    const int columns = ceil_div(d.nx, FT_X) * ceil_div(d.ny, FT_Y);
+    return std::max(4, std::min(FT_ZC, ceil_div(d.nz, ceil_div(3 * 152, columns))));
+}
 
 struct FilterArgs {
     Dims d;
-    int R;
-    const float* w;        // (2R+1)^3 cone weights
+    int zc;                // layers per CTA
+    float wc[kMaxFilterR + 1][kFilterClasses];  // cone weights by |dz| and class (|dx|, |dy|)
     const uint8_t* active;
     const float* Hs;
     const float* in;       // FWD/BWD/PHYS input field
@@ -78,14 +90,11 @@ __device__ __forceinline__ float oc_xn(float x, float dcx, float dvx, float lam,
     return oc_xn(oc_elem(x, dcx, dvx, move), lam, oc_rl(lam));
 }
 
-// the filter's input value of element (gi, gj, gk) (zero outside the grid and on inactive
-// elements): the active flag and the field are loaded independently of each other
+// the filter's input value of element e (zero on inactive elements): the active flag and the
+// field are loaded independently of each other
 template <int MODE>
-__device__ __forceinline__ float filter_input(const FilterArgs& a, int gi, int gj, int gk) {
-    const Dims& d = a.d;
-    if (gi < 0 || gj < 0 || gk < 0 || gi >= d.nx || gj >= d.ny || gk >= d.nz) return 0.f;
-    const int64_t e = d.elem(gi, gj, gk);
-    if (!ANL_IN_RANGE(e, d.ne())) return 0.f;
+__device__ __forceinline__ float filter_input(const FilterArgs& a, int64_t e) {
+    if (!ANL_IN_RANGE(e, a.d.ne())) return 0.f;
     const bool act = a.active[e] != 0;
     float v = 1.f;
     if (MODE == F_FWD || MODE == F_PHYS) v = a.in[e];
@@ -94,60 +103,79 @@ __device__ __forceinline__ float filter_input(const FilterArgs& a, int gi, int g
     return act ? v : 0.f;
 }
 
-// RT: the halo at compile time (1: the 27-tap cone of radii up to 2, weights in registers),
-// or 0 for any R up to kMaxFilterR
-template <int MODE, int RT>
+// The staged plane of a halo-R tile: which elements this thread stages.
+template <int R>
+struct FilterTile {
+    static constexpr int TX = FT_X + 2 * R, PL = TX * (FT_Y + 2 * R), PF = (PL + FT_N - 1) / FT_N;
+    int64_t exy[PF];  // index within an element plane, -1 outside the grid or the tile
+    __device__ FilterTile(const Dims& d, int i0, int j0, int tid) {
+#pragma unroll
+        for (int q = 0; q < PF; ++q) {
+            const int t = tid + q * FT_N, y = t / TX, x = t - y * TX, gi = i0 - R + x, gj = j0 - R + y;
+            exy[q] = t < PL && gi >= 0 && gj >= 0 && gi < d.nx && gj < d.ny ? gi + (int64_t)d.nx * gj : -1;
+        }
+    }
+};
+
+// Adds the plane's contribution around (tx, ty) to the 2R + 1 layers of acc: acc[R] is the
+// plane's own layer.
+template <int R>
+__device__ __forceinline__ void filter_plane(const float (&wc)[kMaxFilterR + 1][kFilterClasses], const float* pl,
+                                             int tx, int ty, float (&acc)[2 * R + 1]) {
+    constexpr int NC = (R + 1) * (R + 2) / 2;
+    float cs[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) cs[c] = 0.f;
+#pragma unroll
+    for (int dy = -R; dy <= R; ++dy)
+#pragma unroll
+        for (int dx = -R; dx <= R; ++dx) {
+            const int ax = dx < 0 ? -dx : dx, ay = dy < 0 ? -dy : dy;
+            cs[filter_class(ax, ay)] += pl[(ty + R + dy) * FilterTile<R>::TX + tx + R + dx];
+        }
+#pragma unroll
+    for (int q = 0; q <= R; ++q) {
+        float s = wc[q][0] * cs[0];
+#pragma unroll
+        for (int c = 1; c < NC; ++c) s = fmaf(wc[q][c], cs[c], s);
+        acc[R - q] += s;
+        if (q > 0) acc[R + q] += s;
+    }
+}
+
+template <int MODE, int R>
 __global__ void __launch_bounds__(FT_N) k_filter(FilterArgs a) {
-    extern __shared__ float sm[];
+    using Tile = FilterTile<R>;
+    __shared__ float pl[2][Tile::PL];
     const Dims d = a.d;
-    const int R = RT > 0 ? RT : a.R, W = 2 * R + 1;
-    const int TX = FT_X + 2 * R, TY = FT_Y + 2 * R, PL = TX * TY, NS = W + 1;  // ring of NS planes
-    float* ring = sm;
-    float* wts = sm + NS * PL;
     const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + FT_X * ty;
-    const int i0 = blockIdx.x * FT_X, j0 = blockIdx.y * FT_Y, kb = blockIdx.z * FT_ZC;
-    const int kend = min(kb + FT_ZC, d.nz);
-    for (int t = tid; t < W * W * W; t += FT_N) wts[t] = a.w[t];
-    // stage element plane gk into its ring slot
-    auto stage = [&](int gk) {
-        float* pl = ring + ((gk + NS * (kMaxFilterR + 1)) % NS) * PL;
-        for (int y = ty; y < TY; y += FT_Y)
-            for (int x = tx; x < TX; x += FT_X) pl[y * TX + x] = filter_input<MODE>(a, i0 - R + x, j0 - R + y, gk);
-    };
-    // the next plane's values of this thread, loaded a layer ahead (registers; the plane of a
-    // 27-tap filter is 34 x 10 values, at most 2 per thread)
-    constexpr int PF = RT == 1 ? (34 * 10 + FT_N - 1) / FT_N : 1;
-    float pf[PF];
+    const int i0 = blockIdx.x * FT_X, j0 = blockIdx.y * FT_Y, kb = blockIdx.z * a.zc;
+    const int kend = min(kb + a.zc, d.nz);
+    const int64_t eplane = (int64_t)d.nx * d.ny;
+    const Tile tile(d, i0, j0, tid);
+    float pf[Tile::PF];  // the next plane's values of this thread, loaded a layer ahead
     auto prefetch = [&](int gk) {
 #pragma unroll
-        for (int q = 0; q < PF; ++q) {
-            const int t = tid + q * FT_N, y = t / (FT_X + 2), x = t - y * (FT_X + 2);
-            pf[q] = t < PL ? filter_input<MODE>(a, i0 - 1 + x, j0 - 1 + y, gk) : 0.f;
-        }
+        for (int q = 0; q < Tile::PF; ++q)
+            pf[q] = tile.exy[q] >= 0 && gk >= 0 && gk < d.nz ? filter_input<MODE>(a, tile.exy[q] + gk * eplane) : 0.f;
     };
-    auto commit = [&](int gk) {
-        float* pl = ring + ((gk + NS * (kMaxFilterR + 1)) % NS) * PL;
-#pragma unroll
-        for (int q = 0; q < PF; ++q) {
-            const int t = tid + q * FT_N;
-            if (t < PL) pl[t] = pf[q];
-        }
-    };
-    for (int gk = kb - R; gk < kb + R; ++gk) stage(gk);
-    if (RT == 1) prefetch(kb + R);
-    __syncthreads();
-    float wr[RT > 0 ? 27 : 1];
-    if (RT == 1) {
-#pragma unroll
-        for (int q = 0; q < (RT > 0 ? 27 : 1); ++q) wr[q] = wts[q];
-    }
+    prefetch(kb - R);
     const int i = i0 + tx, j = j0 + ty;
     const bool in_xy = i < d.nx && j < d.ny;
+    float acc[2 * R + 1];
+#pragma unroll
+    for (int q = 0; q < 2 * R + 1; ++q) acc[q] = 0.f;
     double vol = 0.0;
-    for (int k = kb; k < kend; ++k) {
-        // this layer's epilogue inputs, loaded before the barrier so their latency overlaps it
-        const int64_t e = in_xy ? d.elem(i, j, k) : 0;
-        const bool in_e = in_xy && ANL_IN_RANGE(e, d.ne());
+    for (int gk = kb - R; gk < kend + R; ++gk) {
+        float* buf = pl[gk & 1];
+#pragma unroll
+        for (int q = 0; q < Tile::PF; ++q)
+            if (tid + q * FT_N < Tile::PL) buf[tid + q * FT_N] = pf[q];
+        if (gk + 1 < kend + R) prefetch(gk + 1);
+        // the epilogue inputs of the layer that this plane completes
+        const int k = gk - R;
+        const int64_t e = in_xy && k >= kb ? d.elem(i, j, k) : 0;
+        const bool in_e = in_xy && k >= kb && ANL_IN_RANGE(e, d.ne());
         bool act = false, fzn = false;
         float hs = 1.f, ph = 0.f;
         if (in_e) {
@@ -156,34 +184,13 @@ __global__ void __launch_bounds__(FT_N) k_filter(FilterArgs a) {
             if (MODE == F_PHYS || MODE == F_OCVOL) fzn = a.frozen[e] != 0;
             if (MODE == F_OCVOL) ph = a.phi[e];
         }
-        if (RT == 1) {  // plane k + 1 was loaded during the previous layer; load plane k + 2
-            commit(k + 1);
-            if (k + 1 < kend) prefetch(k + 2);
-        } else {
-            stage(k + R);
-        }
         __syncthreads();
+        filter_plane<R>(a.wc, buf, tx, ty, acc);
+        const float s = acc[0];
+#pragma unroll
+        for (int q = 0; q < 2 * R; ++q) acc[q] = acc[q + 1];
+        acc[2 * R] = 0.f;
         if (in_e) {
-            float s = 0.f;
-            if (RT == 1) {
-#pragma unroll
-                for (int dz = 0; dz < 3; ++dz) {
-                    const float* pl = ring + ((k - 1 + dz + NS * (kMaxFilterR + 1)) % NS) * PL;
-#pragma unroll
-                    for (int dy = 0; dy < 3; ++dy)
-#pragma unroll
-                        for (int dx = 0; dx < 3; ++dx) s = fmaf(wr[(dz * 3 + dy) * 3 + dx], pl[(ty + dy) * TX + tx + dx], s);
-                }
-            } else {
-                for (int dz = 0; dz < W; ++dz) {
-                    const float* pl = ring + ((k - R + dz + NS * (kMaxFilterR + 1)) % NS) * PL;
-                    for (int dy = 0; dy < W; ++dy) {
-                        const float* row = pl + (ty + dy) * TX + tx;
-                        const float* w = wts + (dz * W + dy) * W;
-                        for (int dx = 0; dx < W; ++dx) s = fmaf(w[dx], row[dx], s);
-                    }
-                }
-            }
             if (MODE == F_HS) {
                 a.out[e] = s == 0.f ? 1.f : s;
             } else if (MODE == F_FWD) {
@@ -225,19 +232,23 @@ __global__ void __launch_bounds__(FT_N) k_filter(FilterArgs a) {
 static int launch_filter(anl_ctx* c, int mode, FilterArgs a, cudaStream_t s) {
     const Dims& d = c->d;
     a.d = d;
-    a.R = c->filt.R;
-    a.w = c->filt.w;
+    std::memcpy(a.wc, c->filt.wc, sizeof(a.wc));
     a.active = c->active;
     a.Hs = c->filt.Hs;
-    const int W = 2 * a.R + 1;
-    const size_t smem = sizeof(float) * ((W + 1) * (FT_X + 2 * a.R) * (FT_Y + 2 * a.R) + W * W * W);
-    dim3 grid(ceil_div(d.nx, FT_X), ceil_div(d.ny, FT_Y), ceil_div(d.nz, FT_ZC)), block(FT_X, FT_Y);
+    a.zc = filter_chunk(d);
+    dim3 grid(ceil_div(d.nx, FT_X), ceil_div(d.ny, FT_Y), ceil_div(d.nz, a.zc)), block(FT_X, FT_Y);
     if (mode == F_OCVOL && (int64_t)grid.x * grid.y * grid.z > c->part_cap) {
         set_error("filter reduction needs %d blocks, scratch holds %d", grid.x * grid.y * grid.z, c->part_cap);
         return ANL_ERR_BADARG;
     }
-#define F_LAUNCH(M)                                                              \
-    (a.R == 1 ? k_filter<M, 1><<<grid, block, smem, s>>>(a) : k_filter<M, 0><<<grid, block, smem, s>>>(a))
+#define F_LAUNCH(M)                                                    \
+    switch (c->filt.R) {                                               \
+        case 1: k_filter<M, 1><<<grid, block, 0, s>>>(a); break;       \
+        case 2: k_filter<M, 2><<<grid, block, 0, s>>>(a); break;       \
+        case 3: k_filter<M, 3><<<grid, block, 0, s>>>(a); break;       \
+        case 4: k_filter<M, 4><<<grid, block, 0, s>>>(a); break;       \
+        default: k_filter<M, 5><<<grid, block, 0, s>>>(a); break;      \
+    }
     switch (mode) {
         case F_HS: F_LAUNCH(F_HS); break;
         case F_FWD: F_LAUNCH(F_FWD); break;
@@ -258,25 +269,17 @@ int filter_init(anl_ctx* c, double r, cudaStream_t s) {
         set_error("filter radius %.3f voxels needs a %d-element halo; at most %d is supported", r, R, kMaxFilterR);
         return ANL_ERR_BADARG;
     }
-    const int W = 2 * R + 1;
-    std::vector<float> w(W * W * W);
-    for (int dz = -R; dz <= R; ++dz)
-        for (int dy = -R; dy <= R; ++dy)
-            for (int dx = -R; dx <= R; ++dx) {
-                const double v = r - std::sqrt((double)(dx * dx + dy * dy + dz * dz));
-                w[(dx + R) + W * ((dy + R) + W * (dz + R))] = v > 0 ? (float)v : 0.f;
+    for (int q = 0; q <= kMaxFilterR; ++q)
+        for (int ax = 0; ax <= kMaxFilterR; ++ax)
+            for (int ay = 0; ay <= ax; ++ay) {
+                const double v = r - std::sqrt((double)(ax * ax + ay * ay + q * q));
+                c->filt.wc[q][filter_class(ax, ay)] = v > 0 ? (float)v : 0.f;
             }
-    std::lock_guard<std::recursive_mutex> lock(device_sync_mutex());
-    if (c->filt.w) cudaFree(c->filt.w);
-    c->filt.w = nullptr;
-    ANL_CUDA(cudaMalloc(&c->filt.w, sizeof(float) * w.size()));
-    ANL_CUDA(cudaMemcpyAsync(c->filt.w, w.data(), sizeof(float) * w.size(), cudaMemcpyHostToDevice, s));
     c->filt.R = R;
     c->filt.r = r;
     FilterArgs a{};
     a.out = c->filt.Hs;
     ANL_TRY(launch_filter(c, F_HS, a, s));
-    ANL_CUDA(cudaStreamSynchronize(s));  // the host weights vector goes out of scope
     c->filt.ready = true;
     return ANL_OK;
 }
