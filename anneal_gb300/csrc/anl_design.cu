@@ -4,6 +4,7 @@
 // Element fields are FP32 on the full grid (x fastest, zero on inactive elements); sums
 // that decide the OC bisection and the history values accumulate in FP64.
 #include <algorithm>
+#include <climits>
 #include <cstddef>
 #include <cmath>
 #include <cstring>
@@ -26,7 +27,7 @@ static inline int dgrid(int64_t n) { return (int)std::max<int64_t>(1, std::min<i
 // (2R+1)-th of the shared-memory loads and, at R = 2, 42 instead of 125 multiply-adds: the kernel
 // was bound by them at R >= 2 and by its latency chain at R = 1. Forward with projection and
 // backward at 128x64x64, r = 2.6: 166 -> 23 us together (memory floor 2 us).
-enum { F_HS = 0, F_FWD = 1, F_BWD = 2, F_PHYS = 3, F_OCVOL = 4 };
+enum { F_HS = 0, F_FWD = 1, F_BWD = 2, F_PHYS = 3 };
 
 constexpr int FT_X = 32, FT_Y = 8, FT_ZC = 16, FT_N = FT_X * FT_Y;
 // Layers per CTA. A chunk stages 2R layers more than it writes, and a layer is a chain of memory
@@ -50,15 +51,6 @@ struct FilterArgs {
     const uint8_t* frozen;
     float* dxp;
     float beta, eta, t0, t1;
-    // OCVOL: the filtered field is xn(lambda) built on the fly
-    const float* x;
-    const float* dcx;
-    const float* dvx;
-    const float* phi;
-    float lam, move;
-    double* partials;
-    unsigned* counter;
-    double* red_out;
 };
 
 // optimize.py:150-152: ratio = sqrt(max(-dcx,0) / max(dvx*lam, 1e-300)),
@@ -99,7 +91,6 @@ __device__ __forceinline__ float filter_input(const FilterArgs& a, int64_t e) {
     float v = 1.f;
     if (MODE == F_FWD || MODE == F_PHYS) v = a.in[e];
     else if (MODE == F_BWD) v = a.in[e] / a.Hs[e];
-    else if (MODE == F_OCVOL) v = a.frozen[e] ? 1.f : oc_xn(a.x[e], a.dcx[e], a.dvx[e], a.lam, a.move);
     return act ? v : 0.f;
 }
 
@@ -165,7 +156,6 @@ __global__ void __launch_bounds__(FT_N) k_filter(FilterArgs a) {
     float acc[2 * R + 1];
 #pragma unroll
     for (int q = 0; q < 2 * R + 1; ++q) acc[q] = 0.f;
-    double vol = 0.0;
     for (int gk = kb - R; gk < kend + R; ++gk) {
         float* buf = pl[gk & 1];
 #pragma unroll
@@ -177,12 +167,11 @@ __global__ void __launch_bounds__(FT_N) k_filter(FilterArgs a) {
         const int64_t e = in_xy && k >= kb ? d.elem(i, j, k) : 0;
         const bool in_e = in_xy && k >= kb && ANL_IN_RANGE(e, d.ne());
         bool act = false, fzn = false;
-        float hs = 1.f, ph = 0.f;
+        float hs = 1.f;
         if (in_e) {
             act = a.active[e] != 0;
-            if (MODE == F_FWD || MODE == F_PHYS || MODE == F_OCVOL) hs = a.Hs[e];
-            if (MODE == F_PHYS || MODE == F_OCVOL) fzn = a.frozen[e] != 0;
-            if (MODE == F_OCVOL) ph = a.phi[e];
+            if (MODE == F_FWD || MODE == F_PHYS) hs = a.Hs[e];
+            if (MODE == F_PHYS) fzn = a.frozen[e] != 0;
         }
         __syncthreads();
         filter_plane<R>(a.wc, buf, tx, ty, acc);
@@ -199,65 +188,42 @@ __global__ void __launch_bounds__(FT_N) k_filter(FilterArgs a) {
                 a.out[e] = act ? s : 0.f;
             } else {
                 // physical(): projection (optimize.py:81-87), frozen -> 1 (optimize.py:92)
-                float xt = act ? s / hs : 0.f;
-                float xp = xt, g = 1.f;
+                float xp = act ? s / hs : 0.f, g = 1.f;
                 if (a.beta > 0.f) {
-                    const float th = tanhf(a.beta * (xt - a.eta));
+                    const float th = tanhf(a.beta * (xp - a.eta));
                     xp = (a.t0 + th) / (a.t0 + a.t1);
                     g = a.beta * (1.f - th * th) / (a.t0 + a.t1);
                 }
-                if (fzn) xp = 1.f;
-                if (!act) {
-                    xp = 0.f;
-                    g = 0.f;
-                }
-                if (MODE == F_PHYS) {
-                    a.out[e] = xp;
-                    if (a.dxp) a.dxp[e] = g;
-                } else {
-                    vol += act ? (double)ph * (double)xp : 0.0;
-                }
+                a.out[e] = act ? (fzn ? 1.f : xp) : 0.f;
+                if (a.dxp) a.dxp[e] = act ? g : 0.f;
             }
         }
     }
-    if (MODE == F_OCVOL) {
-        __shared__ double red[FT_N / 32];
-        double v[1] = {vol};
-        block_sum<1, FT_N>(v, red, tid);
-        const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-        finish_reduction<1, FT_N>(v, bid, gridDim.x * gridDim.y * gridDim.z, a.partials, a.counter, a.red_out, tid, red);
-    }
 }
 
-static int launch_filter(anl_ctx* c, int mode, FilterArgs a, cudaStream_t s) {
-    const Dims& d = c->d;
-    a.d = d;
-    std::memcpy(a.wc, c->filt.wc, sizeof(a.wc));
+static FilterArgs filter_args(const anl_ctx* c) {
+    FilterArgs a{};
+    a.d = c->d;
     a.active = c->active;
     a.Hs = c->filt.Hs;
-    a.zc = filter_chunk(d);
-    dim3 grid(ceil_div(d.nx, FT_X), ceil_div(d.ny, FT_Y), ceil_div(d.nz, a.zc)), block(FT_X, FT_Y);
-    if (mode == F_OCVOL && (int64_t)grid.x * grid.y * grid.z > c->part_cap) {
-        set_error("filter reduction needs %d blocks, scratch holds %d", grid.x * grid.y * grid.z, c->part_cap);
-        return ANL_ERR_BADARG;
+    std::memcpy(a.wc, c->filt.wc, sizeof(a.wc));
+    a.zc = filter_chunk(a.d);
+    return a;
+}
+static dim3 filter_grid(const FilterArgs& a) {
+    return dim3(ceil_div(a.d.nx, FT_X), ceil_div(a.d.ny, FT_Y), ceil_div(a.d.nz, a.zc));
+}
+
+template <int MODE>
+static int launch_filter(anl_ctx* c, const FilterArgs& a, cudaStream_t s) {
+    const dim3 grid = filter_grid(a), block(FT_X, FT_Y);
+    switch (c->filt.R) {
+        case 1: k_filter<MODE, 1><<<grid, block, 0, s>>>(a); break;
+        case 2: k_filter<MODE, 2><<<grid, block, 0, s>>>(a); break;
+        case 3: k_filter<MODE, 3><<<grid, block, 0, s>>>(a); break;
+        case 4: k_filter<MODE, 4><<<grid, block, 0, s>>>(a); break;
+        default: k_filter<MODE, 5><<<grid, block, 0, s>>>(a); break;
     }
-#define F_LAUNCH(M)                                                    \
-    switch (c->filt.R) {                                               \
-        case 1: k_filter<M, 1><<<grid, block, 0, s>>>(a); break;       \
-        case 2: k_filter<M, 2><<<grid, block, 0, s>>>(a); break;       \
-        case 3: k_filter<M, 3><<<grid, block, 0, s>>>(a); break;       \
-        case 4: k_filter<M, 4><<<grid, block, 0, s>>>(a); break;       \
-        default: k_filter<M, 5><<<grid, block, 0, s>>>(a); break;      \
-    }
-    switch (mode) {
-        case F_HS: F_LAUNCH(F_HS); break;
-        case F_FWD: F_LAUNCH(F_FWD); break;
-        case F_BWD: F_LAUNCH(F_BWD); break;
-        case F_PHYS: F_LAUNCH(F_PHYS); break;
-        case F_OCVOL: F_LAUNCH(F_OCVOL); break;
-        default: return ANL_ERR_BADARG;
-    }
-#undef F_LAUNCH
     ANL_LAUNCH_CHECK();
     return ANL_OK;
 }
@@ -277,23 +243,23 @@ int filter_init(anl_ctx* c, double r, cudaStream_t s) {
             }
     c->filt.R = R;
     c->filt.r = r;
-    FilterArgs a{};
+    FilterArgs a = filter_args(c);
     a.out = c->filt.Hs;
-    ANL_TRY(launch_filter(c, F_HS, a, s));
+    ANL_TRY(launch_filter<F_HS>(c, a, s));
     c->filt.ready = true;
     return ANL_OK;
 }
 
 int filter_apply(anl_ctx* c, bool forward, const float* in, float* out, cudaStream_t s) {
-    FilterArgs a{};
+    FilterArgs a = filter_args(c);
     a.in = in;
     a.out = out;
-    return launch_filter(c, forward ? F_FWD : F_BWD, a, s);
+    return forward ? launch_filter<F_FWD>(c, a, s) : launch_filter<F_BWD>(c, a, s);
 }
 
 int physical(anl_ctx* c, const float* x, const uint8_t* frozen, double beta, double eta, float* xphys, float* dxp,
              cudaStream_t s) {
-    FilterArgs a{};
+    FilterArgs a = filter_args(c);
     a.in = x;
     a.out = xphys;
     a.frozen = frozen;
@@ -304,7 +270,7 @@ int physical(anl_ctx* c, const float* x, const uint8_t* frozen, double beta, dou
         a.t0 = (float)std::tanh(beta * eta);
         a.t1 = (float)std::tanh(beta * (1 - eta));
     }
-    return launch_filter(c, F_PHYS, a, s);
+    return launch_filter<F_PHYS>(c, a, s);
 }
 
 // ------------------------------------------------------------------ stiffness scale
@@ -553,16 +519,24 @@ __global__ void k_oc_scale(int64_t ne, const uint8_t* active, const uint8_t* fro
     finish_pair_sums<3>(v, partials, counter, out, sm);
 }
 
-// With no projection the volume is linear in xn: vol = sum_j wv_j xn_j + sum_frozen phi,
-// wv = Filter.backward(phi on non-frozen elements). One pass evaluates a bank of up to OC_BANK
-// lambdas, the nodes of OC_BANK_DEPTH consecutive bisection steps; each volume is its own
-// deterministic two-stage sum, so the bisection takes the decisions a pass per step would.
-// The part of each element's update that does not depend on lambda is formed once per OC
-// update (k_oc_prep): (s, dvx, lo, hi) and (g, w), with g the value where dvx lambda underflows
-// (hi if the element grows, else lo), frozen elements as lo = hi = 1 and inactive ones with w = 0.
-// A pass then costs a multiply, a compare, a clamp and a multiply-add per lambda and element.
-constexpr int OC_BANK_DEPTH = 4;
-constexpr int OC_BANK = (1 << OC_BANK_DEPTH) - 1;
+// The bisection (optimize.py:147-160) on the device. Its answer is the last midpoint lambda, the
+// updates use lambda in FP32, and the volume falls with lambda, so the bisection is decided once
+// two neighbouring floats are known with the volume above the target at the lower one and not
+// above it at the upper one: its midpoints then fall on either side without another volume.
+// Each pass evaluates the volume at a bank of lambdas inside the bracket known so far and its last
+// block narrows the bracket and picks the next bank (oc_advance): 4-5 passes of 15 or 6-7 passes
+// of 3 lambdas instead of one volume for each of the 36 steps.
+//  * No projection: the volume is linear in xn, vol = sum_j wv_j xn_j + sum_frozen phi, with
+//    wv = Filter.backward(phi on non-frozen elements): k_oc_vol_bank, a stream over the elements,
+//    issue-bound at 15 lambdas (about 8 instructions per lambda and element).
+//  * Projection: xn is filtered and projected for each lambda: k_oc_vol_proj, the filter's march
+//    with 3 lambdas side by side (their staged planes share the loads; more lambdas cost more
+//    than the passes they save).
+// The part of each element's update that does not depend on lambda is formed once per OC update
+// (k_oc_prep): (s, dvx, lo, hi) and (g, w), with g the value where dvx lambda underflows (hi if
+// the element grows, else lo) and w the weight of the volume, frozen elements as lo = hi = 1 and
+// inactive ones with w = 0. A lambda then costs a multiply, a compare and a clamp per element.
+constexpr int OC_BANK = 15, OC_PROJ = 3;
 static_assert(OC_BANK <= kMaxRedVals, "one partial per lambda and block");
 static_assert(OC_BANK <= 16, "the bank's volumes fit red_out");
 struct OcBank {
@@ -588,109 +562,119 @@ __global__ void k_oc_prep(int64_t ne, const uint8_t* __restrict__ active, const 
     }
 }
 
-// One element of the bank pass: adds w * xn(lambda_j) to acc[j] for every lambda of the bank.
-// Each thread takes its elements in grid-stride order and adds them per lambda in FP32 in a
-// fixed order; blocks and the grid add in float pairs.
-// The bisection's state in device memory: the passes, the decisions between them and the final
-// update run back to back on the stream with no host round trip (optimize.py:147-160).
+// The search's state in device memory: the passes and the final update run back to back on the
+// stream with no host round trip. Positive floats order like their bits, so the bracket is kept
+// in bits: an interval of them is a range of lambda on a nearly logarithmic scale.
 struct OcState {
-    double lo, hi, lam;
+    double lo, hi, lam;  // the bisection's first bracket; its last midpoint
     double vfrozen, vtarget;
     int steps, stop;
-    OcBank bank;            // the lambdas of the next pass (FP32, as the passes use them)
-    double lamd[OC_BANK];   // the same lambdas in FP64: the decisions' sqrt(lo hi)
+    int tlo, thi;        // bits of the largest lambda known above the target volume (-1: none yet), of
+                         // the smallest one not above it (INT_MAX: none yet)
+    double flo, fhi;     // their volumes
+    OcBank bank;         // the lambdas of the next pass
 };
 
-// The bank of the next OC_BANK_DEPTH (at most 100 - steps) bisection steps from [lo, hi], by one
-// warp: level by level of the bisection tree (node j of the in-order numbering), the nodes of a
-// level in parallel lanes, so the FP64 square roots (slow on this part) form a chain of `depth`.
-// Each node's value is sqrt(l h) of its interval, as the bisection forms it.
-__device__ void oc_make_bank(OcState* st, int lane) {
-    __shared__ double L[OC_BANK], H[OC_BANK];
-    const int depth = min(OC_BANK_DEPTH, 100 - st->steps);
-    const int nodes = (1 << depth) - 1, root = (1 << (depth - 1)) - 1;
-    if (lane == 0) {
-        L[root] = st->lo;
-        H[root] = st->hi;
-        st->bank.n = nodes;
+// one warp: after a pass, narrow the bracket; then either replay the bisection or choose the next
+// bank of at most nmax lambdas
+__device__ void oc_advance(OcState* st, const double* vols, int nmax, int lane) {
+    int tlo = st->tlo, thi = st->thi;
+    const int n = st->bank.n;
+    const int64_t width = (int64_t)thi - tlo;
+    double flo = st->flo, fhi = st->fhi;
+    const double target = st->vtarget, frozen = st->vfrozen;
+    for (int j = 0; j < n; ++j) {
+        const int p = __float_as_int(st->bank.lam[j]);
+        const double v = vols[j] + frozen;
+        if (v > target && p > tlo) tlo = p, flo = v;
+    }
+    for (int j = 0; j < n; ++j) {
+        const int p = __float_as_int(st->bank.lam[j]);
+        const double v = vols[j] + frozen;
+        if (!(v > target) && p > tlo && p < thi) thi = p, fhi = v;
     }
     __syncwarp();
-    for (int level = 0; level < depth; ++level) {
-        const int half = 1 << (depth - 1 - level);
-        const int j = half - 1 + lane * 2 * half;
-        if (lane < (1 << level)) {
-            const double t = sqrt(L[j] * H[j]);
-            st->lamd[j] = t;
-            st->bank.lam[j] = (float)t;
-            if (level + 1 < depth) {
-                L[j - half / 2] = L[j];
-                H[j - half / 2] = t;
-                L[j + half / 2] = t;
-                H[j + half / 2] = H[j];
+    // the first bank holds both ends of the bisection's bracket: a missing side has no lambda
+    if (tlo < 0 || thi == INT_MAX || thi - tlo <= 1) {
+        if (lane == 0) {  // the bisection's own steps, each decided by the bracket
+            double lo = st->lo, hi = st->hi, lam = st->lam;
+            int steps = 0;
+            while (steps < 100) {
+                lam = sqrt(lo * hi);
+                (__float_as_int((float)lam) <= tlo ? lo : hi) = lam;
+                ++steps;
+                if (hi < lo * (1 + 1e-9)) break;
             }
+            st->lam = lam;
+            st->steps = steps;
+            st->stop = 1;
         }
-        __syncwarp();
+        return;
+    }
+    // Inside: every float while they fit the bank; else around the zero of the line through the
+    // two ends (the line's error shrinks with the square of the interval), at doubling distances;
+    // else, where the last pass narrowed the bracket by less than 4, at even distances.
+    const int gap = thi - tlo - 1, m = min(nmax, gap), h = (m - 1) / 2;
+    int p;
+    if (gap <= nmax) {
+        p = tlo + 1 + lane;
+    } else if (thi - tlo > width / 4 && width < INT_MAX) {
+        p = tlo + (int)((int64_t)(thi - tlo) * (lane + 1) / (m + 1));
+    } else {
+        const double d = thi - tlo;
+        const int r = max(tlo + 1, min(thi - 1, tlo + (int)(d * ((flo - target) / (flo - fhi)))));
+        const double near = fmax(1.0, fmin(d * d * (1.0 / 8388608.0 / 256.0), d / (double)(1 << h)));
+        const int t = lane - h;
+        const double off = t == 0 ? 0.0 : near * (double)(1 << (min(abs(t), 16) - 1));
+        p = t < 0 ? r - (int)off : r + (int)off;
+        p = max(tlo + 1, min(thi - 1, p));
+    }
+    if (lane < m) st->bank.lam[lane] = __int_as_float(p);
+    if (lane == 0) {
+        st->bank.n = m;
+        st->tlo = tlo;
+        st->thi = thi;
+        st->flo = flo;
+        st->fhi = fhi;
     }
 }
 
-// one warp
-__global__ void k_oc_begin(OcState* st, const double* sums, const double* vfrozen, double vtarget) {
-    if (threadIdx.x == 0) {
-        // optimize.py:145: the bracket from the mean sensitivities of the design elements
-        double scale = 1.0;
-        const double nd = sums[2];
-        if (nd > 0) {
-            const double mdc = sums[0] / nd, mdv = sums[1] / nd;
-            scale = fmax(mdc / fmax(mdv, 1e-30), 1e-300);
-        }
-        st->lo = scale * 1e-8;
-        st->hi = scale * 1e8;
-        st->lam = sqrt(st->lo * st->hi);
+// one warp: the bisection's bracket and the first bank, denser around the mean ratio
+__global__ void k_oc_begin(OcState* st, const double* sums, const double* vfrozen, double vtarget, int n) {
+    const int lane = threadIdx.x;
+    // optimize.py:145: the bracket from the mean sensitivities of the design elements
+    double scale = 1.0;
+    const double nd = sums[2];
+    if (nd > 0) {
+        const double mdc = sums[0] / nd, mdv = sums[1] / nd;
+        scale = fmax(mdc / fmax(mdv, 1e-30), 1e-300);
+    }
+    const double lo = scale * 1e-8, hi = scale * 1e8;
+    if (lane < n) {
+        const int h = (n - 1) / 2, t = lane - h;
+        const int a = __float_as_int((float)lo), b = __float_as_int((float)hi), c = __float_as_int((float)scale);
+        const double u = (double)t / h, off = u * u * u;
+        const int p = c + (int)(off * (t < 0 ? c - a : b - c));
+        st->bank.lam[lane] = __int_as_float(t == -h ? a : t == h ? b : p);
+    }
+    if (lane == 0) {
+        st->lo = lo;
+        st->hi = hi;
+        st->lam = sqrt(lo * hi);
         st->vfrozen = vfrozen ? *vfrozen : 0.0;
         st->vtarget = vtarget;
         st->steps = 0;
         st->stop = 0;
+        st->tlo = -1;
+        st->thi = INT_MAX;
+        st->flo = st->fhi = 0.0;
+        st->bank.n = n;
     }
-    __syncwarp();
-    oc_make_bank(st, threadIdx.x);
-}
-
-// one warp: the bank's steps, one per level of the tree (optimize.py:147-160), then the next bank
-__global__ void k_oc_decide(OcState* st, const double* vols) {
-    if (st->stop) return;  // the same for every lane
-    if (threadIdx.x == 0) {
-        const int depth = min(OC_BANK_DEPTH, 100 - st->steps);
-        int idx = (1 << (depth - 1)) - 1, step = depth >= 2 ? 1 << (depth - 2) : 0;
-        double lo = st->lo, hi = st->hi, lam = st->lam;
-        for (int d = 0; d < depth; ++d) {
-            lam = st->lamd[idx];  // sqrt(lo hi) of the current bracket
-            const double vol = vols[idx] + st->vfrozen;
-            if (vol > st->vtarget) {
-                lo = lam;
-                idx += step;
-            } else {
-                hi = lam;
-                idx -= step;
-            }
-            step >>= 1;
-            ++st->steps;
-            if (hi / lo < 1 + 1e-9) {
-                st->stop = 1;
-                break;
-            }
-        }
-        st->lo = lo;
-        st->hi = hi;
-        st->lam = lam;
-        if (st->steps >= 100) st->stop = 1;
-    }
-    __syncwarp();
-    if (!st->stop) oc_make_bank(st, threadIdx.x);
 }
 
 constexpr int OCB_T = 512;  // threads of a bank pass: one CTA per SM, each thread ~54 elements at 12.8M DOF
 __global__ void __launch_bounds__(OCB_T, 1) k_oc_vol_bank(int64_t ne, const float4* __restrict__ el,
-                                                    const float2* __restrict__ gw, const OcState* st,
+                                                    const float2* __restrict__ gw, OcState* st,
                                                     double* partials, unsigned* counter, double* out) {
     if (st->stop) return;  // the same for every block
     const OcBank bank = st->bank;
@@ -730,7 +714,114 @@ __global__ void __launch_bounds__(OCB_T, 1) k_oc_vol_bank(int64_t ne, const floa
 #pragma unroll
     for (int j = 0; j < OC_BANK; ++j) lo[j] = 0.f;
     block_pair_sum<OC_BANK, OCB_T>(acc, lo, sm, threadIdx.x);
-    finish_pair_reduction<OC_BANK, OCB_T>(acc, lo, blockIdx.x, gridDim.x, partials, counter, out, threadIdx.x, sm);
+    if (finish_pair_reduction<OC_BANK, OCB_T>(acc, lo, blockIdx.x, gridDim.x, partials, counter, out, threadIdx.x, sm) &&
+        threadIdx.x < 32) {
+        __syncwarp();  // lane 0 wrote the volumes
+        oc_advance(st, out, OC_BANK, threadIdx.x);
+    }
+}
+
+// One pass with projection: the volume sum phi physical(xn(lambda)) of each lambda of the bank,
+// xn filtered as in k_filter; phi xp is summed exactly as float pairs.
+struct OcProjArgs {
+    FilterArgs f;
+    const float4* el;
+    const float2* gw;
+    OcState* st;
+    double* partials;
+    unsigned* counter;
+    double* out;
+};
+template <int R>
+__global__ void __launch_bounds__(FT_N) k_oc_vol_proj(OcProjArgs a) {
+    if (a.st->stop) return;  // the same for every block
+    using Tile = FilterTile<R>;
+    __shared__ float pl[2][OC_PROJ][Tile::PL];
+    __shared__ float2 sm[OC_PROJ * FT_N / 32];
+    const Dims d = a.f.d;
+    const int n = a.st->bank.n;
+    float lam[OC_PROJ], rl[OC_PROJ];
+#pragma unroll
+    for (int m = 0; m < OC_PROJ; ++m) {
+        lam[m] = a.st->bank.lam[min(m, n - 1)];
+        rl[m] = oc_rl(lam[m]);
+    }
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + FT_X * ty;
+    const int i0 = blockIdx.x * FT_X, j0 = blockIdx.y * FT_Y, kb = blockIdx.z * a.f.zc;
+    const int kend = min(kb + a.f.zc, d.nz);
+    const int64_t eplane = (int64_t)d.nx * d.ny;
+    const Tile tile(d, i0, j0, tid);
+    float4 pe[Tile::PF];  // the next plane's elements of this thread, loaded a layer ahead
+    float pg[Tile::PF];
+    auto prefetch = [&](int gk) {
+#pragma unroll
+        for (int q = 0; q < Tile::PF; ++q) {
+            const int64_t e = tile.exy[q] + gk * eplane;
+            const bool in = tile.exy[q] >= 0 && gk >= 0 && gk < d.nz && ANL_IN_RANGE(e, d.ne());
+            pe[q] = in ? a.el[e] : make_float4(0.f, 1.f, 0.f, 0.f);
+            pg[q] = in ? a.gw[e].x : 0.f;
+        }
+    };
+    prefetch(kb - R);
+    const int i = i0 + tx, j = j0 + ty;
+    const bool in_xy = i < d.nx && j < d.ny;
+    float acc[OC_PROJ][2 * R + 1];
+    PairSum vol[OC_PROJ];
+#pragma unroll
+    for (int m = 0; m < OC_PROJ; ++m)
+#pragma unroll
+        for (int q = 0; q < 2 * R + 1; ++q) acc[m][q] = 0.f;
+    for (int gk = kb - R; gk < kend + R; ++gk) {
+        float(&buf)[OC_PROJ][Tile::PL] = pl[gk & 1];
+#pragma unroll
+        for (int q = 0; q < Tile::PF; ++q)
+            if (tid + q * FT_N < Tile::PL) {
+#pragma unroll
+                for (int m = 0; m < OC_PROJ; ++m)  // oc_xn with the element's lambda-free parts
+                    buf[m][tid + q * FT_N] = pe[q].y * lam[m] > 1e-30f
+                                                 ? fminf(fmaxf(pe[q].x * rl[m], pe[q].z), pe[q].w) : pg[q];
+            }
+        if (gk + 1 < kend + R) prefetch(gk + 1);
+        const int k = gk - R;
+        const int64_t e = in_xy && k >= kb ? d.elem(i, j, k) : 0;
+        const bool in_e = in_xy && k >= kb && ANL_IN_RANGE(e, d.ne());
+        bool fzn = false;
+        float hs = 1.f, ph = 0.f;
+        if (in_e) {
+            ph = a.gw[e].y;  // zero on inactive elements
+            hs = a.f.Hs[e];
+            fzn = a.f.frozen[e] != 0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < OC_PROJ; ++m) {
+            filter_plane<R>(a.f.wc, buf[m], tx, ty, acc[m]);
+            if (in_e) {
+                const float th = tanhf(a.f.beta * (acc[m][0] / hs - a.f.eta));
+                const float xp = fzn ? 1.f : (a.f.t0 + th) / (a.f.t0 + a.f.t1);
+                float pv, pr;
+                two_prod(ph, xp, pv, pr);
+                vol[m].add(pv);
+                vol[m].l += pr;
+            }
+#pragma unroll
+            for (int q = 0; q < 2 * R; ++q) acc[m][q] = acc[m][q + 1];
+            acc[m][2 * R] = 0.f;
+        }
+    }
+    float h[OC_PROJ], l[OC_PROJ];
+#pragma unroll
+    for (int m = 0; m < OC_PROJ; ++m) {
+        h[m] = vol[m].h;
+        l[m] = vol[m].l;
+    }
+    block_pair_sum<OC_PROJ, FT_N>(h, l, sm, tid);
+    const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    if (finish_pair_reduction<OC_PROJ, FT_N>(h, l, bid, gridDim.x * gridDim.y * gridDim.z, a.partials, a.counter, a.out,
+                                             tid, sm) && tid < 32) {
+        __syncwarp();  // lane 0 wrote the volumes
+        oc_advance(a.st, a.out, OC_PROJ, tid);
+    }
 }
 
 __global__ void k_oc_weights(int64_t ne, const uint8_t* active, const uint8_t* frozen, const float* phi, float* v,
@@ -767,90 +858,75 @@ int oc_update(anl_ctx* c, const float* x, const float* dcx, const float* dvx, co
     k_oc_scale<<<dgrid(ne), DT, 0, s>>>(ne, c->active, frozen, dcx, dvx, c->partials, c->counter, c->red_out);
     ANL_LAUNCH_CHECK();
     const double mv = beta <= 1 ? move : move / 2;  // optimize.py:151
+    ANL_TRY(grow(c->oc_el, c->oc_el_cap, (size_t)ne, sizeof(float4)));
+    ANL_TRY(grow(c->oc_gw, c->oc_gw_cap, (size_t)ne, sizeof(float2)));
     const bool linear = !(beta > 0);
-    if (linear) {
-        // With no projection the volume is linear in xn (see k_oc_vol_bank): frozen volume and
-        // the filtered weights, the lambda-free element data, then the passes, each followed by
-        // its decisions, on the device; one synchronisation at the end
+    const float* weight = phi;
+    if (linear) {  // frozen volume and filtered weights: the volume is linear in xn
         k_oc_weights<<<dgrid(ne), DT, 0, s>>>(ne, c->active, frozen, phi, c->ftmp2, c->partials, c->counter,
                                               c->red_out + 8);
         ANL_LAUNCH_CHECK();
-        k_oc_begin<<<1, 32, 0, s>>>(st, c->red_out, c->red_out + 8, vtarget);
-        ANL_LAUNCH_CHECK();
-        ANL_TRY(filter_apply(c, false, c->ftmp2, c->ftmp, s));
-        ANL_TRY(grow(c->oc_el, c->oc_el_cap, (size_t)ne, sizeof(float4)));
-        ANL_TRY(grow(c->oc_gw, c->oc_gw_cap, (size_t)ne, sizeof(float2)));
-        k_oc_prep<<<dgrid(ne), DT, 0, s>>>(ne, c->active, frozen, x, dcx, dvx, c->ftmp, (float)mv, c->oc_el,
-                                           c->oc_gw);
-        ANL_LAUNCH_CHECK();
-        // the bracket ratio starts at 1e16 and is square-rooted by every step: 36 steps reach
-        // 1 + 1e-9; passes for 40, then more only if the state has not stopped (never seen)
-        int passes = (40 + OC_BANK_DEPTH - 1) / OC_BANK_DEPTH;
-        static int sms = 0;
-        if (sms == 0) {
-            int dev = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        weight = c->ftmp;
+    }
+    k_oc_begin<<<1, 32, 0, s>>>(st, c->red_out, linear ? c->red_out + 8 : nullptr, vtarget, linear ? OC_BANK : OC_PROJ);
+    ANL_LAUNCH_CHECK();
+    if (linear) ANL_TRY(filter_apply(c, false, c->ftmp2, c->ftmp, s));
+    k_oc_prep<<<dgrid(ne), DT, 0, s>>>(ne, c->active, frozen, x, dcx, dvx, weight, (float)mv, c->oc_el, c->oc_gw);
+    ANL_LAUNCH_CHECK();
+    static int sms = 0;
+    if (sms == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    }
+    const int bank_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(sms, (ne + OCB_T - 1) / OCB_T));
+    OcProjArgs pa{};
+    dim3 pgrid, pblock(FT_X, FT_Y);
+    if (!linear) {
+        pa.f = filter_args(c);
+        pa.f.frozen = frozen;
+        pa.f.beta = (float)beta;
+        pa.f.eta = (float)eta;
+        pa.f.t0 = (float)std::tanh(beta * eta);
+        pa.f.t1 = (float)std::tanh(beta * (1 - eta));
+        pa.el = c->oc_el;
+        pa.gw = c->oc_gw;
+        pa.st = st;
+        pa.partials = c->partials;
+        pa.counter = c->counter;
+        pa.out = c->red_out;
+        pgrid = filter_grid(pa.f);
+        if ((int64_t)pgrid.x * pgrid.y * pgrid.z > c->part_cap) {
+            set_error("filter reduction needs %d blocks, scratch holds %d", pgrid.x * pgrid.y * pgrid.z, c->part_cap);
+            return ANL_ERR_BADARG;
         }
-        const int bank_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(sms, (ne + OCB_T - 1) / OCB_T));
-        for (int round = 0; round < 100 / OC_BANK_DEPTH + 1; ++round) {
-            for (int q = 0; q < passes; ++q) {
+    }
+    // the usual number of passes at once (a pass after the last decision returns at once), then
+    // two more at a time: every pass or the one after it narrows the bracket fourfold
+    int passes = linear ? 5 : 7;
+    for (int done = 0; done < 80; done += passes, passes = 2) {
+        for (int q = 0; q < passes; ++q) {
+            if (linear) {
                 k_oc_vol_bank<<<bank_blocks, OCB_T, 0, s>>>(ne, c->oc_el, c->oc_gw, st, c->partials, c->counter,
                                                             c->red_out);
-                ANL_LAUNCH_CHECK();
-                k_oc_decide<<<1, 32, 0, s>>>(st, c->red_out);
-                ANL_LAUNCH_CHECK();
+            } else {
+                switch (c->filt.R) {
+                    case 1: k_oc_vol_proj<1><<<pgrid, pblock, 0, s>>>(pa); break;
+                    case 2: k_oc_vol_proj<2><<<pgrid, pblock, 0, s>>>(pa); break;
+                    case 3: k_oc_vol_proj<3><<<pgrid, pblock, 0, s>>>(pa); break;
+                    case 4: k_oc_vol_proj<4><<<pgrid, pblock, 0, s>>>(pa); break;
+                    default: k_oc_vol_proj<5><<<pgrid, pblock, 0, s>>>(pa); break;
+                }
             }
-            ANL_CUDA(cudaMemcpyAsync(c->red_h, st, offsetof(OcState, bank), cudaMemcpyDeviceToHost, s));
-            ANL_CUDA(cudaStreamSynchronize(s));
-            if (reinterpret_cast<const OcState*>(c->red_h)->stop) break;
-            passes = 1;
+            ANL_LAUNCH_CHECK();
         }
-    } else {
-        ANL_TRY(read_red(c, 3, s));
-        double scale = 1.0;  // optimize.py:145
-        const double nd = c->red_h[2];
-        if (nd > 0) {
-            const double mdc = c->red_h[0] / nd, mdv = c->red_h[1] / nd;
-            scale = std::max(mdc / std::max(mdv, 1e-30), 1e-300);
-        }
-        double lo = scale * 1e-8, hi = scale * 1e8, lam = std::sqrt(lo * hi);
-        int steps = 0;
-        for (int k = 0; k < 100; ++k) {  // projected volume: one filter pass per step
-            lam = std::sqrt(lo * hi);
-            FilterArgs a{};
-            a.frozen = frozen;
-            a.beta = (float)beta;
-            a.eta = (float)eta;
-            a.t0 = (float)std::tanh(beta * eta);
-            a.t1 = (float)std::tanh(beta * (1 - eta));
-            a.x = x;
-            a.dcx = dcx;
-            a.dvx = dvx;
-            a.phi = phi;
-            a.lam = (float)lam;
-            a.move = (float)mv;
-            a.partials = c->partials;
-            a.counter = c->counter;
-            a.red_out = c->red_out;
-            ANL_TRY(launch_filter(c, F_OCVOL, a, s));
-            ANL_TRY(read_red(c, 1, s));
-            const double vol = c->red_h[0];
-            if (vol > vtarget) lo = lam;
-            else hi = lam;
-            ++steps;
-            if (hi / lo < 1 + 1e-9) break;
-        }
-        OcState* h = reinterpret_cast<OcState*>(c->red_h);  // pinned; its head fields only
-        h->lo = lo;
-        h->hi = hi;
-        h->lam = lam;
-        h->vfrozen = 0.0;
-        h->vtarget = vtarget;
-        h->steps = steps;
-        h->stop = 1;
-        ANL_CUDA(cudaMemcpyAsync(st, h, offsetof(OcState, bank), cudaMemcpyHostToDevice, s));
+        ANL_CUDA(cudaMemcpyAsync(c->red_h, st, offsetof(OcState, tlo), cudaMemcpyDeviceToHost, s));
         ANL_CUDA(cudaStreamSynchronize(s));
+        if (reinterpret_cast<const OcState*>(c->red_h)->stop) break;
+    }
+    if (!reinterpret_cast<const OcState*>(c->red_h)->stop) {
+        set_error("OC update: the multiplier's bracket did not close");
+        return ANL_ERR_STATE;
     }
     k_oc_final<<<dgrid(ne), DT, 0, s>>>(ne, c->active, frozen, x, dcx, dvx, st, (float)mv, xnew);
     ANL_LAUNCH_CHECK();
