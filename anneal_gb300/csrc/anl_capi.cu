@@ -425,26 +425,26 @@ static int create(anl_ctx** out, int nx, int ny, int nz, double h, double nu, in
         free_ctx(c);
         return ANL_ERR_CUDA;
     }
-    // the V-cycle tail: the first level (level 2 or below, on the box levels) from which every
-    // level to the coarsest fits one CTA (at most 1024 elements, the vectors in shared memory)
+    // the V-cycle tail: the first level from which every level to the coarsest fits one cluster
+    // (ANL_TAIL=0 turns it off)
     {
-        // on by default (ANL_TAIL=0 turns it off): on the 256x128x128 L-bracket the tail takes
-        // levels 4-6 in 104 us per V-cycle against about 180 us for their 35 launches, 34.7
-        // against 33.9 SIMP iterations/s at the same CG iterations
         const char* e = std::getenv("ANL_TAIL");
         const bool tail_on = !(e && std::atoi(e) == 0);
         const int nl = (int)c->lev.size();
         if (tail_on && !c->fp64 && c->dense_coarse && nl >= 2) {
-            for (int l = std::max(c->box_from, 2); l <= nl - 2 && c->tail_from < 0; ++l) {
-                if (nl - l > kTailMaxLevels || c->lev[l].d.ne() > 1024) continue;
-                TailLevel tl[kTailMaxLevels];
-                for (int q = l; q < nl; ++q) tl[q - l].d = c->lev[q].d;
-                if (tail_smem_bytes(tl, nl - l) <= (size_t)kTailMaxSmem) c->tail_from = l;
+            if (vtail_prepare(&c->tail_ctas) != ANL_OK) {
+                free_ctx(c);
+                return ANL_ERR_CUDA;
             }
-        }
-        if (c->tail_from >= 0 && vtail_prepare() != ANL_OK) {
-            free_ctx(c);
-            return ANL_ERR_CUDA;
+            for (int l = 0; l <= nl - 2 && c->tail_from < 0; ++l) {
+                if (nl - l > kTailMaxLevels) continue;
+                TailLevel tl[kTailMaxLevels];
+                for (int q = l; q < nl; ++q) {
+                    tl[q - l].d = c->lev[q].d;
+                    tl[q - l].degree = c->degree(q);
+                }
+                if (vtail_fits(tl, nl - l, c->tail_ctas)) c->tail_from = l;
+            }
         }
     }
     c->b0_base = c->lev[0].b;

@@ -83,13 +83,15 @@ struct anl_ctx {
 #define ANL_MG_DEGREE_COARSE 8
 #endif
     int mg_degree_coarse = ANL_MG_DEGREE_COARSE;
+    int degree(size_t l) const { return l >= 2 ? mg_degree_coarse : mg_degree; }
     // first level smoothed by the box kernels (anl_kbox.cu; FP32 contexts): on the levels below
     // 128 x 64 x 64 elements a z-marching K u launch is a chain of latencies
     int box_from = 2;
     // the finest level's K u passes on the tensor cores (anl_kutc.cu; FP32 contexts)
     bool use_tc = false;
-    // first level of the one-CTA V-cycle tail (anl_vtail.cu; FP32 contexts), -1 for none
-    int tail_from = -1;
+    // first level of the V-cycle tail (anl_vtail.cu; FP32 contexts), -1 for none, and the CTAs of
+    // its cluster
+    int tail_from = -1, tail_ctas = 0;
     // right-hand-side slots (ANL_FLAG_RHS): the solve's per-vector state (the hierarchy's
     // vectors, p, q, the FP64 solution and right-hand side, its float-pair split, the PCG
     // scalars, the restart flags, the reduction scratch) exists once per slot; a batched solve

@@ -139,39 +139,40 @@ struct KbArgs {
 int launch_kbox(int mode, const KbArgs& a, const KeModal<float>& km, cudaStream_t s);
 void kbox_prepare();
 
-// ------------------------------------------------------------------ V-cycle tail in one CTA
+// ------------------------------------------------------------------ V-cycle tail in one cluster
 
-// The smallest levels of the V-cycle and the coarsest dense solve in one CTA (anl_vtail.cu):
-// level 0 of the tail takes b0 and returns its V-cycle correction in x0. Every level but the
-// last is smoothed (`degree` Chebyshev steps before and after); the last is solved with the
-// dense inverse as float pairs (ainv_hi + ainv_lo, nc x nc, symmetric).
-constexpr int kTailMaxLevels = 6;
-constexpr int kTailMaxSmem = 200 * 1024;
+// The smallest levels of the V-cycle and the coarsest dense solve in one thread-block cluster
+// (anl_vtail.cu): level 0 of the tail takes b0 and returns its V-cycle correction in lev[0].x.
+// Every level but the last is smoothed (`degree` Chebyshev steps before and after); the last is
+// solved with the dense inverse as float pairs (ainv_hi + ainv_lo, nc x nc, symmetric).
+constexpr int kTailMaxLevels = 8;
+constexpr int kTailMaxSmem = 220 * 1024;
 struct TailLevel {
     Dims d{};
     const float* E = nullptr;
     const uint8_t* nmask = nullptr;
     const float* diag = nullptr;
     const double* cheb = nullptr;  // (c1, c2) pairs of the level's sweep
+    int degree = 0;
+    float* r = nullptr;            // the level's residual and correction, slots vs floats apart
+    float* x = nullptr;
+    int64_t vs = 0;
 };
 struct TailArgs {
-    int nlev = 0;
+    int nlev = 0, ctas = 0;
     TailLevel lev[kTailMaxLevels];
-    int degree = 0;
-    const float* b0 = nullptr;
-    float* x0 = nullptr;
+    float* b0 = nullptr;
     const float* ainv_hi = nullptr;
     const float* ainv_lo = nullptr;
     int nc = 0;
     const int* done = nullptr;
     KeModal<float> km{};
-    // right-hand-side slots: CTA r works on slot r (b0, x0 and done offset by these strides)
+    // right-hand-side slots: cluster r works on slot r
     int nrhs = 1;
-    int64_t vstride = 0;  // floats between the slots' vectors of the first tail level
-    int sc_bytes = 0;     // bytes between the slots' done flags
+    int sc_bytes = 0;  // bytes between the slots' done flags
 };
-size_t tail_smem_bytes(const TailLevel* lev, int nlev);
-int vtail_prepare();
+int vtail_prepare(int* ctas);
+bool vtail_fits(const TailLevel* lev, int nlev, int ctas);
 int launch_vtail(const TailArgs& a, cudaStream_t s);
 
 // ------------------------------------------------------------------ tensor-core K u (fine grid)

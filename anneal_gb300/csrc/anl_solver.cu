@@ -1136,11 +1136,12 @@ static int vcycle_box(anl_ctx* c, size_t l, int deg, const int* done, cudaStream
     return ANL_OK;
 }
 
-// The levels from tail_from down in one CTA per right-hand-side slot: b of level l in, its
+// The levels from tail_from down in one cluster per right-hand-side slot: b of level l in, its
 // correction x out.
 static int vcycle_tail(anl_ctx* c, size_t l, const int* done, cudaStream_t s) {
     TailArgs a;
     a.nlev = (int)(c->lev.size() - l);
+    a.ctas = c->tail_ctas;
     for (int q = 0; q < a.nlev; ++q) {
         const Level& Lq = c->lev[l + q];
         a.lev[q].d = Lq.d;
@@ -1148,17 +1149,18 @@ static int vcycle_tail(anl_ctx* c, size_t l, const int* done, cudaStream_t s) {
         a.lev[q].nmask = Lq.nmask;
         a.lev[q].diag = Lq.diag;
         a.lev[q].cheb = c->cheb_d + (l + q) * kChebStride + 1;
+        a.lev[q].degree = c->degree(l + q);
+        a.lev[q].r = (float*)Lq.r;
+        a.lev[q].x = (float*)Lq.x;
+        a.lev[q].vs = Lq.vs;
     }
-    a.degree = c->mg_degree_coarse;
-    a.b0 = (const float*)c->lev[l].b;
-    a.x0 = (float*)c->lev[l].x;
+    a.b0 = (float*)c->lev[l].b;
     a.ainv_hi = c->ainv_hi;
     a.ainv_lo = c->ainv_lo;
     a.nc = c->nc;
     a.done = done;
     a.km = c->kmf;
     a.nrhs = c->rb;
-    a.vstride = c->lev[l].vs;
     a.sc_bytes = (int)sizeof(PcgScalars);
     return launch_vtail(a, s);
 }
@@ -1178,7 +1180,7 @@ static int vcycle(anl_ctx* c, size_t l, const int* done, cudaStream_t s) {
         return smooth<T>(c, L, 16, true, done, s);
     }
     Level& C = c->lev[l + 1];
-    const int deg = l >= 2 ? c->mg_degree_coarse : c->mg_degree;
+    const int deg = c->degree(l);
     if (sizeof(T) == 4 && (int)l >= c->box_from) return vcycle_box(c, l, deg, done, s);
     ANL_TRY(smooth<T>(c, L, deg, true, done, s));
     KuArgs<T> a = ku_args<T>(c, L);

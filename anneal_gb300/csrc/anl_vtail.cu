@@ -1,19 +1,37 @@
-// anl_vtail.cu -- the smallest levels of the V-cycle in one CTA, entirely in shared memory.
+// anl_vtail.cu -- the small levels of the V-cycle in one thread-block cluster, in shared memory.
 //
-// Below about a thousand elements a multigrid level is pure latency: each of its ~17 passes per
-// V-cycle (8 + 8 Chebyshev steps, the residual, the grid transfers) is a launch that moves a few
-// kilobytes. Here one CTA takes the right-hand side of the first such level and returns its
-// V-cycle correction: it smooths, restricts, solves the coarsest grid with the dense inverse
-// (kept as float pairs), prolongs and smooths back up, with only __syncthreads between the
-// steps. The arithmetic is that of the per-level kernels: the modal element product
-// (modal_element), Chebyshev on D^-1 K with the level's coefficients, trilinear transfers,
-// masks on fixed DOFs.
+// On a level of at most a few thousand elements a smoothing step is pure latency: as a launch of
+// its own it costs 6-7 us whatever it moves, and there are some 17 of them per level and V-cycle.
+// Here one cluster (16 CTAs, 8 where the part cannot place 16) takes the right-hand side of the
+// first level that fits it and returns its V-cycle correction: it smooths, restricts, solves the
+// coarsest grid with the dense inverse (kept as float pairs), prolongs and smooths back up. The
+// arithmetic is that of the per-level kernels: the modal element product (modal_element),
+// Chebyshev on D^-1 K with the level's coefficients, trilinear transfers, masks on fixed DOFs.
 //
-// K x on a level is two phases with one barrier after each: every element writes its 8 corner
-// forces to shared memory (structure of arrays, corner-component major), then every node sums
-// the corners of its up to 8 elements in a fixed order and applies its Chebyshev update (or
-// forms its residual) in the same pass. Node coordinates and element corner nodes come from
-// per-level tables built once per launch, so the steps do no integer division.
+// A level is cut into slabs of element layers along AXIS, the first level's longest side. A CTA
+// owns its layers' lower node planes (the last CTA also the top plane) and computes its own
+// element layers and the one below, so a step needs its neighbours' boundary planes of the
+// iterate and nothing else:
+//   1. every element writes its 8 corner forces to shared memory;
+//   2. __syncthreads; every owned node sums the forces that meet there in a fixed order, applies
+//      its Chebyshev update and writes its new value to its own copy of the iterate and, from a
+//      boundary plane, to the neighbour's halo plane: st.async into distributed shared memory,
+//      counted by the neighbour's mbarrier;
+//   3. the CTA waits for its own two halo planes only. The iterate is double-buffered and there is
+//      a barrier per direction and buffer: a neighbour can be one step ahead, never two, since it
+//      needs this CTA's plane of every step. (A cluster barrier a step costs 0.9 us: its release
+//      drains the remote stores first.)
+// A node stays with its thread for a whole sweep: its right-hand side, direction, inverse
+// diagonal and mask stay in registers. A level's forces have a zero row and column between their
+// rows, so a node sums 8 corners without a test; they lie 25 words apart (an odd stride, so
+// neither phase has bank conflicts). The transfers between levels, whose slabs do not match, go
+// through the levels' vectors in global memory, every load of a node in flight at once.
+//
+// What bounds it: the chain of one step (about 48 shared-memory accesses and 250 instructions per
+// element, then 24 and 80 per node, the halo's flight, two block barriers).
+// Measured steps: 1.4 us with 2 layers of 4 x 4 to 8 x 8 elements a CTA, 3.4 us with 3 layers of
+// 16 x 16; a CG iteration at 48x24x24 takes 128 us (168 with a launch per level and step), at
+// 96x48x48 226 us (288), at 256x128x128 944 us (992).
 #include "anl_common.cuh"
 #include "anl_kernels.cuh"
 
@@ -21,428 +39,598 @@ namespace anl {
 
 namespace {
 
-constexpr int TT = 1024;  // threads: one element each on a 1,024-element level
+constexpr int TT = 512;         // threads of a CTA
+constexpr int NPT = 2;          // owned nodes of a thread
+constexpr int FW = 25;          // words between two elements' forces (24 and one of padding)
+constexpr int kWaitTries = 1 << 20;  // bound of a halo wait
+constexpr int kTailMaxDegree = 16;  // Chebyshev steps per sweep there is room for
 
-// shared-memory carve-up of the tail, in 4-byte words (floats; int tables; node masks as bytes
-// padded to 4): per level x, b (and on the smoothed levels the direction / residual dv, the
-// inverse diagonal g, E, the packed node coordinates and the elements' first nodes), then one
-// element-force array for the largest smoothed level
-struct TailLayout {
-    int off_x[kTailMaxLevels], off_b[kTailMaxLevels], off_d[kTailMaxLevels], off_g[kTailMaxLevels];
-    int off_e[kTailMaxLevels], off_n[kTailMaxLevels], off_e0[kTailMaxLevels], off_m[kTailMaxLevels];
-    int off_f;
-    int words;
+// A level's slab of one CTA: A x B elements per layer, L layers along AXIS.
+template <int AXIS>
+struct Slab {
+    int A, B, L, per, active, own, nown, PA, planeN;
+    int64_t ns, na, nb, es, ea, eb;  // node and element strides along AXIS, A, B
+    __host__ __device__ Slab(const Dims& d, int rank, int ctas) {
+        const int n[3] = {d.nx, d.ny, d.nz};
+        constexpr int ax = AXIS == 0 ? 1 : 0, bx = AXIS == 2 ? 1 : 2;
+        const int64_t nstr[3] = {1, d.nx + 1, (int64_t)(d.nx + 1) * (d.ny + 1)};
+        const int64_t estr[3] = {1, d.nx, (int64_t)d.nx * d.ny};
+        A = n[ax];
+        B = n[bx];
+        L = n[AXIS];
+        ns = nstr[AXIS], na = nstr[ax], nb = nstr[bx];
+        es = estr[AXIS], ea = estr[ax], eb = estr[bx];
+        per = (L + ctas - 1) / ctas;
+        active = (L + per - 1) / per;
+        own = rank < active ? (per < L - rank * per ? per : L - rank * per) : 0;
+        nown = rank < active ? own + (rank == active - 1 ? 1 : 0) : 0;
+        PA = A + 1;
+        planeN = PA * (B + 1);
+    }
+    // sizes for any rank
+    __host__ __device__ int max_nodes() const { return (per + 1) * planeN; }
+    __host__ __device__ int max_elems() const { return (per + 1) * A * B; }
+    __host__ __device__ int max_padded() const { return (per + 2) * planeN + A + 2; }
 };
 
-__host__ __device__ inline TailLayout tail_layout(const TailLevel* lev, int nlev) {
+// shared-memory carve-up in words: the iterate twice (own planes and two halo planes), the coarsest
+// right-hand side, then per level the forces, the elements' (scale, packed indices) pairs and the
+// nodes' b and x
+struct TailLayout {
+    int x, xlen, c, f[kTailMaxLevels], e[kTailMaxLevels], save[kTailMaxLevels], words;
+};
+
+template <int AXIS>
+__host__ __device__ inline TailLayout tail_layout(const TailLevel* lev, int nlev, int ctas) {
     TailLayout t{};
-    int o = 0, max_ne = 0;
-    for (int l = 0; l < nlev; ++l) {
-        const int nn = (int)lev[l].d.nn(), ne = (int)lev[l].d.ne();
-        const bool coarsest = l == nlev - 1;
-        t.off_x[l] = o;
-        o += 3 * nn;
-        t.off_b[l] = o;
-        o += 3 * nn;
-        t.off_d[l] = t.off_g[l] = t.off_e[l] = t.off_n[l] = t.off_e0[l] = -1;
-        if (!coarsest) {
-            t.off_d[l] = o;
-            o += 3 * nn;
-            t.off_g[l] = o;
-            o += nn;
-            t.off_e[l] = o;
-            o += ne;
-            t.off_n[l] = o;
-            o += nn;
-            t.off_e0[l] = o;
-            o += ne;
-            max_ne = max_ne > ne ? max_ne : ne;
-        }
-        t.off_m[l] = o;
-        o += (nn + 3) / 4;
+    for (int l = 0; l < nlev - 1; ++l) {
+        const Slab<AXIS> g(lev[l].d, 0, ctas);
+        const int x = 3 * (g.max_nodes() + 2 * g.planeN);
+        t.xlen = t.xlen > x ? t.xlen : x;
     }
-    t.off_f = o;
-    o += 24 * max_ne;
-    t.words = o;
+    t.x = 0;
+    int o = 2 * t.xlen;
+    for (int l = 0; l < nlev - 1; ++l) {
+        const Slab<AXIS> g(lev[l].d, 0, ctas);
+        t.e[l] = o;
+        o += 2 * g.max_elems();
+        t.f[l] = o;
+        o += FW * g.max_padded();
+        t.save[l] = o;
+        o += 6 * g.max_nodes();
+        o += o & 1;
+    }
+    t.c = o;
+    t.words = o + 3 * (int)lev[nlev - 1].d.nn();
     return t;
 }
 
-// packed node coordinates (i, j, k < 2048, 2048, 1024)
-__device__ __forceinline__ int pack_ijk(int i, int j, int k) { return i | (j << 11) | (k << 22); }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// one word to another CTA of the cluster, counted on that CTA's barrier
+__device__ __forceinline__ void st_async(uint32_t addr, float v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr),
+                 "r"(__float_as_uint(v)), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void bar_expect(uint32_t bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// false once the wait has run out
+__device__ __forceinline__ bool bar_wait(uint32_t bar, unsigned parity) {
+    for (int q = 0; q < kWaitTries; ++q) {
+        unsigned ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
 
-// Everything a step indexes by level at run time (the levels, the carve-up) lives in shared
-// memory; a reference to the kernel's parameter would copy it to local memory.
-constexpr int kTailMaxDegree = 16;  // Chebyshev steps per sweep the tail holds coefficients for
+// components c0 .. c0 + NC - 1 of (R r)(I, J, K): trilinear weights 1, 1/2, 1/4, 1/8 of the fine
+// residual r; nodes outside the grid are read at its edge with weight 0, so no load depends on a
+// test and a plane's loads are in flight together
+template <int NC>
+__device__ __forceinline__ void restrict_at(const Dims& f, const float* r, int I, int J, int K, int c0,
+                                            float (&acc)[NC]) {
+    const int sy = f.nx + 1, sz = sy * (f.ny + 1);  // a tail level's indices fit an int
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[c] = 0.f;
+#pragma unroll 1
+    for (int dk = -1; dk <= 1; ++dk) {
+        const int k = 2 * K + dk;
+        const float* p = r + 3 * sz * min(max(k, 0), f.nz) + c0;
+        const float wk = k < 0 || k > f.nz ? 0.f : dk ? 0.5f : 1.f;
+        float v[9][NC];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+            const int i = min(max(2 * I + q % 3 - 1, 0), f.nx), j = min(max(2 * J + q / 3 - 1, 0), f.ny);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) v[q][c] = __ldcg(p + 3 * (i + sy * j) + c);
+        }
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+            const int di = q % 3 - 1, dj = q / 3 - 1, i = 2 * I + di, j = 2 * J + dj;
+            const bool in = i >= 0 && j >= 0 && i <= f.nx && j <= f.ny;
+            const float w = in ? (di ? 0.5f : 1.f) * (dj ? 0.5f : 1.f) * wk : 0.f;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) acc[c] = fmaf(w, v[q][c], acc[c]);
+        }
+    }
+}
 
-struct TailCtx {
-    const TailLevel* lev;  // shared-memory copy of the levels
-    const TailLayout& L;   // in shared memory
-    const float (*cheb)[2 * kTailMaxDegree];  // per level (c1, c2) of each step, in shared memory
+// (P xc)(i, j, k): the mean of the coarse nodes the fine node lies between (the unused ones of the
+// 8 are read at the node itself)
+__device__ __forceinline__ void prolong_at(const Dims& cd, const float* xc, int i, int j, int k, float (&acc)[3]) {
+    const int sy = cd.nx + 1, sz = sy * (cd.ny + 1), di = i & 1, dj = j & 1, dk = k & 1;
+    const int n0 = (i >> 1) + sy * (j >> 1) + sz * (k >> 1);
+    float v[8][3];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int n = n0 + (q & di) + sy * ((q >> 1) & dj) + sz * ((q >> 2) & dk);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[q][c] = __ldcg(xc + 3 * n + c);
+    }
+    const float w = (di ? 0.5f : 1.f) * (dj ? 0.5f : 1.f) * (dk ? 0.5f : 1.f);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) acc[c] = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        if (((q & 1) && !di) || ((q & 2) && !dj) || ((q & 4) && !dk)) continue;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[c] += v[q][c];
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) acc[c] *= w;
+}
+
+// an owned node of this thread on the current level
+struct TailNode {
+    int t;          // ordinal among the CTA's owned nodes, -1 for none
+    int nl;         // first word of the node in an iterate buffer
+    int nb;         // padded index of the element above it in every direction
+    int gn;         // node index on the level's grid
+    int i, j, k;
+    unsigned m;     // mask
+    float g;        // inverse diagonal
+    float b[3], d[3], x[3];
+    int down, up;   // words of its copies in the neighbours' halo planes, -1 for none
+};
+
+template <int AXIS>
+struct Tail {
+    const TailArgs& a;
+    const TailLayout& lay;
     float* sm;
-    int tid;
-    KeModal<float> km;
-    const float* ainv_hi;
-    const float* ainv_lo;
-    int nc;
-    __device__ float* X(int l) const { return sm + L.off_x[l]; }
-    __device__ float* B(int l) const { return sm + L.off_b[l]; }
-    __device__ float* Dv(int l) const { return sm + L.off_d[l]; }
-    __device__ float* G(int l) const { return sm + L.off_g[l]; }
-    __device__ float* E(int l) const { return sm + L.off_e[l]; }
-    __device__ int* Nijk(int l) const { return reinterpret_cast<int*>(sm + L.off_n[l]); }
-    __device__ int* E0(int l) const { return reinterpret_cast<int*>(sm + L.off_e0[l]); }
-    __device__ uint8_t* M(int l) const { return reinterpret_cast<uint8_t*>(sm + L.off_m[l]); }
-    __device__ float* F() const { return sm + L.off_f; }
+    uint32_t bar;                 // this CTA's barriers: [direction][buffer], 8 bytes each
+    uint32_t x_down, x_up, b_down, b_up;  // the neighbours' iterate buffers and barriers
+    int tid, rank, ctas, slot;
+    int cur = 0;                  // the buffer that holds the iterate
+    unsigned phase = 0;           // next phase parity of barrier [direction][buffer], one bit each
+    bool lost = false;            // a halo wait ran out
+    TailNode nd[NPT];
 
-    // phase 1 of K x on level l: the corner forces of every element into F (corner q = px +
-    // 2 py + 4 pz, component c at F[(3 q + c) ne + e]); ends with a barrier
-    __device__ void element_forces(int l) const {
-        const Dims d = lev[l].d;
-        const int ne = (int)d.ne();
-        const int sy = d.nx + 1, sz = (d.nx + 1) * (d.ny + 1);
-        const float* x = X(l);
-        const float* Ev = E(l);
-        const int* e0 = E0(l);
-        float* F_ = F();
+    __device__ float* vec(float* p, int l) const { return p + (int64_t)slot * a.lev[l].vs; }
+
+    // the element table of level l and its zeroed forces (once per launch)
+    __device__ void table(int l) {
+        const TailLevel& lv = a.lev[l];
+        const Slab<AXIS> g(lv.d, rank, ctas);
+        float* f = sm + lay.f[l];
+        for (int t = tid; t < FW * g.max_padded(); t += TT) f[t] = 0.f;
+        const int layer = g.A * g.B, ne = g.own > 0 ? (g.own + 1) * layer : 0;
+        float2* et = reinterpret_cast<float2*>(sm + lay.e[l]);
         for (int e = tid; e < ne; e += TT) {
-            const float Ee = Ev[e];
-            V3<float> f[2][2][2];
-            if (Ee != 0.f) {
-                const int n0 = e0[e];
-                V3<float> u[2][2][2];
+            const int q = e / layer, in = e - q * layer, b = in / g.A, aa = in - b * g.A;
+            const int gl = rank * g.per - 1 + q;
+            const int64_t ge = gl * g.es + aa * g.ea + b * g.eb;
+            const float Ee = gl >= 0 && ANL_IN_RANGE(ge, lv.d.ne()) ? __ldg(lv.E + ge) : 0.f;
+            const int n0 = q * g.planeN + aa + g.PA * b, pe = (q * (g.B + 1) + b + 1) * g.PA + aa + 1;
+            et[e] = make_float2(Ee, __int_as_float(n0 | (pe << 16)));
+        }
+    }
+
+    // this thread's nodes of level l
+    __device__ void enter(int l) {
+        const TailLevel& lv = a.lev[l];
+        const Slab<AXIS> g(lv.d, rank, ctas);
 #pragma unroll
-                for (int pz = 0; pz < 2; ++pz)
+        for (int r = 0; r < NPT; ++r) {
+            TailNode& n = nd[r];
+            const int t = tid + r * TT;
+            n.t = -1;
+            n.m = 0;
+            n.g = 0.f;
 #pragma unroll
-                    for (int py = 0; py < 2; ++py)
+            for (int c = 0; c < 3; ++c) n.b[c] = n.d[c] = n.x[c] = 0.f;
+            if (t >= g.nown * g.planeN) continue;
+            const int p = 1 + t / g.planeN, in = t - (p - 1) * g.planeN, b = in / g.PA, aa = in - b * g.PA;
+            const int s = rank * g.per + p - 1;
+            n.gn = (int)(s * g.ns + aa * g.na + b * g.nb);
+            if (!ANL_IN_RANGE(n.gn, lv.d.nn())) continue;
+            n.t = t;
+            n.nl = 3 * (p * g.planeN + in);
+            n.nb = FW * ((p * (g.B + 1) + b + 1) * g.PA + aa + 1);
+            n.i = AXIS == 0 ? s : aa;
+            n.j = AXIS == 1 ? s : AXIS == 0 ? aa : b;
+            n.k = AXIS == 2 ? s : b;
+            n.m = __ldg(lv.nmask + n.gn) & 7u;
+            n.g = __ldg(lv.diag + n.gn);
+            n.down = p == 1 && rank > 0 ? 3 * ((g.per + 1) * g.planeN + in) : -1;
+            n.up = p == g.nown && rank + 1 < g.active ? 3 * in : -1;
+        }
+    }
+
+    // the nodes' x into the other buffer and the neighbours' halo planes; then the wait for the own
+    // halo planes
+    __device__ void exchange(int l) {
+        const Dims& d = a.lev[l].d;
+        const int L = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;
+        const int per = (L + ctas - 1) / ctas, active = (L + per - 1) / per;
+        const int planeN = ((AXIS == 0 ? d.ny : d.nx) + 1) * ((AXIS == 2 ? d.ny : d.nz) + 1);
+        cur ^= 1;
+        const bool from[2] = {rank > 0 && rank < active, rank + 1 < active};
+        if (tid == 0) {
 #pragma unroll
-                        for (int px = 0; px < 2; ++px) {
-                            const float* p = x + 3 * (n0 + px + py * sy + pz * sz);
-                            u[px][py][pz].xy = make_float2(p[0], p[1]);
-                            u[px][py][pz].z = p[2];
-                        }
-                V3<float> dxb[2], dxt[2], dyb[2], dyt[2], dz[2][2];
+            for (int q = 0; q < 2; ++q)
+                if (from[q]) bar_expect(bar + 8u * (2 * q + cur), 12u * (unsigned)planeN);
+        }
+        const int o = cur * lay.xlen;
 #pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    dxb[q] = u[1][q][0] - u[0][q][0];
-                    dxt[q] = u[1][q][1] - u[0][q][1];
-                    dyb[q] = u[q][1][0] - u[q][0][0];
-                    dyt[q] = u[q][1][1] - u[q][0][1];
-                }
+        for (int r = 0; r < NPT; ++r) {
+            const TailNode& n = nd[r];
+            if (n.t < 0) continue;
 #pragma unroll
-                for (int px = 0; px < 2; ++px)
-#pragma unroll
-                    for (int py = 0; py < 2; ++py) dz[px][py] = u[px][py][1] - u[px][py][0];
-                modal_element<float>(km, Ee, dxb, dxt, dyb, dyt, dz, f);
-            } else {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) (&f[0][0][0])[q] = v3zero<float>();
+            for (int c = 0; c < 3; ++c) {
+                // this CTA lies above rank - 1 and below rank + 1
+                if (n.down >= 0) st_async(x_down + 4u * (unsigned)(o + n.down + c), n.x[c], b_down + 8u * (2 + cur));
+                if (n.up >= 0) st_async(x_up + 4u * (unsigned)(o + n.up + c), n.x[c], b_up + 8u * cur);
             }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) sm[lay.x + o + n.nl + c] = n.x[c];
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (!from[q]) continue;
+            const unsigned bit = 2 * q + cur;
+            if (!lost) lost = !bar_wait(bar + 8u * bit, (phase >> bit) & 1u);
+            phase ^= 1u << bit;
+        }
+        __syncthreads();
+    }
+
+    // the corner forces of the CTA's elements (corner pa + 2 pb + 4 ps in slab directions)
+    __device__ void elements(int l) const {
+        const Dims& d = a.lev[l].d;
+        const int A = AXIS == 0 ? d.ny : d.nx, B = AXIS == 2 ? d.ny : d.nz, L = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;
+        const int per = (L + ctas - 1) / ctas, own = min(per, L - rank * per);
+        const int ne = own > 0 ? (own + 1) * A * B : 0;
+        const float* x = sm + lay.x + cur * lay.xlen;
+        const float2* et = reinterpret_cast<const float2*>(sm + lay.e[l]);
+        float* F = sm + lay.f[l];
+        const int sa = 3, sb = 3 * (A + 1), ss = sb * (B + 1);
+        const int sx = AXIS == 0 ? ss : sa, sy = AXIS == 1 ? ss : AXIS == 0 ? sa : sb, sz = AXIS == 2 ? ss : sb;
+        for (int e = tid; e < ne; e += TT) {
+            const float2 te = et[e];
+            if (te.x == 0.f) continue;  // its forces stay the zeros of table()
+            const int tab = __float_as_int(te.y);
+            const float* p0 = x + 3 * (tab & 0xffff);
+            V3<float> u[2][2][2];
 #pragma unroll
             for (int pz = 0; pz < 2; ++pz)
 #pragma unroll
                 for (int py = 0; py < 2; ++py)
 #pragma unroll
                     for (int px = 0; px < 2; ++px) {
-                        const int q = px + 2 * py + 4 * pz;
-                        F_[(3 * q) * ne + e] = f[px][py][pz].xy.x;
-                        F_[(3 * q + 1) * ne + e] = f[px][py][pz].xy.y;
-                        F_[(3 * q + 2) * ne + e] = f[px][py][pz].z;
+                        const float* p = p0 + px * sx + py * sy + pz * sz;
+                        u[px][py][pz].xy = make_float2(p[0], p[1]);
+                        u[px][py][pz].z = p[2];
+                    }
+            V3<float> dxb[2], dxt[2], dyb[2], dyt[2], dz[2][2], f[2][2][2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                dxb[q] = u[1][q][0] - u[0][q][0];
+                dxt[q] = u[1][q][1] - u[0][q][1];
+                dyb[q] = u[q][1][0] - u[q][0][0];
+                dyt[q] = u[q][1][1] - u[q][0][1];
+            }
+#pragma unroll
+            for (int px = 0; px < 2; ++px)
+#pragma unroll
+                for (int py = 0; py < 2; ++py) dz[px][py] = u[px][py][1] - u[px][py][0];
+            modal_element<float>(a.km, te.x, dxb, dxt, dyb, dyt, dz, f);
+            float* fo = F + FW * (tab >> 16);
+#pragma unroll
+            for (int pz = 0; pz < 2; ++pz)
+#pragma unroll
+                for (int py = 0; py < 2; ++py)
+#pragma unroll
+                    for (int px = 0; px < 2; ++px) {
+                        const int pa = AXIS == 0 ? py : px, pb = AXIS == 2 ? py : pz;
+                        const int ps = AXIS == 0 ? px : AXIS == 1 ? py : pz;
+                        const int q = pa + 2 * pb + 4 * ps;
+                        fo[3 * q] = f[px][py][pz].xy.x;
+                        fo[3 * q + 1] = f[px][py][pz].xy.y;
+                        fo[3 * q + 2] = f[px][py][pz].z;
                     }
         }
         __syncthreads();
     }
 
-    // phase 2: (K x)(n), the corners of node n's elements summed in a fixed order
-    __device__ __forceinline__ void node_force(int l, int n, float (&y)[3]) const {
-        const Dims d = lev[l].d;
-        const int ne = (int)d.ne();
-        const int pk = Nijk(l)[n];
-        const int i = pk & 2047, j = (pk >> 11) & 2047, k = pk >> 22;
-        const float* F_ = F();
+    // (K x)(n): the 8 corners that meet at the node, in a fixed order
+    __device__ void force(int l, const TailNode& n, float (&y)[3]) const {
+        const Dims& d = a.lev[l].d;
+        const int PA = (AXIS == 0 ? d.ny : d.nx) + 1, planeN = PA * ((AXIS == 2 ? d.ny : d.nz) + 1);
+        const float* F = sm + lay.f[l] + n.nb;
         y[0] = y[1] = y[2] = 0.f;
 #pragma unroll
-        for (int pz = 0; pz < 2; ++pz) {
-            const int ke = k - pz;
-            if (ke < 0 || ke >= d.nz) continue;
+        for (int q = 0; q < 8; ++q) {
+            const float* p = F - FW * ((q & 1) + ((q >> 1) & 1) * PA + (q >> 2) * planeN) + 3 * q;
 #pragma unroll
-            for (int py = 0; py < 2; ++py) {
-                const int je = j - py;
-                if (je < 0 || je >= d.ny) continue;
-#pragma unroll
-                for (int px = 0; px < 2; ++px) {
-                    const int ie = i - px;
-                    if (ie < 0 || ie >= d.nx) continue;
-                    const int e = ie + d.nx * (je + d.ny * ke);
-                    const int q = px + 2 * py + 4 * pz;
-                    y[0] += F_[(3 * q) * ne + e];
-                    y[1] += F_[(3 * q + 1) * ne + e];
-                    y[2] += F_[(3 * q + 2) * ne + e];
-                }
-            }
+            for (int c = 0; c < 3; ++c) y[c] += p[c];
         }
     }
 
-    // `deg` Chebyshev steps on level l (from x = 0 when `from_zero`)
-    __device__ void smooth(int l, int deg, bool from_zero) const {
-        const int nn = (int)lev[l].d.nn();
-        const float* cf = cheb[l];
-        float* x = X(l);
-        float* dv = Dv(l);
-        const float* b = B(l);
-        const float* g = G(l);
-        const uint8_t* m = M(l);
-        int k0 = 0;
-        if (from_zero) {  // step 0: x = d = c2_0 D^-1 b
-            const float c2 = cf[1];
-            for (int n = tid; n < nn; n += TT) {
-                const uint8_t mn = m[n];
-                const float gn = c2 * g[n];
+    // one Chebyshev step
+    __device__ void step(int l, float c1, float c2) {
+        elements(l);
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const float v = (mn >> c) & 1 ? gn * b[3 * n + c] : 0.f;
-                    x[3 * n + c] = v;
-                    dv[3 * n + c] = v;
-                }
-            }
-            __syncthreads();
-            k0 = 1;
-        }
-        for (int k = k0; k < deg; ++k) {
-            element_forces(l);
-            const float c1 = (k == 0) ? 0.f : cf[2 * k], c2 = cf[2 * k + 1];
-            for (int n = tid; n < nn; n += TT) {
-                const uint8_t mn = m[n];
-                if (!(mn & 7)) continue;
-                float y[3];
-                node_force(l, n, y);
-                const float gn = c2 * g[n];
+        for (int r = 0; r < NPT; ++r) {
+            TailNode& n = nd[r];
+            if (n.m == 0) continue;
+            float y[3];
+            force(l, n, y);
+            const float gn = c2 * n.g;
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    if ((mn >> c) & 1) {
-                        const int q = 3 * n + c;
-                        const float dn = c1 * dv[q] + (b[q] - y[c]) * gn;
-                        dv[q] = dn;
-                        x[q] += dn;
-                    }
-                }
+            for (int c = 0; c < 3; ++c) {
+                const float dn = (n.m >> c) & 1 ? c1 * n.d[c] + (n.b[c] - y[c]) * gn : 0.f;
+                n.d[c] = dn;
+                n.x[c] += dn;
             }
-            __syncthreads();
         }
+        exchange(l);
     }
+};
 
-    // Dv(l) = b - K x (masked): the residual restricted to level l + 1 (the post-smoothing's
-    // first step does not read the direction)
-    __device__ void residual(int l) const {
-        element_forces(l);
-        const int nn = (int)lev[l].d.nn();
-        float* r = Dv(l);
-        const float* b = B(l);
-        const uint8_t* m = M(l);
-        for (int n = tid; n < nn; n += TT) {
-            const uint8_t mn = m[n];
+template <int AXIS>
+__global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArgs a) {
+    extern __shared__ __align__(16) float tail_smem[];
+    __shared__ TailLayout lay;
+    __shared__ float cf[kTailMaxLevels][2 * kTailMaxDegree];
+    __shared__ __align__(8) uint64_t bars[2][2];
+    const int tid = threadIdx.x, ctas = a.ctas;
+    const int rank = blockIdx.x % ctas, slot = blockIdx.x / ctas;
+    const int* done = slot_bytes(a.done, slot, a.sc_bytes);
+    if (done != nullptr && *done) return;  // the same for the whole cluster
+    const int last = a.nlev - 1;
+    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&bars[0][0]);
+    if (tid == 0) {
+        lay = tail_layout<AXIS>(a.lev, a.nlev, ctas);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8u * q) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int q = tid; q < last * 2 * kTailMaxDegree; q += TT) {
+        const int l = q / (2 * kTailMaxDegree), k = q - l * 2 * kTailMaxDegree;
+        if (k < 2 * a.lev[l].degree) cf[l][k] = (float)a.lev[l].cheb[k];
+    }
+    __syncthreads();
+    Tail<AXIS> t{a, lay, tail_smem, bar, 0, 0, 0, 0, tid, rank, ctas, slot};
+    {
+        const uint32_t xb = (uint32_t)__cvta_generic_to_shared(tail_smem + lay.x);
+        const int below = rank > 0 ? rank - 1 : 0, above = rank + 1 < ctas ? rank + 1 : rank;
+        t.x_down = map_rank(xb, below);
+        t.x_up = map_rank(xb, above);
+        t.b_down = map_rank(bar, below);
+        t.b_up = map_rank(bar, above);
+    }
+    for (int l = 0; l < last; ++l) t.table(l);
+    cluster_sync();  // every CTA's barriers are ready before its shared memory is written
+
+    for (int l = 0; l < last; ++l) {  // down: smooth from zero, residual
+        const int deg = a.lev[l].degree;
+        float* save = tail_smem + lay.save[l];
+        t.enter(l);
+#pragma unroll
+        for (int r = 0; r < NPT; ++r) {
+            TailNode& n = t.nd[r];
+            if (n.t < 0) continue;
+            if (l == 0) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) n.b[c] = __ldg(t.vec(a.b0, 0) + 3 * n.gn + c);
+            } else {
+                restrict_at<3>(a.lev[l - 1].d, t.vec(a.lev[l - 1].r, l - 1), n.i, n.j, n.k, 0, n.b);
+            }
+            const float gn = cf[l][1] * n.g;  // step 0: x = d = c2_0 D^-1 b
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if (!((n.m >> c) & 1)) n.b[c] = 0.f;
+                n.x[c] = n.d[c] = gn * n.b[c];
+                save[6 * n.t + c] = n.b[c];
+            }
+        }
+        t.exchange(l);
+        for (int k = 1; k < deg; ++k) t.step(l, cf[l][2 * k], cf[l][2 * k + 1]);
+        t.elements(l);
+        float* res = t.vec(a.lev[l].r, l);
+#pragma unroll
+        for (int r = 0; r < NPT; ++r) {
+            const TailNode& n = t.nd[r];
+            if (n.t < 0) continue;
             float y[3] = {0.f, 0.f, 0.f};
-            if (mn & 7) node_force(l, n, y);
+            if (n.m) t.force(l, n, y);
 #pragma unroll
-            for (int c = 0; c < 3; ++c) r[3 * n + c] = (mn >> c) & 1 ? b[3 * n + c] - y[c] : 0.f;
-        }
-        __syncthreads();
-    }
-
-    // B(l + 1) = P^T Dv(l): trilinear weights 1, 1/2, 1/4, 1/8, zero on fixed coarse DOFs
-    __device__ void restrict_to(int l) const {
-        const Dims f = lev[l].d, c = lev[l + 1].d;
-        const float* r = Dv(l);
-        float* bc = B(l + 1);
-        const uint8_t* mc = M(l + 1);
-        const int cnn = (int)c.nn();
-        const int fsy = f.nx + 1, fsz = (f.nx + 1) * (f.ny + 1);
-        const int cx = c.nx + 1, cxy = (c.nx + 1) * (c.ny + 1);
-        for (int N = tid; N < cnn; N += TT) {
-            const uint8_t m = mc[N];
-            if (!(m & 7)) {
-                bc[3 * N] = bc[3 * N + 1] = bc[3 * N + 2] = 0.f;
-                continue;
+            for (int c = 0; c < 3; ++c) {
+                res[3 * n.gn + c] = (n.m >> c) & 1 ? n.b[c] - y[c] : 0.f;
+                save[6 * n.t + 3 + c] = n.x[c];
             }
-            const int K = N / cxy, J = (N - K * cxy) / cx, I = N - K * cxy - J * cx;
-            float acc[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-            for (int dk = -1; dk <= 1; ++dk) {
-                const int k = 2 * K + dk;
-                if (k < 0 || k > f.nz) continue;
-                const float wk = dk == 0 ? 1.f : 0.5f;
-#pragma unroll
-                for (int dj = -1; dj <= 1; ++dj) {
-                    const int j = 2 * J + dj;
-                    if (j < 0 || j > f.ny) continue;
-                    const float wj = dj == 0 ? wk : 0.5f * wk;
-#pragma unroll
-                    for (int di = -1; di <= 1; ++di) {
-                        const int i = 2 * I + di;
-                        if (i < 0 || i > f.nx) continue;
-                        const float w = di == 0 ? wj : 0.5f * wj;
-                        const float* p = r + 3 * (i + fsy * j + fsz * k);
-                        acc[0] += w * p[0];
-                        acc[1] += w * p[1];
-                        acc[2] += w * p[2];
-                    }
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < 3; ++q) bc[3 * N + q] = (m >> q) & 1 ? acc[q] : 0.f;
         }
-        __syncthreads();
+        cluster_sync();
     }
 
-    // X(l) += P X(l + 1) on free fine DOFs
-    __device__ void prolong_add(int l) const {
-        const Dims f = lev[l].d, c = lev[l + 1].d;
-        const float* xc = X(l + 1);
-        float* xf = X(l);
-        const uint8_t* mf = M(l);
-        const int* nijk = Nijk(l);
-        const int fnn = (int)f.nn();
-        const int csy = c.nx + 1, csz = (c.nx + 1) * (c.ny + 1);
-        for (int n = tid; n < fnn; n += TT) {
-            const uint8_t m = mf[n];
-            if (!(m & 7)) continue;
-            const int pk = nijk[n];
-            const int i = pk & 2047, j = (pk >> 11) & 2047, k = pk >> 22;
-            const int I = i >> 1, J = j >> 1, K = k >> 1, di = i & 1, dj = j & 1, dk = k & 1;
-            const float w = (di ? 0.5f : 1.f) * (dj ? 0.5f : 1.f) * (dk ? 0.5f : 1.f);
-            float acc[3] = {0.f, 0.f, 0.f};
-            for (int g = 0; g <= dk; ++g)
-                for (int bb = 0; bb <= dj; ++bb)
-                    for (int aa = 0; aa <= di; ++aa) {
-                        const float* p = xc + 3 * ((I + aa) + csy * (J + bb) + csz * (K + g));
-                        acc[0] += p[0];
-                        acc[1] += p[1];
-                        acc[2] += p[2];
-                    }
-#pragma unroll
-            for (int q = 0; q < 3; ++q)
-                if ((m >> q) & 1) xf[3 * n + q] += w * acc[q];
+    {  // the coarsest grid: its right-hand side in every CTA, the rows of the inverse shared out
+        const Dims d = a.lev[last].d;
+        float* bc = tail_smem + lay.c;
+        const float* rf = t.vec(a.lev[last - 1].r, last - 1);
+        for (int q = tid; q < 3 * (int)d.nn(); q += TT) {
+            const int N = q / 3, c = q - 3 * N;
+            const int K = N / ((d.nx + 1) * (d.ny + 1)), J = N / (d.nx + 1) % (d.ny + 1), I = N % (d.nx + 1);
+            const unsigned m = __ldg(a.lev[last].nmask + N);
+            float v[1];
+            restrict_at<1>(a.lev[last - 1].d, rf, I, J, K, c, v);
+            bc[q] = (m >> c) & 1 ? v[0] : 0.f;
         }
         __syncthreads();
-    }
-
-    // X(L) = A^-1 B(L) on the coarsest grid: the inverse as float pairs, one warp per row (the
-    // inverse is symmetric: lane t reads entries t, t + 32, ... of column `row`), compensated
-    // FP32 accumulation, the lanes' pairs added in a fixed tree
-    __device__ void coarse_solve(int l) const {
-        const int n = nc;
-        const float* b = B(l);
-        float* x = X(l);
-        const uint8_t* m = M(l);
-        const int lane = tid & 31, warp = tid >> 5;
-        for (int row = warp; row < n; row += TT / 32) {
+        const int n = a.nc, lane = tid & 31;
+        float* xc = t.vec(a.lev[last].x, last);
+        for (int row = rank * (TT / 32) + (tid >> 5); row < n; row += ctas * (TT / 32)) {
+            // one warp per row, compensated FP32 sums, the lanes' pairs added in a fixed tree
+            const float* hi = a.ainv_hi + (int64_t)row * n;
+            const float* lo = a.ainv_lo + (int64_t)row * n;
             Acc2 acc;
-            const float* hi = ainv_hi + (int64_t)row * n;
-            const float* lo = ainv_lo + (int64_t)row * n;
+#pragma unroll 4
             for (int c = lane; c < n; c += 32) {
-                if (!ANL_IN_RANGE((int64_t)row * n + c, (int64_t)n * n)) break;
-                const float bc = b[c];
-                acc.add_prod(__ldg(hi + c), bc);
-                acc.add_prod(__ldg(lo + c), bc);
+                const float h = __ldg(hi + c), q = __ldg(lo + c), b = bc[c];
+                acc.add_prod(h, b);
+                acc.add_prod(q, b);
             }
             float s = acc.s, e = acc.c;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 const float s2 = __shfl_down_sync(0xffffffffu, s, o), e2 = __shfl_down_sync(0xffffffffu, e, o);
-                float t, f;
-                two_sum(s, s2, t, f);
-                s = t;
+                float v, f;
+                two_sum(s, s2, v, f);
+                s = v;
                 e += e2 + f;
             }
-            if (lane == 0) x[row] = (m[row / 3] >> (row % 3)) & 1 ? s + e : 0.f;
+            if (lane == 0) xc[row] = (__ldg(a.lev[last].nmask + row / 3) >> (row % 3)) & 1 ? s + e : 0.f;
         }
-        __syncthreads();
+        cluster_sync();
     }
-};
 
-__global__ void __launch_bounds__(TT, 1) k_vtail(TailArgs a) {
-    const int slot = blockIdx.x;
-    const int* done = slot_bytes(a.done, slot, a.sc_bytes);
-    if (done != nullptr && *done) return;
-    const float* b0 = slot_ptr(a.b0, slot, a.vstride);
-    float* x0 = slot_ptr(a.x0, slot, a.vstride);
-    extern __shared__ __align__(16) float tail_smem[];
-    __shared__ TailLevel slev[kTailMaxLevels];
-    const int tid = threadIdx.x;
+    for (int l = last - 1; l >= 0; --l) {  // up: add the correction, smooth
+        const int deg = a.lev[l].degree;
+        const float* save = tail_smem + lay.save[l];
+        t.enter(l);
+        const float* xc = t.vec(a.lev[l + 1].x, l + 1);
 #pragma unroll
-    for (int q = 0; q < kTailMaxLevels; ++q)  // static indices: the parameter stays in its bank
-        if (tid == q) slev[q] = a.lev[q];
-    __shared__ TailLayout sL;
-    __shared__ float scheb[kTailMaxLevels][2 * kTailMaxDegree];
-    __syncthreads();
-    if (tid == 0) sL = tail_layout(slev, a.nlev);
-    {  // the sweeps' coefficients: a dependent global load per step otherwise
-        const int l = tid / (2 * kTailMaxDegree), q = tid % (2 * kTailMaxDegree);
-        if (l < a.nlev - 1 && q < 2 * a.degree) scheb[l][q] = (float)slev[l].cheb[q];
-    }
-    __syncthreads();
-    const TailCtx t{slev, sL, scheb, tail_smem, tid, a.km, a.ainv_hi, a.ainv_lo, a.nc};
-    // the levels' element scales, inverse diagonals, masks and index tables, and the first
-    // level's b
-    for (int l = 0; l < a.nlev; ++l) {
-        const TailLevel& lv = slev[l];
-        const Dims d = lv.d;
-        const int nn = (int)d.nn(), ne = (int)d.ne();
-        for (int q = tid; q < nn; q += TT) t.M(l)[q] = lv.nmask[q];
-        if (l < a.nlev - 1) {
-            for (int q = tid; q < ne; q += TT) {
-                t.E(l)[q] = lv.E[q];
-                const int i = q % d.nx, j = (q / d.nx) % d.ny, k = q / (d.nx * d.ny);
-                t.E0(l)[q] = (int)d.node(i, j, k);
-            }
-            for (int q = tid; q < nn; q += TT) {
-                t.G(l)[q] = lv.diag[q];
-                const int i = q % (d.nx + 1), j = (q / (d.nx + 1)) % (d.ny + 1), k = q / ((d.nx + 1) * (d.ny + 1));
-                t.Nijk(l)[q] = pack_ijk(i, j, k);
+        for (int r = 0; r < NPT; ++r) {
+            TailNode& n = t.nd[r];
+            if (n.t < 0) continue;
+            float p[3];
+            prolong_at(a.lev[l + 1].d, xc, n.i, n.j, n.k, p);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                n.b[c] = save[6 * n.t + c];
+                n.x[c] = save[6 * n.t + 3 + c] + ((n.m >> c) & 1 ? p[c] : 0.f);
             }
         }
+        t.exchange(l);
+        for (int k = 0; k < deg; ++k) t.step(l, k == 0 ? 0.f : cf[l][2 * k], cf[l][2 * k + 1]);
+        float* xo = t.vec(a.lev[l].x, l);
+#pragma unroll
+        for (int r = 0; r < NPT; ++r) {
+            const TailNode& n = t.nd[r];
+            if (n.t < 0) continue;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) xo[3 * n.gn + c] = t.lost ? NAN : n.x[c];  // a lost halo fails the solve
+        }
+        cluster_sync();  // the coarse correction is written; at the end no CTA leaves before its neighbours' stores
     }
-    {
-        const int nn = (int)slev[0].d.nn();
-        for (int q = tid; q < 3 * nn; q += TT) t.B(0)[q] = b0[q];
+}
+
+int tail_axis(const Dims& d) { return d.nx >= d.ny && d.nx >= d.nz ? 0 : d.ny >= d.nz ? 1 : 2; }
+
+template <int AXIS>
+bool tail_fits(const TailLevel* lev, int nlev, int ctas, size_t* bytes) {
+    for (int l = 0; l < nlev - 1; ++l) {
+        const Slab<AXIS> g(lev[l].d, 0, ctas);
+        if (lev[l].degree < 1 || lev[l].degree > kTailMaxDegree) return false;
+        if (g.planeN > TT * NPT || g.max_nodes() > TT * NPT || g.max_padded() > 0x7fff) return false;
+        if (g.max_nodes() + 2 * g.planeN > 0xffff) return false;
     }
-    __syncthreads();
-    const int last = a.nlev - 1;
-    for (int l = 0; l < last; ++l) {
-        t.smooth(l, a.degree, true);
-        t.residual(l);
-        t.restrict_to(l);
-    }
-    t.coarse_solve(last);
-    for (int l = last - 1; l >= 0; --l) {
-        t.prolong_add(l);
-        t.smooth(l, a.degree, false);
-    }
-    const int nn = (int)slev[0].d.nn();
-    for (int q = tid; q < 3 * nn; q += TT) x0[q] = t.X(0)[q];
+    *bytes = sizeof(float) * (size_t)tail_layout<AXIS>(lev, nlev, ctas).words;
+    return *bytes <= (size_t)kTailMaxSmem;
+}
+
+cudaLaunchConfig_t tail_config(int ctas, int nrhs, size_t bytes, cudaStream_t s, cudaLaunchAttribute* attr) {
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)ctas;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(ctas * nrhs));
+    cfg.blockDim = dim3(TT);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+template <int AXIS>
+int tail_prepare_axis() {
+    ANL_CUDA(cudaFuncSetAttribute(k_vtail<AXIS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailMaxSmem));
+    ANL_CUDA(cudaFuncSetAttribute(k_vtail<AXIS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    return ANL_OK;
 }
 
 }  // namespace
 
-size_t tail_smem_bytes(const TailLevel* lev, int nlev) { return sizeof(float) * (size_t)tail_layout(lev, nlev).words; }
-
-int vtail_prepare() {
-    static bool done = false;
-    if (!done) {
-        ANL_CUDA(cudaFuncSetAttribute(k_vtail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailMaxSmem));
-        done = true;
+// CTAs of the tail's cluster: 16 where the device can place such a cluster with the largest
+// shared memory, else 8 (the portable size).
+int vtail_prepare(int* ctas) {
+    static int n = 0;
+    if (n == 0) {
+        ANL_TRY(tail_prepare_axis<0>());
+        ANL_TRY(tail_prepare_axis<1>());
+        ANL_TRY(tail_prepare_axis<2>());
+        cudaLaunchAttribute attr;
+        cudaLaunchConfig_t cfg = tail_config(16, 1, kTailMaxSmem, nullptr, &attr);
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, k_vtail<0>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            fit = 0;
+        }
+        n = fit >= 1 ? 16 : 8;
     }
+    *ctas = n;
     return ANL_OK;
 }
 
+bool vtail_fits(const TailLevel* lev, int nlev, int ctas) {
+    size_t bytes = 0;
+    switch (tail_axis(lev[0].d)) {
+        case 0: return tail_fits<0>(lev, nlev, ctas, &bytes);
+        case 1: return tail_fits<1>(lev, nlev, ctas, &bytes);
+        default: return tail_fits<2>(lev, nlev, ctas, &bytes);
+    }
+}
+
 int launch_vtail(const TailArgs& a, cudaStream_t s) {
-    const size_t bytes = tail_smem_bytes(a.lev, a.nlev);
-    if (a.degree > kTailMaxDegree || a.nlev > kTailMaxLevels || bytes > (size_t)kTailMaxSmem || a.lev[0].d.ne() > 1024 || a.lev[0].d.nx > 2047 || a.lev[0].d.ny > 2047 ||
-        a.lev[0].d.nz > 1023) {
-        set_error("V-cycle tail: %zu bytes of shared memory or %lld elements exceed one CTA", bytes,
-                  (long long)a.lev[0].d.ne());
+    const int axis = tail_axis(a.lev[0].d);
+    size_t bytes = 0;
+    const bool ok = a.nlev >= 2 && a.nlev <= kTailMaxLevels &&
+                    (axis == 0 ? tail_fits<0>(a.lev, a.nlev, a.ctas, &bytes)
+                               : axis == 1 ? tail_fits<1>(a.lev, a.nlev, a.ctas, &bytes)
+                                           : tail_fits<2>(a.lev, a.nlev, a.ctas, &bytes));
+    if (!ok) {
+        set_error("V-cycle tail: the levels exceed one cluster of %d CTAs", a.ctas);
         return ANL_ERR_BADARG;
     }
-    k_vtail<<<std::max(1, a.nrhs), TT, bytes, s>>>(a);
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg = tail_config(a.ctas, std::max(1, a.nrhs), bytes, s, &attr);
+    switch (axis) {
+        case 0: ANL_CUDA(cudaLaunchKernelEx(&cfg, k_vtail<0>, a)); break;
+        case 1: ANL_CUDA(cudaLaunchKernelEx(&cfg, k_vtail<1>, a)); break;
+        default: ANL_CUDA(cudaLaunchKernelEx(&cfg, k_vtail<2>, a)); break;
+    }
     ANL_LAUNCH_CHECK();
     return ANL_OK;
 }
