@@ -35,7 +35,9 @@ struct DotAcc<DF> {  // the accurate residual: ||r||^2 of its FP32 values, compe
 
 // KU_CHEB0: the first two Chebyshev steps from x = 0 in one pass: x1 = c2_0 D^-1 b is formed
 // on the fly from the staged b and diagonal, then x2 = x1 + c1_1 x1 + c2_1 D^-1 (b - K x1)
-enum { KU_APPLY = 0, KU_APPLY_DOT = 1, KU_RESID = 2, KU_CHEB = 3, KU_CHEB0 = 4 };
+// KU_APPLY_RAW: the caller's K u in one pass: u is masked and the element scale formed while they
+// are staged (E = active ? h escale : 0, also stored for the context), then as KU_APPLY
+enum { KU_APPLY = 0, KU_APPLY_DOT = 1, KU_RESID = 2, KU_CHEB = 3, KU_CHEB0 = 4, KU_APPLY_RAW = 5 };
 
 template <class T>
 struct KuArgs {
@@ -56,6 +58,9 @@ struct KuArgs {
     int dv_keep = 1;                 // CHEB, CHEB0: 0 on the last step of a sweep (d is not stored)
     const double* cheb0 = nullptr;   // CHEB0: {c1_0, c2_0} of the step from x = 0
     const float* diag = nullptr;     // CHEB, CHEB0: inverse diagonal of K per node (0 where unused)
+    const uint8_t* active = nullptr; // APPLY_RAW: active flags; E is then the caller's escale
+    float hscale = 0.f;              // APPLY_RAW: h
+    float* Eout = nullptr;           // APPLY_RAW: receives the context's element scale
     T kdiag = T(0);                  // diagonal entry of Ke(1) (all 24 are equal)
     double* partials = nullptr;      // APPLY_DOT reduction scratch
     unsigned* counter = nullptr;

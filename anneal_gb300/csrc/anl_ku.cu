@@ -102,6 +102,7 @@ struct KuEpi {
     uint8_t nm;
     T b[3], dv[3];
     float dg;  // CHEB: the inverse diagonal of the output node (level's diag array)
+    uint8_t m[2], act;  // APPLY_RAW: masks of the own nodes above the output node, the element's flag
 };
 
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, bool valid) {
@@ -150,7 +151,7 @@ struct KuTile {
     T c1s = T(0), c2s = T(0); // CHEB, CHEB0: the step's coefficients (read and converted once)
     const float* iD = nullptr;
     // segment geometry
-    bool r0in, rNin, ein, owner;
+    bool r0in, r1in, rNin, ein, owner;
     int64_t n0, e0;
     // staging cursor: next layer ik; sources of node plane ik + 1 and element layer ik
     int ik;
@@ -182,6 +183,7 @@ struct KuTile {
         const int ie = bx * KmCfg<T>::OX - 1 + lane, je = by * KmCfg<T>::OY - 1 + w;
         const bool xin = ie >= 0 && ie < NXn;
         r0in = xin && je >= 0 && je < NYn;
+        r1in = xin && je + 1 >= 0 && je + 1 < NYn;
         rNin = xin && by * KmCfg<T>::OY - 1 + NW < NYn;  // the extra row of the last warp
         ein = ie >= 0 && ie < a.d.nx && je >= 0 && je < a.d.ny;
         owner = lane >= 1 && lane <= KmCfg<T>::OX && w >= 1 && xin && je < NYn;
@@ -256,9 +258,29 @@ struct KuTile {
         }
     }
 
+    // APPLY_RAW: the masks of this thread's two nodes of plane pk, whose node (ie, je) is n
+    __device__ __forceinline__ void raw_masks(int64_t n, int pk, uint8_t (&m)[2]) const {
+        const bool kin = pk >= 0 && pk < NZn;
+        m[0] = kin && r0in && ANL_IN_RANGE(n, plane * NZn) ? __ldg(a.nmask + n) : uint8_t(0);
+        m[1] = kin && r1in && ANL_IN_RANGE(n + NXn, plane * NZn) ? __ldg(a.nmask + n + NXn) : uint8_t(0);
+    }
+    __device__ __forceinline__ void raw_apply(const uint8_t (&m)[2], V3<T> (&u)[2]) const {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            if (!(m[r] & 1)) u[r].xy.x = T(0);
+            if (!(m[r] & 2)) u[r].xy.y = T(0);
+            if (!(m[r] & 4)) u[r].z = T(0);
+        }
+    }
+
     // epilogue loads of output node n (plane kk)
-    __device__ __forceinline__ void epi_load(int64_t n, bool emit, KuEpi<T>& e) const {
+    __device__ __forceinline__ void epi_load(int64_t n, int kk, bool emit, KuEpi<T>& e) const {
         e.nm = 0;
+        if (MODE == KU_APPLY_RAW) {
+            raw_masks(n + plane, kk + 1, e.m);
+            const int64_t el = e0 + (int64_t)kk * eplane;
+            e.act = ein && kk >= 0 && kk < a.d.nz && ANL_IN_RANGE(el, eplane * a.d.nz) ? __ldg(a.active + el) : uint8_t(0);
+        }
         if (emit && ANL_IN_RANGE(n, plane * NZn)) {
             e.nm = __ldg(a.nmask + n);
             if (MODE == KU_RESID || MODE == KU_CHEB) {  // CHEB0 has b staged already
@@ -274,8 +296,13 @@ struct KuTile {
     }
 
     // carry of the node plane staged in `slot` (edge differences only, no forces yet)
-    __device__ __forceinline__ void start(int slot, KuCarry<T>& c) const {
+    __device__ __forceinline__ void start(int slot, KuCarry<T>& c, int64_t n, int k) const {
         node_pair(slot, c.ub, &c.braw, &c.dg);
+        if (MODE == KU_APPLY_RAW) {
+            uint8_t m[2];
+            raw_masks(n, k, m);
+            raw_apply(m, c.ub);
+        }
         const V3<T> nb0 = shfl_down3(c.ub[0]), nb1 = shfl_down3(c.ub[1]);
         c.dxb[0] = nb0 - c.ub[0];
         c.dxb[1] = nb1 - c.ub[1];
@@ -292,10 +319,16 @@ struct KuTile {
                                          KuCarry<T>& o, const KuEpi<T>& ep, KuEpi<T>& epn, DotAcc<T>& dot) {
         const int slot = kk & (KU_RING - 1);
         issue_next(kend);
-        epi_load(n + plane, owner && kk + 1 < kend, epn);
+        epi_load(n + plane, kk + 1, owner && kk + 1 < kend, epn);
         V3<T> cu[2];
         node_pair(slot, cu, &o.braw, &o.dg);
-        const float Ee = sm.E[slot][w][lane];
+        float Ee = sm.E[slot][w][lane];
+        if (MODE == KU_APPLY_RAW) {
+            raw_apply(ep.m, cu);
+            Ee = ep.act ? a.hscale * Ee : 0.f;
+            // the owner of node (ie, je, kk) stores its element
+            if (emit && owner && ein && kk < a.d.nz) a.Eout[e0 + (int64_t)kk * eplane] = Ee;
+        }
         // edge differences of the upper plane
         const V3<T> un0 = shfl_down3(cu[0]), un1 = shfl_down3(cu[1]);
         o.dxb[0] = un0 - cu[0];
@@ -349,7 +382,7 @@ struct KuTile {
             const T b[3] = {MODE == KU_CHEB0 ? in.braw.xy.x : ep.b[0], MODE == KU_CHEB0 ? in.braw.xy.y : ep.b[1],
                             MODE == KU_CHEB0 ? in.braw.z : ep.b[2]};
             const uint8_t nm = ep.nm;
-            if (MODE == KU_APPLY || MODE == KU_APPLY_DOT) {
+            if (MODE == KU_APPLY || MODE == KU_APPLY_DOT || MODE == KU_APPLY_RAW) {
                 T* yp = a.y + 3 * n;
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
@@ -431,9 +464,9 @@ __global__ void __launch_bounds__(KmCfg<T>::NT, KmCfg<T>::MINB) ku_kernel(KuArgs
         __syncthreads();
         KuCarry<T> A, B;
         KuEpi<T> EA, EB;
-        t.start((k0 - 2) & (KU_RING - 1), A);
         int64_t n = t.n0 + (int64_t)(k0 - 1) * t.plane;  // node (ie, je, kk)
-        t.epi_load(n, false, EA);
+        t.start((k0 - 2) & (KU_RING - 1), A, n, k0 - 1);
+        t.epi_load(n, k0 - 1, false, EA);
         __syncthreads();  // slot of layer k0-2 is read before the loop refills it
         if constexpr (std::is_same<T, DF>::value) {
             // one step per trip and the carries copied: the pair arithmetic of a step is long
@@ -496,11 +529,13 @@ void ku_prepare() {
     ku_resident<float, KU_RESID>();
     ku_resident<float, KU_CHEB>();
     ku_resident<float, KU_CHEB0>();
+    ku_resident<float, KU_APPLY_RAW>();
     ku_resident<double, KU_APPLY>();
     ku_resident<double, KU_APPLY_DOT>();
     ku_resident<double, KU_RESID>();
     ku_resident<double, KU_CHEB>();
     ku_resident<double, KU_CHEB0>();
+    ku_resident<double, KU_APPLY_RAW>();
     ku_resident<DF, KU_RESID>();
 }
 
@@ -517,6 +552,7 @@ int launch_ku(int mode, const KuArgs<T>& args, const KeModal<T>& km, cudaStream_
         case KU_RESID: resident = ku_resident<T, KU_RESID>(); break;
         case KU_CHEB: resident = ku_resident<T, KU_CHEB>(); break;
         case KU_CHEB0: resident = ku_resident<T, KU_CHEB0>(); break;
+        case KU_APPLY_RAW: resident = ku_resident<T, KU_APPLY_RAW>(); break;
         default: return ANL_ERR_BADARG;
     }
     // one wave of CTAs per right-hand side. A segment costs one extra element layer, but a
@@ -538,6 +574,7 @@ int launch_ku(int mode, const KuArgs<T>& args, const KeModal<T>& km, cudaStream_
         case KU_RESID: ku_kernel<T, KU_RESID><<<grid, block, sizeof(KuSmem<T, KU_RESID>), s>>>(a, km); break;
         case KU_CHEB: ku_kernel<T, KU_CHEB><<<grid, block, sizeof(KuSmem<T, KU_CHEB>), s>>>(a, km); break;
         case KU_CHEB0: ku_kernel<T, KU_CHEB0><<<grid, block, sizeof(KuSmem<T, KU_CHEB0>), s>>>(a, km); break;
+        case KU_APPLY_RAW: ku_kernel<T, KU_APPLY_RAW><<<grid, block, sizeof(KuSmem<T, KU_APPLY_RAW>), s>>>(a, km); break;
         default: return ANL_ERR_BADARG;
     }
     ANL_LAUNCH_CHECK();
