@@ -278,48 +278,46 @@ __host__ __device__ __forceinline__ T modal_energy(const KeModal<T>& k, const V3
     return e;
 }
 
+// The modal forces g1..g7 of the amplitudes b1..b7: the sparse modal stiffness, scaled by E (g0 is
+// zero: the rigid translations carry no force).
+#pragma nv_exec_check_disable
+template <class T>
+__host__ __device__ __forceinline__ void modal_forces(const KeModal<T>& k, T E, const V3<T> (&b)[8], V3<T> (&g)[8]) {
+    const T ab = E * k.ab, bb = E * k.b, cc = E * k.c, dd = E * k.d, ff = E * k.f, gh = E * k.gh, hh = E * k.h,
+            jj = E * k.j;
+    const T tr = bb * (b[1].xy.x + b[2].xy.y + b[3].z);
+    g[1].xy.x = ab * b[1].xy.x + tr;
+    g[2].xy.y = ab * b[2].xy.y + tr;
+    g[3].z = ab * b[3].z + tr;
+    g[1].xy.y = g[2].xy.x = cc * (b[1].xy.y + b[2].xy.x);
+    g[1].z = g[3].xy.x = cc * (b[1].z + b[3].xy.x);
+    g[2].z = g[3].xy.y = cc * (b[2].z + b[3].xy.y);
+    g[4].xy.x = dd * b[4].xy.x + ff * b[5].z;
+    g[5].z = ff * b[4].xy.x + dd * b[5].z;
+    g[4].xy.y = dd * b[4].xy.y + ff * b[6].z;
+    g[6].z = ff * b[4].xy.y + dd * b[6].z;
+    g[5].xy.y = dd * b[5].xy.y + ff * b[6].xy.x;
+    g[6].xy.x = ff * b[5].xy.y + dd * b[6].xy.x;
+    const T s3 = hh * (b[4].z + b[5].xy.x + b[6].xy.y);
+    g[4].z = gh * b[4].z + s3;
+    g[5].xy.x = gh * b[5].xy.x + s3;
+    g[6].xy.y = gh * b[6].xy.y + s3;
+    g[7] = jj * b[7];
+}
+
 #pragma nv_exec_check_disable
 template <class T>
 __host__ __device__ __forceinline__ void modal_element(const KeModal<T>& k, T E, const V3<T> (&dxb)[2],
                                                        const V3<T> (&dxt)[2], const V3<T> (&dyb)[2],
                                                        const V3<T> (&dyt)[2], const V3<T> (&dz)[2][2],
                                                        V3<T> (&f)[2][2][2]) {
-    // mode amplitudes (Walsh-Hadamard transform through the edges)
-    V3<T> bm[8];
-    modal_amplitudes<T>(dxb, dxt, dyb, dyt, dz, bm);
-    const V3<T>& b1 = bm[1];
-    const V3<T>& b2 = bm[2];
-    const V3<T>& b3 = bm[3];
-    const V3<T>& b4 = bm[4];
-    const V3<T>& b5 = bm[5];
-    const V3<T>& b6 = bm[6];
-    const V3<T>& b7 = bm[7];
-    // the sparse modal stiffness, scaled by E
-    const T ab = E * k.ab, bb = E * k.b, cc = E * k.c, dd = E * k.d, ff = E * k.f, gh = E * k.gh, hh = E * k.h,
-            jj = E * k.j;
-    V3<T> g1, g2, g3, g4, g5, g6;
-    const T tr = b1.xy.x + b2.xy.y + b3.z;
-    g1.xy.x = ab * b1.xy.x + bb * tr;
-    g2.xy.y = ab * b2.xy.y + bb * tr;
-    g3.z = ab * b3.z + bb * tr;
-    g1.xy.y = g2.xy.x = cc * (b1.xy.y + b2.xy.x);
-    g1.z = g3.xy.x = cc * (b1.z + b3.xy.x);
-    g2.z = g3.xy.y = cc * (b2.z + b3.xy.y);
-    g4.xy.x = dd * b4.xy.x + ff * b5.z;
-    g5.z = ff * b4.xy.x + dd * b5.z;
-    g4.xy.y = dd * b4.xy.y + ff * b6.z;
-    g6.z = ff * b4.xy.y + dd * b6.z;
-    g5.xy.y = dd * b5.xy.y + ff * b6.xy.x;
-    g6.xy.x = ff * b5.xy.y + dd * b6.xy.x;
-    const T s3 = b4.z + b5.xy.x + b6.xy.y;
-    g4.z = gh * b4.z + hh * s3;
-    g5.xy.x = gh * b5.xy.x + hh * s3;
-    g6.xy.y = gh * b6.xy.y + hh * s3;
-    const V3<T> g7 = jj * b7;
+    V3<T> b[8], g[8];
+    modal_amplitudes<T>(dxb, dxt, dyb, dyt, dz, b);
+    modal_forces<T>(k, E, b, g);
     // back to the corners: f(p) = sum_m s_m(p) g_m = A(py,pz) + sx B(py,pz)
-    const V3<T> am = g2 - g5, ap = g2 + g5;
-    const V3<T> n00 = am + g3, a10 = am - g3, a01 = g3 - ap, a11 = ap + g3;  // A(0,0) = -n00
-    const V3<T> cm = g1 - g6, cp = g1 + g6, dm = g4 - g7, dp = g4 + g7;
+    const V3<T> am = g[2] - g[5], ap = g[2] + g[5];
+    const V3<T> n00 = am + g[3], a10 = am - g[3], a01 = g[3] - ap, a11 = ap + g[3];  // A(0,0) = -n00
+    const V3<T> cm = g[1] - g[6], cp = g[1] + g[6], dm = g[4] - g[7], dp = g[4] + g[7];
     const V3<T> q00 = cm - dm, q10 = cm + dm, q01 = cp - dp, q11 = cp + dp;
     f[0][0][0] = v3zero<T>() - (n00 + q00);
     f[1][0][0] = q00 - n00;
