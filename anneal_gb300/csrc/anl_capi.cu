@@ -253,6 +253,7 @@ static void free_ctx(anl_ctx* c) {
     f(c->y1);
     f(c->y2);
     f(c->tmp);
+    f(c->f64);
     f(c->xbuf);
     f(c->bbuf);
     f(c->sc);
@@ -394,10 +395,19 @@ static int create(anl_ctx** out, int nx, int ny, int nz, double h, double nu, in
     ALLOC(c->y1, 3 * nn * ts);
     ALLOC(c->y2, 3 * nn * ts);
     ALLOC(c->tmp, 3 * nn * ts);
+    if (c->fp64) {
+        int64_t most = 0;
+        for (auto& L : c->lev) {
+            L.split = ku_prefers_split(L.d);
+            if (L.split) most = std::max(most, L.d.ne());
+        }
+        if (most > 0) ALLOC(c->f64, 24 * most * sizeof(double));
+    }
     ALLOC(c->xbuf, R * vs0 * sizeof(double));
     ALLOC(c->bbuf, R * vs0 * sizeof(double));
     ALLOC(c->sc, R * sizeof(PcgScalars));
     c->part_cap = std::max(ku_grid_blocks(c->d), kRedBlocks);
+    if (c->fp64 && c->lev[0].split) c->part_cap = std::max(c->part_cap, ceil_div(nn, 128));  // its p.Kp partials
     {
         // the filter reduction grid (32 x 8 columns of 16 layers) can exceed both
         const int fb = ceil_div(c->d.nx, 32) * ceil_div(c->d.ny, 8) * ceil_div(c->d.nz, 16);
@@ -497,6 +507,7 @@ int anl_debug_oob(long long* count_h, long long* first_h) {
 #if ANL_DEBUG
     unsigned long long n = 0;
     ANL_TRY(anl::debug_take_ku(&n, first_h));
+    ANL_TRY(anl::debug_take_ku64(&n, first_h));
     ANL_TRY(anl::debug_take_kbox(&n, first_h));
     ANL_TRY(anl::debug_take_solver(&n, first_h));
     ANL_TRY(anl::debug_take_design(&n, first_h));

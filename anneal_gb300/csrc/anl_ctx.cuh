@@ -25,6 +25,7 @@ struct Level {
     // x, xt, b, r and dv hold one vector per right-hand-side slot, vs values apart (3 nn
     // rounded up to 64 values, so every slot starts on a 256-byte boundary)
     int64_t vs = 0;
+    bool split = false;       // FP64 contexts: the level's K u passes are anl_ku64.cu's
 };
 
 constexpr int kMaxFilterR = 5;
@@ -149,6 +150,7 @@ struct anl_ctx {
     void* y1 = nullptr;
     void* y2 = nullptr;
     void* tmp = nullptr;
+    double* f64 = nullptr;  // FP64 mode: the element forces of the split levels
     double* xbuf = nullptr;
     double* bbuf = nullptr;
 

@@ -105,6 +105,10 @@ __host__ __device__ __forceinline__ void ku_to_slot(KuArgs<T>& a, int r) {
 template <class T>
 int launch_ku(int mode, const KuArgs<T>& a, const KeModal<T>& km, cudaStream_t s);
 int launch_ku_resid_df(const KuArgs<DF>& a, const KeModal<DF>& km, cudaStream_t s);
+// the FP64 passes of small and middle levels (anl_ku64.cu), F: 24 N_e doubles of scratch
+bool ku64_split(const Dims& d, int sms, int march_ox, int march_oy, int march_warps);
+int launch_ku64(int mode, const KuArgs<double>& a, const KeModal<double>& km, double* F, cudaStream_t s);
+bool ku_prefers_split(const Dims& d);
 
 // ------------------------------------------------------------------ small-grid smoother passes
 
@@ -195,6 +199,7 @@ int kutc_error_flag(int* out_h);
 // The out-of-range records of the checked translation units (ANL_IN_RANGE, anl_common.cuh).
 #if ANL_DEBUG
 int debug_take_ku(unsigned long long* count, long long* first);
+int debug_take_ku64(unsigned long long* count, long long* first);
 int debug_take_kbox(unsigned long long* count, long long* first);
 int debug_take_solver(unsigned long long* count, long long* first);
 int debug_take_design(unsigned long long* count, long long* first);

@@ -610,6 +610,13 @@ int launch_ku_resid_df(const KuArgs<DF>& args, const KeModal<DF>& km, cudaStream
     return ANL_OK;
 }
 
+bool ku_prefers_split(const Dims& d) {
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return ku64_split(d, sms, KmCfg<double>::OX, KmCfg<double>::OY, KmCfg<double>::NW);
+}
+
 // Upper bound of the K u grids (one CTA per SM and resident slot, at most 8 per SM): sizes the
 // reduction scratch.
 int ku_grid_blocks(const Dims& d) {

@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include <utility>
 
 #include "anl_ctx.cuh"
@@ -890,6 +891,9 @@ static int ku_pass(anl_ctx* c, const Level& L, int mode, const KuArgs<T>& a, cud
             return launch_kutc(mode, t, c->kmf, s);
         }
     }
+    if constexpr (std::is_same<T, double>::value) {
+        if (L.split) return launch_ku64(mode, a, c->kmd, c->f64, s);
+    }
     return launch_ku<T>(mode, a, modal_of<T>(c), s);
 }
 
@@ -1027,7 +1031,7 @@ template <class T>
 static int smooth(anl_ctx* c, Level& L, int degree, bool x_is_zero, const int* done, cudaStream_t s) {
     const double* cf = c->cheb_d + (size_t)level_index(c, L) * kChebStride + 1;  // (c1, c2) pairs
     int k0 = 0;
-    if (x_is_zero && degree >= 2) {  // steps 0 and 1 in one pass: x1 = c2_0 D^-1 b is never stored
+    if (x_is_zero && degree >= 2 && !L.split) {  // steps 0 and 1 in one pass: x1 = c2_0 D^-1 b is never stored
         KuArgs<T> a = ku_args<T>(c, L);
         a.b = (const T*)L.b;
         a.diag = L.diag;

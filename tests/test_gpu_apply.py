@@ -26,3 +26,22 @@ def test_fused_apply_matches_in_place_apply(shape, fp64):
     c.apply_K(E, u, u)
     assert torch.equal(y, u)
     c.close()
+
+
+# grids on the two-kernel FP64 pass (a single element, partial warps and blocks, odd sides)
+@pytest.mark.parametrize("shape", [(1, 1, 1), (5, 3, 2), (31, 9, 17), (64, 32, 32)])
+def test_split_fp64_pass_matches_the_march(shape):
+    """The FP64 pass of small levels against the marching one: a value is a sum of 8 corner forces of
+    some 40 operations each, so the two orders differ by at most 8 * 40 * 1.1e-16 = 4e-14 of the
+    forces' size, here bounded by the largest value of |K| |u|."""
+    rng = np.random.default_rng(sum(shape))
+    c = Context(shape, 1.0, 0.3, fp64=True)
+    c.set_domain(torch.ones(c.ne, dtype=torch.uint8, device="cuda"), torch.zeros(c.ndof, dtype=torch.uint8, device="cuda"))
+    E = to_dev(rng.uniform(0.1, 2.0, c.ne), torch.float32)
+    u = to_dev(rng.normal(size=c.ndof), torch.float64)
+    y, z = torch.empty_like(u), torch.empty_like(u)
+    c.apply_K(E, u, y)
+    c.profile_apply(u, z, 1)   # the solver's own pass on the same element scales
+    bound = 2.0 * 8 * 4.0 * float(u.abs().max())   # E, corners, the row sums of |Ke| (below 4), u
+    assert float((y - z).abs().max()) <= 4e-14 * bound
+    c.close()
