@@ -209,7 +209,9 @@ __device__ __forceinline__ float2 psub(float2 a, float2 b) {  // a - b, one roun
     return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
 }
 __device__ __forceinline__ float2 pscale(float s, float2 a) { return __fmul2_rn(make_float2(s, s), a); }
+__device__ __forceinline__ float2 ptwice_plus(float2 a, float2 b) { return __ffma2_rn(a, make_float2(2.f, 2.f), b); }
 #endif
+__host__ __device__ __forceinline__ dpair ptwice_plus(dpair a, dpair b) { return {2.0 * a.x + b.x, 2.0 * a.y + b.y}; }
 
 #pragma nv_exec_check_disable
 template <class T>
@@ -225,6 +227,14 @@ __host__ __device__ __forceinline__ V3<T> operator-(const V3<T>& a, const V3<T>&
 template <class T>
 __host__ __device__ __forceinline__ V3<T> operator*(T s, const V3<T>& a) {
     return V3<T>{pscale(s, a.xy), s * a.z};
+}
+__host__ __device__ __forceinline__ float twice_plus(float a, float b) { return 2.f * a + b; }
+__host__ __device__ __forceinline__ double twice_plus(double a, double b) { return 2.0 * a + b; }
+// 2 a + b
+#pragma nv_exec_check_disable
+template <class T>
+__host__ __device__ __forceinline__ V3<T> twice_plus(const V3<T>& a, const V3<T>& b) {
+    return V3<T>{ptwice_plus(a.xy, b.xy), twice_plus(a.z, b.z)};
 }
 template <class T>
 __host__ __device__ __forceinline__ V3<T> v3zero() {
@@ -311,8 +321,18 @@ __host__ __device__ __forceinline__ void modal_element(const KeModal<T>& k, T E,
                                                        const V3<T> (&dxt)[2], const V3<T> (&dyb)[2],
                                                        const V3<T> (&dyt)[2], const V3<T> (&dz)[2][2],
                                                        V3<T> (&f)[2][2][2]) {
+    // as modal_amplitudes with the y and z edges of the side px = 0 alone: the edges of the other
+    // side differ from them by differences of x edges, dy(1) - dy(0) = dx(py = 1) - dx(py = 0)
     V3<T> b[8], g[8];
-    modal_amplitudes<T>(dxb, dxt, dyb, dyt, dz, b);
+    const V3<T> s0 = dxb[0] + dxb[1], s1 = dxt[0] + dxt[1];
+    b[1] = s0 + s1;
+    b[6] = s1 - s0;
+    const V3<T> p0 = dxb[1] - dxb[0], p1 = dxt[1] - dxt[0];
+    b[4] = p0 + p1;
+    b[7] = p1 - p0;
+    b[2] = twice_plus(dyb[0] + dyt[0], b[4]);
+    b[5] = twice_plus(dyt[0] - dyb[0], b[7]);
+    b[3] = twice_plus(dz[0][0] + dz[0][1], b[6]);
     modal_forces<T>(k, E, b, g);
     // back to the corners: f(p) = sum_m s_m(p) g_m = A(py,pz) + sx B(py,pz)
     const V3<T> am = g[2] - g[5], ap = g[2] + g[5];
@@ -613,6 +633,8 @@ struct PairOf<DF> {
 __device__ __forceinline__ dfpair padd(dfpair a, dfpair b) { return {a.x + b.x, a.y + b.y}; }
 __device__ __forceinline__ dfpair psub(dfpair a, dfpair b) { return {a.x - b.x, a.y - b.y}; }
 __device__ __forceinline__ dfpair pscale(DF s, dfpair a) { return {s * a.x, s * a.y}; }
+__device__ __forceinline__ DF twice_plus(DF a, DF b) { return DF(2.f * a.hi, 2.f * a.lo) + b; }
+__device__ __forceinline__ dfpair ptwice_plus(dfpair a, dfpair b) { return {twice_plus(a.x, b.x), twice_plus(a.y, b.y)}; }
 #endif
 
 // Compensated accumulator: adds a*b exactly up to FP32 rounding of the error terms.

@@ -14,8 +14,8 @@
 // next is applied, without atomics: across x by a shuffle from lane l - 1, across y through
 // shared memory from warp w - 1, and across z in registers from the previous layer. Against
 // forming 8 corner forces per element and adding them up, and with the x and y mode sums of the
-// lower node plane carried over from the previous layer, an element takes 150 instead of 190
-// additions and multiplications and 21 instead of 24 shuffles. So lanes 1..30 of warps 1..NW-1 own
+// lower node plane carried over from the previous layer, an element takes 145 instead of 190
+// additions and multiplications and 18 instead of 24 shuffles. So lanes 1..30 of warps 1..NW-1 own
 // complete nodes; the outer lanes and warp 0 compute the halo elements of the tile (a 13 % overlap
 // at NW = 16). Warps whose 32 elements are all void skip the element arithmetic.
 // HBM traffic is u once, y once, E once and the node mask once (halo re-reads hit L2).
@@ -316,7 +316,7 @@ struct KuTile {
         const V3<T> d0 = nb0 - c.ub[0], d1 = nb1 - c.ub[1];
         c.sx = d0 + d1;
         c.px = d1 - d0;
-        c.ty = (c.ub[1] - c.ub[0]) + (nb1 - nb0);
+        c.ty = twice_plus(c.ub[1] - c.ub[0], c.px);  // Dy of column ie + 1 is that of ie plus px
     }
 
     // Element layer kk (between node planes kk and kk + 1), staged in ring slot kk % KU_RING;
@@ -342,7 +342,6 @@ struct KuTile {
         plane_modes(o);
         V3<T> n0, ny, nz, nyz;  // node column ie: the sums over its two elements in x, by y and z mode
         const V3<T> dz = (cu[0] - in.ub[0]) + (cu[1] - in.ub[1]);
-        const V3<T> dzr = shfl_down3(dz);
         if (__any_sync(FULL, Ee != 0.f)) {
             V3<T> b[8], g[8];
             b[1] = in.sx + o.sx;
@@ -351,7 +350,7 @@ struct KuTile {
             b[7] = o.px - in.px;
             b[2] = in.ty + o.ty;
             b[5] = o.ty - in.ty;
-            b[3] = dz + dzr;
+            b[3] = twice_plus(dz, b[6]);  // column ie + 1 adds the differences of Dx across the layer
             modal_forces<T>(km, T(Ee), b, g);
             // back transform one direction at a time, each direction summed onto its nodes before
             // the next: in x the side px = 1 of lane l - 1 meets px = 0 of lane l
