@@ -156,20 +156,33 @@ void kbox_prepare();
 // solved with the dense inverse as float pairs (ainv_hi + ainv_lo, nc x nc, symmetric).
 constexpr int kTailMaxLevels = 8;
 constexpr int kTailMaxSmem = 220 * 1024;
+struct TailGeo {          // a level's slabs (anl_vtail.cu)
+    int A = 0, B = 0, L = 0, per = 0, active = 0, PA = 0, planeN = 0;
+    int ns = 0, na = 0, nb = 0, es = 0, ea = 0, eb = 0;
+    int p[3] = {0, 0, 0}; // node strides of the tail's own vectors along x, y, z
+};
+struct TailLayout {       // shared memory, in words
+    int xlen = 0, c = 0, words = 0;
+    int f[kTailMaxLevels], flen[kTailMaxLevels], e[kTailMaxLevels];
+};
 struct TailLevel {
     Dims d{};
+    TailGeo g;
     const float* E = nullptr;
     const uint8_t* nmask = nullptr;
     const float* diag = nullptr;
     const double* cheb = nullptr;  // (c1, c2) pairs of the level's sweep
     int degree = 0;
-    float* r = nullptr;            // the level's residual and correction, slots vs floats apart
+    float* b = nullptr;            // the level's vectors, slots vs floats apart
+    float* r = nullptr;
     float* x = nullptr;
+    float* xt = nullptr;
     int64_t vs = 0;
 };
 struct TailArgs {
     int nlev = 0, ctas = 0;
     TailLevel lev[kTailMaxLevels];
+    TailLayout lay;                // set by the launcher, as the levels' g
     float* b0 = nullptr;
     const float* ainv_hi = nullptr;
     const float* ainv_lo = nullptr;
@@ -181,7 +194,7 @@ struct TailArgs {
     int sc_bytes = 0;  // bytes between the slots' done flags
 };
 int vtail_prepare(int* ctas);
-bool vtail_fits(const TailLevel* lev, int nlev, int ctas);
+bool vtail_fits(TailLevel* lev, int nlev, int ctas);  // fills the levels' g
 int launch_vtail(const TailArgs& a, cudaStream_t s);
 
 // ------------------------------------------------------------------ tensor-core K u (fine grid)

@@ -16,8 +16,8 @@
 // forming 8 corner forces per element and adding them up, and with the x and y mode sums of the
 // lower node plane carried over from the previous layer, an element takes 145 instead of 190
 // additions and multiplications and 18 instead of 24 shuffles. So lanes 1..30 of warps 1..NW-1 own
-// complete nodes; the outer lanes and warp 0 compute the halo elements of the tile (a 13 % overlap
-// at NW = 16). Warps whose 32 elements are all void skip the element arithmetic.
+// complete nodes; the outer lanes and warp 0 compute the halo elements of the tile (a 22 % overlap
+// at NW = 8). Warps whose 32 elements are all void skip the element arithmetic.
 // HBM traffic is u once, y once, E once and the node mask once (halo re-reads hit L2).
 //
 // The same kernel in double-float arithmetic (T = DF, residual mode only) evaluates the FP64
@@ -32,11 +32,17 @@
 
 namespace anl {
 
+// Two CTAs of 8 warps per SM: their barriers are apart, so one fills the other's waits, and small
+// grids split into twice as many CTAs. Against one CTA of 16 warps (back to back, apply / p.Kp /
+// residual / first two steps / post-smoothing): 48x24x24 6.2 / 8.2 / 6.2 / 6.2 / 6.2 / 6.2 us (7.2 / 10.3
+// / 8.2 / 8.2 / 8.2 / 8.2), 192x96x96 28.6 / 32.8 / 30.5 / 33.7 / 35.9 / 34.9 (32.8 / 34.8 / 34.8 / 36.9 /
+// 41.0 / 36.9), 256x128x128 57.4 / 64.6 / 63.5 / 70.1 / 81.9 / 78.2 (61.5 / 65.1 / 63.6 / 71.7 / 82.0 /
+// 76.2), although a tile of 7 owned rows recomputes 14 % of its elements where one of 15 did 7 %.
 #ifndef KU_NW32
-#define KU_NW32 16  // warps per CTA of the FP32 K u kernel
+#define KU_NW32 8  // warps per CTA of the FP32 K u kernel
 #endif
 #ifndef KU_MINB32
-#define KU_MINB32 1  // resident CTAs per SM its registers are sized for
+#define KU_MINB32 2  // resident CTAs per SM its registers are sized for
 #endif
 #ifndef KU_DEPTH
 #define KU_DEPTH 3  // layers staged ahead by cp.async
@@ -60,7 +66,7 @@ __device__ __forceinline__ float shfl_upv(float v) { return __shfl_up_sync(0xfff
 __device__ __forceinline__ double shfl_upv(double v) { return __shfl_up_sync(0xffffffffu, v, 1); }
 __device__ __forceinline__ DF shfl_upv(DF v) { return DF(shfl_upv(v.hi), shfl_upv(v.lo)); }
 
-// warps per CTA: 16 in FP32 (15 owned node rows), 8 in FP64 (shared memory and registers)
+// warps per CTA (NW - 1 owned node rows)
 template <class T>
 struct KmCfg {
     static constexpr int NW = sizeof(T) == 4 ? KU_NW32 : 8;

@@ -1154,8 +1154,10 @@ static int vcycle_tail(anl_ctx* c, size_t l, const int* done, cudaStream_t s) {
         a.lev[q].diag = Lq.diag;
         a.lev[q].cheb = c->cheb_d + (l + q) * kChebStride + 1;
         a.lev[q].degree = c->degree(l + q);
+        a.lev[q].b = (float*)Lq.b;
         a.lev[q].r = (float*)Lq.r;
         a.lev[q].x = (float*)Lq.x;
+        a.lev[q].xt = (float*)Lq.xt;
         a.lev[q].vs = Lq.vs;
     }
     a.b0 = (float*)c->lev[l].b;

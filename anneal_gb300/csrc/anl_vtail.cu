@@ -28,10 +28,8 @@
 // through the levels' vectors in global memory, every load of a node in flight at once.
 //
 // What bounds it: the chain of one step (about 48 shared-memory accesses and 250 instructions per
-// element, then 24 and 80 per node, the halo's flight, two block barriers).
-// Measured steps: 1.4 us with 2 layers of 4 x 4 to 8 x 8 elements a CTA, 3.4 us with 3 layers of
-// 16 x 16; a CG iteration at 48x24x24 takes 128 us (168 with a launch per level and step), at
-// 96x48x48 226 us (288), at 256x128x128 944 us (992).
+// element, then 24 and 80 per node, the halo's flight, two block barriers). The tail's own vectors
+// between levels are in slab-major order, so a warp's loads of them coalesce whatever the axis.
 #include "anl_common.cuh"
 #include "anl_kernels.cuh"
 
@@ -45,60 +43,50 @@ constexpr int FW = 25;          // words between two elements' forces (24 and on
 constexpr int kWaitTries = 1 << 20;  // bound of a halo wait
 constexpr int kTailMaxDegree = 16;  // Chebyshev steps per sweep there is room for
 
-// A level's slab of one CTA: A x B elements per layer, L layers along AXIS.
-template <int AXIS>
-struct Slab {
-    int A, B, L, per, active, own, nown, PA, planeN;
-    int64_t ns, na, nb, es, ea, eb;  // node and element strides along AXIS, A, B
-    __host__ __device__ Slab(const Dims& d, int rank, int ctas) {
-        const int n[3] = {d.nx, d.ny, d.nz};
-        constexpr int ax = AXIS == 0 ? 1 : 0, bx = AXIS == 2 ? 1 : 2;
-        const int64_t nstr[3] = {1, d.nx + 1, (int64_t)(d.nx + 1) * (d.ny + 1)};
-        const int64_t estr[3] = {1, d.nx, (int64_t)d.nx * d.ny};
-        A = n[ax];
-        B = n[bx];
-        L = n[AXIS];
-        ns = nstr[AXIS], na = nstr[ax], nb = nstr[bx];
-        es = estr[AXIS], ea = estr[ax], eb = estr[bx];
-        per = (L + ctas - 1) / ctas;
-        active = (L + per - 1) / per;
-        own = rank < active ? (per < L - rank * per ? per : L - rank * per) : 0;
-        nown = rank < active ? own + (rank == active - 1 ? 1 : 0) : 0;
-        PA = A + 1;
-        planeN = PA * (B + 1);
-    }
-    // sizes for any rank
-    __host__ __device__ int max_nodes() const { return (per + 1) * planeN; }
-    __host__ __device__ int max_elems() const { return (per + 1) * A * B; }
-    __host__ __device__ int max_padded() const { return (per + 2) * planeN + A + 2; }
-};
+// A level's slabs: A x B elements per layer, L layers along the tail's axis, `per` layers to a CTA.
+// Levels of at most kAloneElems elements stay in one CTA: its step (0.8 us at 128 elements, 1.2 at
+// 432) is shorter than a shared one, whose halo flight alone takes 0.7 us.
+constexpr int kAloneElems = 512;
+
+TailGeo slab_geo(int axis, const Dims& d, int ctas) {
+    const int n[3] = {d.nx, d.ny, d.nz};
+    const int ax = axis == 0 ? 1 : 0, bx = axis == 2 ? 1 : 2;
+    const int nstr[3] = {1, d.nx + 1, (d.nx + 1) * (d.ny + 1)}, estr[3] = {1, d.nx, d.nx * d.ny};
+    TailGeo g;
+    g.A = n[ax];
+    g.B = n[bx];
+    g.L = n[axis];
+    g.ns = nstr[axis], g.na = nstr[ax], g.nb = nstr[bx];
+    g.es = estr[axis], g.ea = estr[ax], g.eb = estr[bx];
+    const int use = d.ne() <= kAloneElems ? 1 : ctas;
+    g.per = (g.L + use - 1) / use;
+    g.active = (g.L + g.per - 1) / g.per;
+    g.PA = g.A + 1;
+    g.planeN = g.PA * (g.B + 1);
+    // the slab-major node order of the tail's own vectors: index = s planeN + b PA + a
+    g.p[axis] = g.planeN;
+    g.p[ax] = 1;
+    g.p[bx] = g.PA;
+    return g;
+}
+// sizes that hold for every CTA
+int max_nodes(const TailGeo& g) { return (g.per + 1) * g.planeN; }
+int max_elems(const TailGeo& g) { return (g.per + (g.active > 1 ? 1 : 0)) * g.A * g.B; }
+int max_padded(const TailGeo& g) { return (g.per + 2) * g.planeN + g.A + 2; }
 
 // shared-memory carve-up in words: the iterate twice (own planes and two halo planes), the coarsest
-// right-hand side, then per level the forces, the elements' (scale, packed indices) pairs and the
-// nodes' b and x
-struct TailLayout {
-    int x, xlen, c, f[kTailMaxLevels], e[kTailMaxLevels], save[kTailMaxLevels], words;
-};
-
-template <int AXIS>
-__host__ __device__ inline TailLayout tail_layout(const TailLevel* lev, int nlev, int ctas) {
+// right-hand side, then per level the forces and the elements' (scale, packed indices) pairs
+TailLayout tail_layout(const TailLevel* lev, int nlev) {
     TailLayout t{};
-    for (int l = 0; l < nlev - 1; ++l) {
-        const Slab<AXIS> g(lev[l].d, 0, ctas);
-        const int x = 3 * (g.max_nodes() + 2 * g.planeN);
-        t.xlen = t.xlen > x ? t.xlen : x;
-    }
-    t.x = 0;
+    for (int l = 0; l < nlev - 1; ++l) t.xlen = std::max(t.xlen, 3 * (max_nodes(lev[l].g) + 2 * lev[l].g.planeN));
+    t.xlen = (t.xlen + 3) / 4 * 4;
     int o = 2 * t.xlen;
     for (int l = 0; l < nlev - 1; ++l) {
-        const Slab<AXIS> g(lev[l].d, 0, ctas);
         t.e[l] = o;
-        o += 2 * g.max_elems();
+        o += (2 * max_elems(lev[l].g) + 3) / 4 * 4;
         t.f[l] = o;
-        o += FW * g.max_padded();
-        t.save[l] = o;
-        o += 6 * g.max_nodes();
-        o += o & 1;
+        t.flen[l] = (FW * max_padded(lev[l].g) + 3) / 4 * 4;
+        o += t.flen[l];
     }
     t.c = o;
     t.words = o + 3 * (int)lev[nlev - 1].d.nn();
@@ -135,30 +123,31 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, unsigned parity) {
 }
 
 // components c0 .. c0 + NC - 1 of (R r)(I, J, K): trilinear weights 1, 1/2, 1/4, 1/8 of the fine
-// residual r; nodes outside the grid are read at its edge with weight 0, so no load depends on a
-// test and a plane's loads are in flight together
+// residual r (slab-major, strides p); nodes outside the grid are read at its edge with weight 0, so
+// no load depends on a test and a plane's loads are in flight together
 template <int NC>
-__device__ __forceinline__ void restrict_at(const Dims& f, const float* r, int I, int J, int K, int c0,
+__device__ __forceinline__ void restrict_at(const TailLevel& f, const float* r, int I, int J, int K, int c0,
                                             float (&acc)[NC]) {
-    const int sy = f.nx + 1, sz = sy * (f.ny + 1);  // a tail level's indices fit an int
+    const Dims& d = f.d;
+    const int px = 3 * f.g.p[0], py = 3 * f.g.p[1], pz = 3 * f.g.p[2];
 #pragma unroll
     for (int c = 0; c < NC; ++c) acc[c] = 0.f;
 #pragma unroll 1
     for (int dk = -1; dk <= 1; ++dk) {
         const int k = 2 * K + dk;
-        const float* p = r + 3 * sz * min(max(k, 0), f.nz) + c0;
-        const float wk = k < 0 || k > f.nz ? 0.f : dk ? 0.5f : 1.f;
+        const float* p = r + pz * min(max(k, 0), d.nz) + c0;
+        const float wk = k < 0 || k > d.nz ? 0.f : dk ? 0.5f : 1.f;
         float v[9][NC];
 #pragma unroll
         for (int q = 0; q < 9; ++q) {
-            const int i = min(max(2 * I + q % 3 - 1, 0), f.nx), j = min(max(2 * J + q / 3 - 1, 0), f.ny);
+            const int i = min(max(2 * I + q % 3 - 1, 0), d.nx), j = min(max(2 * J + q / 3 - 1, 0), d.ny);
 #pragma unroll
-            for (int c = 0; c < NC; ++c) v[q][c] = __ldcg(p + 3 * (i + sy * j) + c);
+            for (int c = 0; c < NC; ++c) v[q][c] = p[px * i + py * j + c];
         }
 #pragma unroll
         for (int q = 0; q < 9; ++q) {
             const int di = q % 3 - 1, dj = q / 3 - 1, i = 2 * I + di, j = 2 * J + dj;
-            const bool in = i >= 0 && j >= 0 && i <= f.nx && j <= f.ny;
+            const bool in = i >= 0 && j >= 0 && i <= d.nx && j <= d.ny;
             const float w = in ? (di ? 0.5f : 1.f) * (dj ? 0.5f : 1.f) * wk : 0.f;
 #pragma unroll
             for (int c = 0; c < NC; ++c) acc[c] = fmaf(w, v[q][c], acc[c]);
@@ -167,16 +156,16 @@ __device__ __forceinline__ void restrict_at(const Dims& f, const float* r, int I
 }
 
 // (P xc)(i, j, k): the mean of the coarse nodes the fine node lies between (the unused ones of the
-// 8 are read at the node itself)
-__device__ __forceinline__ void prolong_at(const Dims& cd, const float* xc, int i, int j, int k, float (&acc)[3]) {
-    const int sy = cd.nx + 1, sz = sy * (cd.ny + 1), di = i & 1, dj = j & 1, dk = k & 1;
-    const int n0 = (i >> 1) + sy * (j >> 1) + sz * (k >> 1);
+// 8 are read at the node itself); xc has node strides p
+__device__ __forceinline__ void prolong_at(const int (&p)[3], const float* xc, int i, int j, int k, float (&acc)[3]) {
+    const int di = i & 1, dj = j & 1, dk = k & 1;
+    const int n0 = (i >> 1) * p[0] + (j >> 1) * p[1] + (k >> 1) * p[2];
     float v[8][3];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-        const int n = n0 + (q & di) + sy * ((q >> 1) & dj) + sz * ((q >> 2) & dk);
+        const int n = n0 + (q & di) * p[0] + ((q >> 1) & dj) * p[1] + ((q >> 2) & dk) * p[2];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) v[q][c] = __ldcg(xc + 3 * n + c);
+        for (int c = 0; c < 3; ++c) v[q][c] = xc[3 * n + c];
     }
     const float w = (di ? 0.5f : 1.f) * (dj ? 0.5f : 1.f) * (dk ? 0.5f : 1.f);
 #pragma unroll
@@ -193,10 +182,10 @@ __device__ __forceinline__ void prolong_at(const Dims& cd, const float* xc, int 
 
 // an owned node of this thread on the current level
 struct TailNode {
-    int t;          // ordinal among the CTA's owned nodes, -1 for none
-    int nl;         // first word of the node in an iterate buffer
-    int nb;         // padded index of the element above it in every direction
+    int pn;         // node index in slab-major order, -1 for none
     int gn;         // node index on the level's grid
+    int nl;         // first word of the node in an iterate buffer
+    int nb;         // first word of the padded element above it in every direction
     int i, j, k;
     unsigned m;     // mask
     float g;        // inverse diagonal
@@ -207,7 +196,6 @@ struct TailNode {
 template <int AXIS>
 struct Tail {
     const TailArgs& a;
-    const TailLayout& lay;
     float* sm;
     uint32_t bar;                 // this CTA's barriers: [direction][buffer], 8 bytes each
     uint32_t x_down, x_up, b_down, b_up;  // the neighbours' iterate buffers and barriers
@@ -219,20 +207,28 @@ struct Tail {
 
     __device__ float* vec(float* p, int l) const { return p + (int64_t)slot * a.lev[l].vs; }
 
+    __device__ int own(const TailGeo& g) const { return rank < g.active ? min(g.per, g.L - rank * g.per) : 0; }
+    // element layers the CTA computes: its own and, but for the first CTA, the one below
+    __device__ int first_layer(const TailGeo& g) const { return g.active > 1 ? rank * g.per - 1 : 0; }
+    __device__ int elems(const TailGeo& g) const {
+        const int o = own(g);
+        return o > 0 ? (o + (g.active > 1 ? 1 : 0)) * g.A * g.B : 0;
+    }
+
     // the element table of level l and its zeroed forces (once per launch)
     __device__ void table(int l) {
         const TailLevel& lv = a.lev[l];
-        const Slab<AXIS> g(lv.d, rank, ctas);
-        float* f = sm + lay.f[l];
-        for (int t = tid; t < FW * g.max_padded(); t += TT) f[t] = 0.f;
-        const int layer = g.A * g.B, ne = g.own > 0 ? (g.own + 1) * layer : 0;
-        float2* et = reinterpret_cast<float2*>(sm + lay.e[l]);
+        const TailGeo& g = lv.g;
+        float4* f = reinterpret_cast<float4*>(sm + a.lay.f[l]);
+        for (int t = tid; t < a.lay.flen[l] / 4; t += TT) f[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int layer = g.A * g.B, ne = elems(g), first = first_layer(g), q0 = g.active > 1 ? 0 : 1;
+        float2* et = reinterpret_cast<float2*>(sm + a.lay.e[l]);
         for (int e = tid; e < ne; e += TT) {
             const int q = e / layer, in = e - q * layer, b = in / g.A, aa = in - b * g.A;
-            const int gl = rank * g.per - 1 + q;
-            const int64_t ge = gl * g.es + aa * g.ea + b * g.eb;
-            const float Ee = gl >= 0 && ANL_IN_RANGE(ge, lv.d.ne()) ? __ldg(lv.E + ge) : 0.f;
-            const int n0 = q * g.planeN + aa + g.PA * b, pe = (q * (g.B + 1) + b + 1) * g.PA + aa + 1;
+            const int ge = (first + q) * g.es + aa * g.ea + b * g.eb;
+            const float Ee = first + q >= 0 && ANL_IN_RANGE(ge, lv.d.ne()) ? __ldg(lv.E + ge) : 0.f;
+            // node plane 0 is the halo below; a level in one CTA starts at plane 1
+            const int n0 = (q + q0) * g.planeN + aa + g.PA * b, pe = ((q + q0) * (g.B + 1) + b + 1) * g.PA + aa + 1;
             et[e] = make_float2(Ee, __int_as_float(n0 | (pe << 16)));
         }
     }
@@ -240,22 +236,23 @@ struct Tail {
     // this thread's nodes of level l
     __device__ void enter(int l) {
         const TailLevel& lv = a.lev[l];
-        const Slab<AXIS> g(lv.d, rank, ctas);
+        const TailGeo& g = lv.g;
+        const int o = own(g), nown = o > 0 ? o + (rank == g.active - 1 ? 1 : 0) : 0;
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
             TailNode& n = nd[r];
             const int t = tid + r * TT;
-            n.t = -1;
+            n.pn = -1;
             n.m = 0;
             n.g = 0.f;
 #pragma unroll
             for (int c = 0; c < 3; ++c) n.b[c] = n.d[c] = n.x[c] = 0.f;
-            if (t >= g.nown * g.planeN) continue;
+            if (t >= nown * g.planeN) continue;
             const int p = 1 + t / g.planeN, in = t - (p - 1) * g.planeN, b = in / g.PA, aa = in - b * g.PA;
             const int s = rank * g.per + p - 1;
-            n.gn = (int)(s * g.ns + aa * g.na + b * g.nb);
+            n.gn = s * g.ns + aa * g.na + b * g.nb;
             if (!ANL_IN_RANGE(n.gn, lv.d.nn())) continue;
-            n.t = t;
+            n.pn = s * g.planeN + in;
             n.nl = 3 * (p * g.planeN + in);
             n.nb = FW * ((p * (g.B + 1) + b + 1) * g.PA + aa + 1);
             n.i = AXIS == 0 ? s : aa;
@@ -264,29 +261,26 @@ struct Tail {
             n.m = __ldg(lv.nmask + n.gn) & 7u;
             n.g = __ldg(lv.diag + n.gn);
             n.down = p == 1 && rank > 0 ? 3 * ((g.per + 1) * g.planeN + in) : -1;
-            n.up = p == g.nown && rank + 1 < g.active ? 3 * in : -1;
+            n.up = p == nown && rank + 1 < g.active ? 3 * in : -1;
         }
     }
 
     // the nodes' x into the other buffer and the neighbours' halo planes; then the wait for the own
     // halo planes
     __device__ void exchange(int l) {
-        const Dims& d = a.lev[l].d;
-        const int L = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;
-        const int per = (L + ctas - 1) / ctas, active = (L + per - 1) / per;
-        const int planeN = ((AXIS == 0 ? d.ny : d.nx) + 1) * ((AXIS == 2 ? d.ny : d.nz) + 1);
+        const TailGeo& g = a.lev[l].g;
         cur ^= 1;
-        const bool from[2] = {rank > 0 && rank < active, rank + 1 < active};
+        const bool from[2] = {rank > 0 && rank < g.active, rank + 1 < g.active};
         if (tid == 0) {
 #pragma unroll
             for (int q = 0; q < 2; ++q)
-                if (from[q]) bar_expect(bar + 8u * (2 * q + cur), 12u * (unsigned)planeN);
+                if (from[q]) bar_expect(bar + 8u * (2 * q + cur), 12u * (unsigned)g.planeN);
         }
-        const int o = cur * lay.xlen;
+        const int o = cur * a.lay.xlen;
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
             const TailNode& n = nd[r];
-            if (n.t < 0) continue;
+            if (n.pn < 0) continue;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 // this CTA lies above rank - 1 and below rank + 1
@@ -294,7 +288,7 @@ struct Tail {
                 if (n.up >= 0) st_async(x_up + 4u * (unsigned)(o + n.up + c), n.x[c], b_up + 8u * cur);
             }
 #pragma unroll
-            for (int c = 0; c < 3; ++c) sm[lay.x + o + n.nl + c] = n.x[c];
+            for (int c = 0; c < 3; ++c) sm[o + n.nl + c] = n.x[c];
         }
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -308,15 +302,12 @@ struct Tail {
 
     // the corner forces of the CTA's elements (corner pa + 2 pb + 4 ps in slab directions)
     __device__ void elements(int l) const {
-        const Dims& d = a.lev[l].d;
-        const int A = AXIS == 0 ? d.ny : d.nx, B = AXIS == 2 ? d.ny : d.nz, L = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;
-        const int per = (L + ctas - 1) / ctas, own = min(per, L - rank * per);
-        const int ne = own > 0 ? (own + 1) * A * B : 0;
-        const float* x = sm + lay.x + cur * lay.xlen;
-        const float2* et = reinterpret_cast<const float2*>(sm + lay.e[l]);
-        float* F = sm + lay.f[l];
-        const int sa = 3, sb = 3 * (A + 1), ss = sb * (B + 1);
-        const int sx = AXIS == 0 ? ss : sa, sy = AXIS == 1 ? ss : AXIS == 0 ? sa : sb, sz = AXIS == 2 ? ss : sb;
+        const TailGeo& g = a.lev[l].g;
+        const int ne = elems(g);
+        const float* x = sm + cur * a.lay.xlen;
+        const float2* et = reinterpret_cast<const float2*>(sm + a.lay.e[l]);
+        float* F = sm + a.lay.f[l];
+        const int sx = 3 * g.p[0], sy = 3 * g.p[1], sz = 3 * g.p[2];
         for (int e = tid; e < ne; e += TT) {
             const float2 te = et[e];
             if (te.x == 0.f) continue;  // its forces stay the zeros of table()
@@ -366,13 +357,12 @@ struct Tail {
 
     // (K x)(n): the 8 corners that meet at the node, in a fixed order
     __device__ void force(int l, const TailNode& n, float (&y)[3]) const {
-        const Dims& d = a.lev[l].d;
-        const int PA = (AXIS == 0 ? d.ny : d.nx) + 1, planeN = PA * ((AXIS == 2 ? d.ny : d.nz) + 1);
-        const float* F = sm + lay.f[l] + n.nb;
+        const TailGeo& g = a.lev[l].g;
+        const float* F = sm + a.lay.f[l] + n.nb;
         y[0] = y[1] = y[2] = 0.f;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const float* p = F - FW * ((q & 1) + ((q >> 1) & 1) * PA + (q >> 2) * planeN) + 3 * q;
+            const float* p = F - FW * ((q & 1) + ((q >> 1) & 1) * g.PA + (q >> 2) * g.planeN) + 3 * q;
 #pragma unroll
             for (int c = 0; c < 3; ++c) y[c] += p[c];
         }
@@ -402,7 +392,6 @@ struct Tail {
 template <int AXIS>
 __global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArgs a) {
     extern __shared__ __align__(16) float tail_smem[];
-    __shared__ TailLayout lay;
     __shared__ float cf[kTailMaxLevels][2 * kTailMaxDegree];
     __shared__ __align__(8) uint64_t bars[2][2];
     const int tid = threadIdx.x, ctas = a.ctas;
@@ -412,7 +401,6 @@ __global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArg
     const int last = a.nlev - 1;
     const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&bars[0][0]);
     if (tid == 0) {
-        lay = tail_layout<AXIS>(a.lev, a.nlev, ctas);
 #pragma unroll
         for (int q = 0; q < 4; ++q) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8u * q) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -422,9 +410,9 @@ __global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArg
         if (k < 2 * a.lev[l].degree) cf[l][k] = (float)a.lev[l].cheb[k];
     }
     __syncthreads();
-    Tail<AXIS> t{a, lay, tail_smem, bar, 0, 0, 0, 0, tid, rank, ctas, slot};
+    Tail<AXIS> t{a, tail_smem, bar, 0, 0, 0, 0, tid, rank, ctas, slot};
     {
-        const uint32_t xb = (uint32_t)__cvta_generic_to_shared(tail_smem + lay.x);
+        const uint32_t xb = (uint32_t)__cvta_generic_to_shared(tail_smem);
         const int below = rank > 0 ? rank - 1 : 0, above = rank + 1 < ctas ? rank + 1 : rank;
         t.x_down = map_rank(xb, below);
         t.x_up = map_rank(xb, above);
@@ -436,40 +424,41 @@ __global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArg
 
     for (int l = 0; l < last; ++l) {  // down: smooth from zero, residual
         const int deg = a.lev[l].degree;
-        float* save = tail_smem + lay.save[l];
         t.enter(l);
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
             TailNode& n = t.nd[r];
-            if (n.t < 0) continue;
+            if (n.pn < 0) continue;
             if (l == 0) {
 #pragma unroll
                 for (int c = 0; c < 3; ++c) n.b[c] = __ldg(t.vec(a.b0, 0) + 3 * n.gn + c);
             } else {
-                restrict_at<3>(a.lev[l - 1].d, t.vec(a.lev[l - 1].r, l - 1), n.i, n.j, n.k, 0, n.b);
+                restrict_at<3>(a.lev[l - 1], t.vec(a.lev[l - 1].r, l - 1), n.i, n.j, n.k, 0, n.b);
             }
             const float gn = cf[l][1] * n.g;  // step 0: x = d = c2_0 D^-1 b
+            float* save = t.vec(a.lev[l].b, l) + 3 * n.pn;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 if (!((n.m >> c) & 1)) n.b[c] = 0.f;
                 n.x[c] = n.d[c] = gn * n.b[c];
-                save[6 * n.t + c] = n.b[c];
+                if (l > 0) save[c] = n.b[c];
             }
         }
         t.exchange(l);
         for (int k = 1; k < deg; ++k) t.step(l, cf[l][2 * k], cf[l][2 * k + 1]);
         t.elements(l);
         float* res = t.vec(a.lev[l].r, l);
+        float* save = t.vec(a.lev[l].xt, l);
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
             const TailNode& n = t.nd[r];
-            if (n.t < 0) continue;
+            if (n.pn < 0) continue;
             float y[3] = {0.f, 0.f, 0.f};
             if (n.m) t.force(l, n, y);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                res[3 * n.gn + c] = (n.m >> c) & 1 ? n.b[c] - y[c] : 0.f;
-                save[6 * n.t + 3 + c] = n.x[c];
+                res[3 * n.pn + c] = (n.m >> c) & 1 ? n.b[c] - y[c] : 0.f;
+                save[3 * n.pn + c] = n.x[c];
             }
         }
         cluster_sync();
@@ -477,14 +466,14 @@ __global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArg
 
     {  // the coarsest grid: its right-hand side in every CTA, the rows of the inverse shared out
         const Dims d = a.lev[last].d;
-        float* bc = tail_smem + lay.c;
+        float* bc = tail_smem + a.lay.c;
         const float* rf = t.vec(a.lev[last - 1].r, last - 1);
         for (int q = tid; q < 3 * (int)d.nn(); q += TT) {
             const int N = q / 3, c = q - 3 * N;
             const int K = N / ((d.nx + 1) * (d.ny + 1)), J = N / (d.nx + 1) % (d.ny + 1), I = N % (d.nx + 1);
             const unsigned m = __ldg(a.lev[last].nmask + N);
             float v[1];
-            restrict_at<1>(a.lev[last - 1].d, rf, I, J, K, c, v);
+            restrict_at<1>(a.lev[last - 1], rf, I, J, K, c, v);
             bc[q] = (m >> c) & 1 ? v[0] : 0.f;
         }
         __syncthreads();
@@ -517,19 +506,21 @@ __global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArg
 
     for (int l = last - 1; l >= 0; --l) {  // up: add the correction, smooth
         const int deg = a.lev[l].degree;
-        const float* save = tail_smem + lay.save[l];
         t.enter(l);
         const float* xc = t.vec(a.lev[l + 1].x, l + 1);
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
             TailNode& n = t.nd[r];
-            if (n.t < 0) continue;
+            if (n.pn < 0) continue;
+            // the values this thread left on the way down
+            const float* b = l == 0 ? t.vec(a.b0, 0) + 3 * n.gn : t.vec(a.lev[l].b, l) + 3 * n.pn;
+            const float* x = t.vec(a.lev[l].xt, l) + 3 * n.pn;
             float p[3];
-            prolong_at(a.lev[l + 1].d, xc, n.i, n.j, n.k, p);
+            prolong_at(a.lev[l + 1].g.p, xc, n.i, n.j, n.k, p);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                n.b[c] = save[6 * n.t + c];
-                n.x[c] = save[6 * n.t + 3 + c] + ((n.m >> c) & 1 ? p[c] : 0.f);
+                n.b[c] = (n.m >> c) & 1 ? b[c] : 0.f;
+                n.x[c] = x[c] + ((n.m >> c) & 1 ? p[c] : 0.f);
             }
         }
         t.exchange(l);
@@ -538,26 +529,34 @@ __global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArg
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
             const TailNode& n = t.nd[r];
-            if (n.t < 0) continue;
+            if (n.pn < 0) continue;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) xo[3 * n.gn + c] = t.lost ? NAN : n.x[c];  // a lost halo fails the solve
+            for (int c = 0; c < 3; ++c)  // a lost halo fails the solve
+                xo[3 * (l == 0 ? n.gn : n.pn) + c] = t.lost ? NAN : n.x[c];
         }
-        cluster_sync();  // the coarse correction is written; at the end no CTA leaves before its neighbours' stores
+        cluster_sync();  // the correction is written; at the end no CTA leaves before its neighbours' stores
     }
 }
 
 int tail_axis(const Dims& d) { return d.nx >= d.ny && d.nx >= d.nz ? 0 : d.ny >= d.nz ? 1 : 2; }
 
-template <int AXIS>
-bool tail_fits(const TailLevel* lev, int nlev, int ctas, size_t* bytes) {
-    for (int l = 0; l < nlev - 1; ++l) {
-        const Slab<AXIS> g(lev[l].d, 0, ctas);
+// fills the levels' geometry and the layout; false where they exceed a cluster
+bool tail_plan(TailLevel* lev, int nlev, int ctas, int axis, TailLayout* lay) {
+    for (int l = 0; l < nlev; ++l) {
+        TailGeo& g = lev[l].g;
+        if (lev[l].d.nn() > 0xffff) return false;
+        if (l == nlev - 1) {  // the coarsest grid: natural order
+            g.p[0] = 1;
+            g.p[1] = lev[l].d.nx + 1;
+            g.p[2] = g.p[1] * (lev[l].d.ny + 1);
+            continue;
+        }
+        g = slab_geo(axis, lev[l].d, ctas);
         if (lev[l].degree < 1 || lev[l].degree > kTailMaxDegree) return false;
-        if (g.planeN > TT * NPT || g.max_nodes() > TT * NPT || g.max_padded() > 0x7fff) return false;
-        if (g.max_nodes() + 2 * g.planeN > 0xffff) return false;
+        if (max_nodes(g) > TT * NPT || max_padded(g) > 0x7fff || max_nodes(g) + 2 * g.planeN > 0xffff) return false;
     }
-    *bytes = sizeof(float) * (size_t)tail_layout<AXIS>(lev, nlev, ctas).words;
-    return *bytes <= (size_t)kTailMaxSmem;
+    *lay = tail_layout(lev, nlev);
+    return sizeof(float) * (size_t)lay->words <= (size_t)kTailMaxSmem;
 }
 
 cudaLaunchConfig_t tail_config(int ctas, int nrhs, size_t bytes, cudaStream_t s, cudaLaunchAttribute* attr) {
@@ -604,26 +603,19 @@ int vtail_prepare(int* ctas) {
     return ANL_OK;
 }
 
-bool vtail_fits(const TailLevel* lev, int nlev, int ctas) {
-    size_t bytes = 0;
-    switch (tail_axis(lev[0].d)) {
-        case 0: return tail_fits<0>(lev, nlev, ctas, &bytes);
-        case 1: return tail_fits<1>(lev, nlev, ctas, &bytes);
-        default: return tail_fits<2>(lev, nlev, ctas, &bytes);
-    }
+bool vtail_fits(TailLevel* lev, int nlev, int ctas) {
+    TailLayout lay;
+    return tail_plan(lev, nlev, ctas, tail_axis(lev[0].d), &lay);
 }
 
-int launch_vtail(const TailArgs& a, cudaStream_t s) {
+int launch_vtail(const TailArgs& args, cudaStream_t s) {
+    TailArgs a = args;
     const int axis = tail_axis(a.lev[0].d);
-    size_t bytes = 0;
-    const bool ok = a.nlev >= 2 && a.nlev <= kTailMaxLevels &&
-                    (axis == 0 ? tail_fits<0>(a.lev, a.nlev, a.ctas, &bytes)
-                               : axis == 1 ? tail_fits<1>(a.lev, a.nlev, a.ctas, &bytes)
-                                           : tail_fits<2>(a.lev, a.nlev, a.ctas, &bytes));
-    if (!ok) {
+    if (a.nlev < 2 || a.nlev > kTailMaxLevels || !tail_plan(a.lev, a.nlev, a.ctas, axis, &a.lay)) {
         set_error("V-cycle tail: the levels exceed one cluster of %d CTAs", a.ctas);
         return ANL_ERR_BADARG;
     }
+    const size_t bytes = sizeof(float) * (size_t)a.lay.words;
     cudaLaunchAttribute attr;
     cudaLaunchConfig_t cfg = tail_config(a.ctas, std::max(1, a.nrhs), bytes, s, &attr);
     switch (axis) {
