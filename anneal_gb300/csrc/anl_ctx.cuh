@@ -121,12 +121,16 @@ struct anl_ctx {
     float* ainv_hi = nullptr;  // the coarsest dense inverse as float pairs (the tail's coarse solve)
     float* ainv_lo = nullptr;
 #ifndef ANL_CHEB_LO
-#define ANL_CHEB_LO 0.03
+#define ANL_CHEB_LO 0.1
 #endif
 #ifndef ANL_CHEB_LO_COARSE
 #define ANL_CHEB_LO_COARSE 0.002
 #endif
-    // lower ends of the smoothed intervals, as fractions of their upper end (levels 0-1, 2+)
+    // Lower ends of the smoothed intervals, as fractions of their upper end (levels 0-1, 2+). With
+    // two steps 0.1 damps what the next level cannot represent and leaves the rest to it; CG
+    // iterations per solve with 0.03, 0.1, 0.15, 0.2: developed designs at 256x128x128 46.3, 39.0,
+    // 39.7, 48.0, at 97x53x34 23.7, 22.3, 23.0, 24.0; SIMP runs from a uniform design at 256x128x128
+    // 27.0, 26.3, 27.1, 27.9, at 113x41x57 20.2, 19.6, 19.7, 20.2.
     double cheb_lo = ANL_CHEB_LO, cheb_lo_coarse = ANL_CHEB_LO_COARSE;
     // per level: {lambda_max bound, then (c1, c2) for up to kChebMax steps}, read by the
     // smoothing kernels from device memory

@@ -44,9 +44,9 @@ constexpr int kWaitTries = 1 << 20;  // bound of a halo wait
 constexpr int kTailMaxDegree = 16;  // Chebyshev steps per sweep there is room for
 
 // A level's slabs: A x B elements per layer, L layers along the tail's axis, `per` layers to a CTA.
-// Levels of at most kAloneElems elements stay in one CTA: its step (0.8 us at 128 elements, 1.2 at
-// 432) is shorter than a shared one, whose halo flight alone takes 0.7 us.
-constexpr int kAloneElems = 512;
+// Levels of at most kAloneElems elements stay in one CTA: its step (0.9 us at 128 elements)
+// is shorter than a shared one, whose halo flight alone takes 0.7 us; at 432 it is not (2 us).
+constexpr int kAloneElems = 256;
 
 TailGeo slab_geo(int axis, const Dims& d, int ctas) {
     const int n[3] = {d.nx, d.ny, d.nz};
