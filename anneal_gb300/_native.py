@@ -39,7 +39,7 @@ EXPORTS = [
     "anl_sensitivity", "anl_stiffness_scale", "anl_filter_init", "anl_filter_fwd",
     "anl_filter_bwd", "anl_physical", "anl_oc_update", "anl_design_stats", "anl_profile_apply",
     "anl_launch_count", "anl_mg_info", "anl_dot_static",
-    "anl_mc_create", "anl_mc_destroy", "anl_mc_extract", "anl_mc_smooth", "anl_mc_components", "anl_mc_copy",
+    "anl_mc_create", "anl_mc_destroy", "anl_mc_extract", "anl_mc_smooth", "anl_mc_components", "anl_mc_prune", "anl_mc_copy",
     "anl_mc_table", "anl_nn_conv3d", "anl_nn_conv3d_bwd_data", "anl_nn_conv3d_bwd_weight", "anl_nn_gelu_bwd",
     "anl_nn_pool2", "anl_nn_up2", "anl_nn_mse", "anl_nn_adam", "anl_element_stress",
     "anl_vox_create", "anl_vox_destroy", "anl_voxel_fill", "anl_output_field", "anl_choose_level",
@@ -93,6 +93,7 @@ _SIGS = {
     "anl_mc_extract": (I, [P, P, I, I, I, I, D, D, ctypes.POINTER(D), ctypes.POINTER(I64), ctypes.POINTER(I64), P]),
     "anl_mc_smooth": (I, [P, I, D, D, P]),
     "anl_mc_components": (I, [P, P, ctypes.POINTER(I), P]),
+    "anl_mc_prune": (I, [P, D, ctypes.POINTER(I64), ctypes.POINTER(I64), ctypes.POINTER(I64), ctypes.POINTER(D), P]),
     "anl_mc_copy": (I, [P, P, P, P]),
     "anl_mc_table": (I, [P, P]),
     "anl_vox_create": (I, [ctypes.POINTER(P)]),

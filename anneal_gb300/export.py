@@ -5,8 +5,8 @@ element, upsamples it linearly, extracts the level set by marching cubes, applie
 smoothing and drops floating fragments under 1 % of the main body's volume, as the
 reference does with ndimage.zoom, skimage and trimesh. The field work, the extraction (a
 stream compaction over the sample grid), the smoothing and the component labelling run in
-the CUDA library (``anl_mc_*``); the host keeps the per-component volume bookkeeping and the
-final orientation check. The result is a ``trimesh.Trimesh`` when trimesh is installed (the
+the CUDA library (``anl_mc_*``), as do the component volumes and the removal of fragments; the
+host keeps the final orientation check. The result is a ``trimesh.Trimesh`` when trimesh is installed (the
 reference's return type), else a ``Mesh`` with the attributes the reference's callers read.
 """
 import ctypes
@@ -113,6 +113,15 @@ class MarchingCubes:
         N.call("anl_mc_components", self.h, ctypes.c_void_p(lab.data_ptr()), ctypes.byref(rounds), _stream())
         return lab[:self.nf]
 
+    def prune(self, fraction):
+        """Drops the components under `fraction` of the largest one's volume. Returns (components
+        dropped, signed volume of the rest)."""
+        nv, nf, dropped, vol = ctypes.c_int64(), ctypes.c_int64(), ctypes.c_int64(), ctypes.c_double()
+        N.call("anl_mc_prune", self.h, float(fraction), ctypes.byref(nv), ctypes.byref(nf), ctypes.byref(dropped),
+               ctypes.byref(vol), _stream())
+        self.nv, self.nf = nv.value, nf.value
+        return dropped.value, vol.value
+
     def mesh_device(self):
         v = torch.empty((max(self.nv, 1), 3), dtype=torch.float32, device="cuda")
         f = torch.empty((max(self.nf, 1), 3), dtype=torch.int32, device="cuda")
@@ -143,29 +152,16 @@ def surface(grid, f, level, upsample=2, smooth=10, log=print):
         mc.extract(field, grid.shape, level, grid.h, grid.origin, upsample)
         if smooth > 0:
             mc.smooth(int(smooth))
-        lab = mc.components()
+        # export.py:135-141: drop fragments under 1 % of the largest component's volume
+        dropped, volume = mc.prune(FRAGMENT_FRACTION)
+        if dropped:
+            log(f"  removed {dropped} floating fragment(s) under 1 % of the main body")
         v, fc = mc.mesh_device()
         verts = v.double().cpu().numpy()
         faces = fc.long().cpu().numpy()
-        labels = lab.long().cpu().numpy()
     finally:
         mc.close()
-    # export.py:135-141: drop fragments under 1 % of the largest component's volume
-    uniq, comp = np.unique(labels, return_inverse=True)
-    if uniq.size > 1:
-        t = verts[faces]
-        tv = np.einsum("ij,ij->i", t[:, 0], np.cross(t[:, 1], t[:, 2])) / 6.0
-        vols = np.abs(np.bincount(comp, weights=tv, minlength=uniq.size))
-        keep = vols >= FRAGMENT_FRACTION * vols.max()
-        if not keep.all():
-            log(f"  removed {int((~keep).sum())} floating fragment(s) under 1 % of the main body")
-            faces = faces[keep[comp]]
-            used, inv = np.unique(faces.ravel(), return_inverse=True)
-            verts = verts[used]
-            faces = inv.reshape(-1, 3)
-    mesh = Mesh(verts, faces)
-    if mesh.volume < 0:   # export.py:145-146
-        mesh = Mesh(verts, faces[:, ::-1])
+    mesh = Mesh(verts, faces if volume >= 0 else faces[:, ::-1])   # export.py:145-146
     try:
         import trimesh
         return trimesh.Trimesh(mesh.vertices, mesh.faces, process=False)

@@ -202,6 +202,14 @@ int anl_mc_smooth(anl_mc* mc, int iterations, double lamb, double mu, anl_stream
    hook-and-jump rounds to *rounds_h when it is not NULL. */
 int anl_mc_components(anl_mc* mc, int32_t* face_label, int* rounds_h, anl_stream_t stream);
 
+/* Replaces the fragment removal of export.surface (export.py:135-141): drops every component whose
+   |signed volume| is below `fraction` of the largest one's. The current mesh becomes the kept
+   components, vertices and faces in their order (as numpy's unique and boolean indexing give
+   them; untouched when nothing is dropped); writes its counts, the number of components dropped
+   and its signed volume (host). A volume that is no number drops everything. */
+int anl_mc_prune(anl_mc* mc, double fraction, int64_t* nverts_h, int64_t* nfaces_h, int64_t* dropped_h, double* volume_h,
+                 anl_stream_t stream);
+
 /* Copies the current mesh out: verts 3*nverts floats, faces 3*nfaces int32 (device or
    pinned host pointers). */
 int anl_mc_copy(anl_mc* mc, float* verts, int32_t* faces, anl_stream_t stream);
