@@ -524,8 +524,8 @@ __global__ void k_oc_scale(int64_t ne, const uint8_t* active, const uint8_t* fro
 // two neighbouring floats are known with the volume above the target at the lower one and not
 // above it at the upper one: its midpoints then fall on either side without another volume.
 // Each pass evaluates the volume at a bank of lambdas inside the bracket known so far and its last
-// block narrows the bracket and picks the next bank (oc_advance): 4-5 passes of 15 or 6-7 passes
-// of 3 lambdas instead of one volume for each of the 36 steps.
+// block narrows the bracket and picks the next bank (oc_advance): 4 passes of 15 or 5-7 passes of 3
+// lambdas instead of one volume for each of the 36 steps.
 //  * No projection: the volume is linear in xn, vol = sum_j wv_j xn_j + sum_frozen phi, with
 //    wv = Filter.backward(phi on non-frozen elements): k_oc_vol_bank, a stream over the elements,
 //    issue-bound at 15 lambdas (about 8 instructions per lambda and element).
@@ -569,9 +569,10 @@ struct OcState {
     double lo, hi, lam;  // the bisection's first bracket; its last midpoint
     double vfrozen, vtarget;
     int steps, stop;
-    int tlo, thi;        // bits of the largest lambda known above the target volume (-1: none yet), of
-                         // the smallest one not above it (INT_MAX: none yet)
-    double flo, fhi;     // their volumes
+    int tlo, thi;        // bits of the largest lambda known above the target volume and of the smallest
+                         // one not above it; next to the bisection's bracket while not known
+    int width;           // the interval before the last pass (0: a side was not known)
+    double flo, fhi;     // their volumes (NaN: not known)
     OcBank bank;         // the lambdas of the next pass
 };
 
@@ -579,23 +580,26 @@ struct OcState {
 // bank of at most nmax lambdas
 __device__ void oc_advance(OcState* st, const double* vols, int nmax, int lane) {
     int tlo = st->tlo, thi = st->thi;
-    const int n = st->bank.n;
-    const int64_t width = (int64_t)thi - tlo;
+    const int n = st->bank.n, width = st->width;
     double flo = st->flo, fhi = st->fhi;
-    const double target = st->vtarget, frozen = st->vfrozen;
-    for (int j = 0; j < n; ++j) {
-        const int p = __float_as_int(st->bank.lam[j]);
-        const double v = vols[j] + frozen;
-        if (v > target && p > tlo) tlo = p, flo = v;
+    const double target = st->vtarget;
+    // a lane per lambda: the largest above the target, then the smallest not above it beyond that
+    const int pj = lane < n ? __float_as_int(st->bank.lam[lane]) : -1;
+    const double vj = lane < n ? vols[lane] + st->vfrozen : 0.0;
+    const bool above = vj > target;
+    const int up = __reduce_max_sync(0xffffffffu, lane < n && above ? pj : -1);
+    if (up > tlo) {
+        tlo = up;
+        flo = __shfl_sync(0xffffffffu, vj, __ffs(__ballot_sync(0xffffffffu, lane < n && above && pj == up)) - 1);
     }
-    for (int j = 0; j < n; ++j) {
-        const int p = __float_as_int(st->bank.lam[j]);
-        const double v = vols[j] + frozen;
-        if (!(v > target) && p > tlo && p < thi) thi = p, fhi = v;
+    const bool low = lane < n && !above && pj > tlo;
+    const int dn = __reduce_min_sync(0xffffffffu, low ? pj : INT_MAX);
+    if (dn < thi) {
+        thi = dn;
+        fhi = __shfl_sync(0xffffffffu, vj, __ffs(__ballot_sync(0xffffffffu, low && pj == dn)) - 1);
     }
-    __syncwarp();
-    // the first bank holds both ends of the bisection's bracket: a missing side has no lambda
-    if (tlo < 0 || thi == INT_MAX || thi - tlo <= 1) {
+    const int gap = thi - tlo - 1;
+    if (gap <= 0) {
         if (lane == 0) {  // the bisection's own steps, each decided by the bracket
             double lo = st->lo, hi = st->hi, lam = st->lam;
             int steps = 0;
@@ -611,19 +615,24 @@ __device__ void oc_advance(OcState* st, const double* vols, int nmax, int lane) 
         }
         return;
     }
-    // Inside: every float while they fit the bank; else around the zero of the line through the
-    // two ends (the line's error shrinks with the square of the interval), at doubling distances;
-    // else, where the last pass narrowed the bracket by less than 4, at even distances.
-    const int gap = thi - tlo - 1, m = min(nmax, gap), h = (m - 1) / 2;
+    // Next: from a known side towards the other end in octaves 2, 8, 32, ...; every float while they
+    // fit the bank; around the zero of the line through the two ends (its error shrinks with the
+    // square of the interval) at doubling distances; or, where that did not halve the interval, at
+    // even distances
+    const int m = min(nmax, gap), h = (m - 1) / 2;
+    const bool known = !isnan(flo) && !isnan(fhi);
     int p;
     if (gap <= nmax) {
         p = tlo + 1 + lane;
-    } else if (thi - tlo > width / 4 && width < INT_MAX) {
+    } else if (!known) {
+        const long long d = 2ll << (23 + 2 * min(lane, 8));
+        p = isnan(fhi) ? (int)min(tlo + d, (long long)thi - 1) : (int)max(thi - d, (long long)tlo + 1);
+    } else if (width > 0 && thi - tlo > width / 2) {
         p = tlo + (int)((int64_t)(thi - tlo) * (lane + 1) / (m + 1));
     } else {
         const double d = thi - tlo;
         const int r = max(tlo + 1, min(thi - 1, tlo + (int)(d * ((flo - target) / (flo - fhi)))));
-        const double near = fmax(1.0, fmin(d * d * (1.0 / 8388608.0 / 256.0), d / (double)(1 << h)));
+        const double near = fmax(1.0, fmin(d * d * (1.0 / 8388608.0 / 16.0), d / (double)(1 << h)));
         const int t = lane - h;
         const double off = t == 0 ? 0.0 : near * (double)(1 << (min(abs(t), 16) - 1));
         p = t < 0 ? r - (int)off : r + (int)off;
@@ -634,12 +643,13 @@ __device__ void oc_advance(OcState* st, const double* vols, int nmax, int lane) 
         st->bank.n = m;
         st->tlo = tlo;
         st->thi = thi;
+        st->width = known ? thi - tlo : 0;
         st->flo = flo;
         st->fhi = fhi;
     }
 }
 
-// one warp: the bisection's bracket and the first bank, denser around the mean ratio
+// one warp: the bisection's bracket and the first bank, two octaves around the mean ratio
 __global__ void k_oc_begin(OcState* st, const double* sums, const double* vfrozen, double vtarget, int n) {
     const int lane = threadIdx.x;
     // optimize.py:145: the bracket from the mean sensitivities of the design elements
@@ -650,12 +660,11 @@ __global__ void k_oc_begin(OcState* st, const double* sums, const double* vfroze
         scale = fmax(mdc / fmax(mdv, 1e-30), 1e-300);
     }
     const double lo = scale * 1e-8, hi = scale * 1e8;
+    const int a = __float_as_int((float)lo), b = __float_as_int((float)hi), c = __float_as_int((float)scale);
     if (lane < n) {
-        const int h = (n - 1) / 2, t = lane - h;
-        const int a = __float_as_int((float)lo), b = __float_as_int((float)hi), c = __float_as_int((float)scale);
-        const double u = (double)t / h, off = u * u * u;
-        const int p = c + (int)(off * (t < 0 ? c - a : b - c));
-        st->bank.lam[lane] = __int_as_float(t == -h ? a : t == h ? b : p);
+        const int h = (n - 1) / 2;
+        const long long p = c + (2ll << 23) * (lane - h) / h;
+        st->bank.lam[lane] = __int_as_float((int)max((long long)a, min((long long)b, p)));
     }
     if (lane == 0) {
         st->lo = lo;
@@ -665,9 +674,10 @@ __global__ void k_oc_begin(OcState* st, const double* sums, const double* vfroze
         st->vtarget = vtarget;
         st->steps = 0;
         st->stop = 0;
-        st->tlo = -1;
-        st->thi = INT_MAX;
-        st->flo = st->fhi = 0.0;
+        st->tlo = a - 1;
+        st->thi = b + 1;
+        st->width = 0;
+        st->flo = st->fhi = NAN;
         st->bank.n = n;
     }
 }
@@ -713,12 +723,9 @@ __global__ void __launch_bounds__(OCB_T, 1) k_oc_vol_bank(int64_t ne, const floa
     float lo[OC_BANK];
 #pragma unroll
     for (int j = 0; j < OC_BANK; ++j) lo[j] = 0.f;
-    block_pair_sum<OC_BANK, OCB_T>(acc, lo, sm, threadIdx.x);
-    if (finish_pair_reduction<OC_BANK, OCB_T>(acc, lo, blockIdx.x, gridDim.x, partials, counter, out, threadIdx.x, sm) &&
-        threadIdx.x < 32) {
-        __syncwarp();  // lane 0 wrote the volumes
+    if (reduce_pairs_wide<OC_BANK, OCB_T>(acc, lo, blockIdx.x, gridDim.x, partials, counter, out, threadIdx.x, sm) &&
+        threadIdx.x < 32)
         oc_advance(st, out, OC_BANK, threadIdx.x);
-    }
 }
 
 // One pass with projection: the volume sum phi physical(xn(lambda)) of each lambda of the bank,
@@ -815,13 +822,10 @@ __global__ void __launch_bounds__(FT_N) k_oc_vol_proj(OcProjArgs a) {
         h[m] = vol[m].h;
         l[m] = vol[m].l;
     }
-    block_pair_sum<OC_PROJ, FT_N>(h, l, sm, tid);
     const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    if (finish_pair_reduction<OC_PROJ, FT_N>(h, l, bid, gridDim.x * gridDim.y * gridDim.z, a.partials, a.counter, a.out,
-                                             tid, sm) && tid < 32) {
-        __syncwarp();  // lane 0 wrote the volumes
+    if (reduce_pairs_wide<OC_PROJ, FT_N>(h, l, bid, gridDim.x * gridDim.y * gridDim.z, a.partials, a.counter, a.out, tid,
+                                         sm) && tid < 32)
         oc_advance(a.st, a.out, OC_PROJ, tid);
-    }
 }
 
 __global__ void k_oc_weights(int64_t ne, const uint8_t* active, const uint8_t* frozen, const float* phi, float* v,
@@ -902,8 +906,8 @@ int oc_update(anl_ctx* c, const float* x, const float* dcx, const float* dvx, co
         }
     }
     // the usual number of passes at once (a pass after the last decision returns at once), then
-    // two more at a time: every pass or the one after it narrows the bracket fourfold
-    int passes = linear ? 5 : 7;
+    // two more at a time: every pass or the one after it narrows the bracket at least to half
+    int passes = linear ? 4 : 6;
     for (int done = 0; done < 80; done += passes, passes = 2) {
         for (int q = 0; q < passes; ++q) {
             if (linear) {
