@@ -26,13 +26,14 @@ __global__ void __launch_bounds__(128) k_ku64_elements(Dims d, const float* __re
     const int64_t n0 = d.node(i, j, k), sy = d.nx + 1, sz = sy * (d.ny + 1);
     const double Ee = E[e];
     V3<double> f[2][2][2];
-    if (Ee != 0.0 && ANL_IN_RANGE(n0 + 1 + sy + sz, d.nn())) {
-        V3<double> v[2][2][2];
+    V3<double> v[2][2][2];  // loaded whatever the scale: one latency for both
+    if (!ANL_IN_RANGE(n0 + 1 + sy + sz, d.nn())) return;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const double* p = u + 3 * (n0 + (q & 1) + ((q >> 1) & 1) * sy + (q >> 2) * sz);
-            v[q & 1][(q >> 1) & 1][q >> 2] = V3<double>{{p[0], p[1]}, p[2]};
-        }
+    for (int q = 0; q < 8; ++q) {
+        const double* p = u + 3 * (n0 + (q & 1) + ((q >> 1) & 1) * sy + (q >> 2) * sz);
+        v[q & 1][(q >> 1) & 1][q >> 2] = V3<double>{{p[0], p[1]}, p[2]};
+    }
+    if (Ee != 0.0) {
         V3<double> dxb[2], dxt[2], dyb[2], dyt[2], dz[2][2];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -71,15 +72,23 @@ __global__ void __launch_bounds__(NT64) k_ku64_nodes(KuArgs<double> a, const dou
         const int NX = d.nx + 1, NY = d.ny + 1;
         const int i = n % NX, j = n / NX % NY, k = n / (NX * NY);
         const uint8_t nm = a.nmask[n];
-        double y[3] = {0.0, 0.0, 0.0};
+        // all loads in flight together; corners outside the grid are read at an element inside
+        double f[8][3];
+        bool in[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const int ie = i - (q & 1), je = j - ((q >> 1) & 1), ke = k - (q >> 2);
-            if (ie < 0 || je < 0 || ke < 0 || ie >= d.nx || je >= d.ny || ke >= d.nz) continue;
-            const double* p = F + (int64_t)(3 * q) * ne + (ie + d.nx * (je + d.ny * ke));
+            in[q] = ie >= 0 && je >= 0 && ke >= 0 && ie < d.nx && je < d.ny && ke < d.nz;
+            const double* p = F + (int64_t)(3 * q) * ne + (in[q] ? ie + d.nx * (je + d.ny * ke) : 0);
 #pragma unroll
-            for (int c = 0; c < 3; ++c) y[c] += p[(int64_t)c * ne];
+            for (int c = 0; c < 3; ++c) f[q][c] = p[(int64_t)c * ne];
         }
+        double y[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (in[q])
+#pragma unroll
+                for (int c = 0; c < 3; ++c) y[c] += f[q][c];
         const int64_t n3 = 3 * (int64_t)n;
         const double inv = MODE == KU_CHEB ? (double)a.diag[n] : 0.0;
         const double c1 = MODE == KU_CHEB && !a.c1_zero ? a.cheb[0] : 0.0, c2 = MODE == KU_CHEB ? a.cheb[1] : 0.0;
