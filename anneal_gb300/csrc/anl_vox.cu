@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(VOX_T) k_vox_zrange(const double* __restrict__
 // xs, ys: sample coordinates (geometry.py:91-94); zq: normalised, clipped sample heights
 // (geometry.py:144); zs_out[0..1] = zlo, zr
 __global__ void __launch_bounds__(VOX_T) k_vox_axes(VoxGrid G, const unsigned long long* zmm, double* xs,
-                                                    double* ys, double* zq, double* zs_out) {
+                                                    double* ys, double* zq, double* frac, double* zs_out) {
     const double zlo = dunkey(zmm[0]), zhi = dunkey(zmm[1]);
     const double zr = __dadd_rn(__dmul_rn(__dsub_rn(zhi, zlo), 1.001), 1e-9);
     const int n = G.nxs + G.nys + G.nzs;
@@ -98,6 +98,9 @@ __global__ void __launch_bounds__(VOX_T) k_vox_axes(VoxGrid G, const unsigned lo
             zq[m] = fmin(fmax(q, 0.0), 0.999999);
         }
     }
+    // the fill fractions of 0..s^3 samples: k_vox_fill's divisions, once
+    const int n3 = G.s * G.s * G.s;
+    for (int c = blockIdx.x * VOX_T + threadIdx.x; c <= n3; c += gridDim.x * VOX_T) frac[c] = (double)c / (double)n3;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         zs_out[0] = zlo;
         zs_out[1] = zr;
@@ -220,12 +223,12 @@ __global__ void __launch_bounds__(VOX_T) k_vox_parity(VoxGrid G, unsigned* __res
     }
 }
 
-// fill fraction per element (x fastest): inside samples / s^3 (geometry.py:147-149)
+// fill fraction per element (x fastest): inside samples / s^3 (geometry.py:147-149), the quotient
+// from a table: an FP64 division per element took 18 of the kernel's 26 us at 128x64x64
 __global__ void __launch_bounds__(VOX_T) k_vox_fill(VoxGrid G, const unsigned* __restrict__ bits,
-                                                    double* __restrict__ fill) {
+                                                    const double* __restrict__ frac, double* __restrict__ fill) {
     const int64_t ne = (int64_t)G.nx * G.ny * G.nz;
     const unsigned mask = (G.s >= 32) ? ~0u : ((1u << G.s) - 1u);
-    const double n3 = (double)(G.s * G.s * G.s);
     for (int64_t e = blockIdx.x * (int64_t)VOX_T + threadIdx.x; e < ne; e += (int64_t)gridDim.x * VOX_T) {
         const int i = (int)(e % G.nx);
         const int64_t r = e / G.nx;
@@ -240,7 +243,7 @@ __global__ void __launch_bounds__(VOX_T) k_vox_fill(VoxGrid G, const unsigned* _
                 if (two) x |= bits[(int64_t)(w + 1) * G.ncol + c] << (32 - sh);
                 count += __popc(x & mask);
             }
-        fill[e] = (double)count / n3;
+        fill[e] = frac[count];
     }
 }
 
@@ -259,7 +262,7 @@ struct anl_vox {
     size_t cnt_cap = 0;
     long long* off = nullptr;
     size_t off_cap = 0;
-    double* axes = nullptr;  // xs | ys | zq
+    double* axes = nullptr;  // xs | ys | zq | fill fractions
     size_t axes_cap = 0;
     unsigned* bits = nullptr;
     size_t bits_cap = 0;
@@ -337,18 +340,19 @@ int anl_voxel_fill(anl_vox* v, const double* tri, int64_t ntri, int nx, int ny, 
     ANL_TRY(grow(v->box, v->box_cap, (size_t)ntri, sizeof(int4)));
     ANL_TRY(grow(v->cnt, v->cnt_cap, (size_t)ntri, sizeof(long long)));
     ANL_TRY(grow(v->off, v->off_cap, (size_t)ntri, sizeof(long long)));
-    ANL_TRY(grow(v->axes, v->axes_cap, (size_t)(nxs + nys + nzs), sizeof(double)));
+    ANL_TRY(grow(v->axes, v->axes_cap, (size_t)(nxs + nys + nzs + s * s * s + 1), sizeof(double)));
     ANL_TRY(grow(v->bits, v->bits_cap, nbits, sizeof(unsigned)));
     double* xs = v->axes;
     double* ys = xs + nxs;
     double* zq = ys + nys;
+    double* frac = zq + nzs;
     double* zs = (double*)(v->sc + 4);
     ANL_CUDA(cudaMemsetAsync(v->sc, 0xff, sizeof(unsigned long long), st));
     ANL_CUDA(cudaMemsetAsync(v->sc + 1, 0, 3 * sizeof(unsigned long long), st));
     ANL_CUDA(cudaMemsetAsync(v->bits, 0, nbits * sizeof(unsigned), st));
     k_vox_zrange<<<vox_blocks(3 * ntri), VOX_T, 0, st>>>(tri, ntri, v->sc);
     ANL_LAUNCH_CHECK();
-    k_vox_axes<<<vox_blocks(nxs + nys + nzs), VOX_T, 0, st>>>(G, v->sc, xs, ys, zq, zs);
+    k_vox_axes<<<vox_blocks(nxs + nys + nzs), VOX_T, 0, st>>>(G, v->sc, xs, ys, zq, frac, zs);
     ANL_LAUNCH_CHECK();
     k_vox_count<<<vox_blocks(ntri), VOX_T, 0, st>>>(tri, ntri, G, xs, ys, v->box, v->cnt);
     ANL_LAUNCH_CHECK();
@@ -358,7 +362,7 @@ int anl_voxel_fill(anl_vox* v, const double* tri, int64_t ntri, int nx, int ny, 
     ANL_LAUNCH_CHECK();
     k_vox_parity<<<vox_blocks(G.ncol), VOX_T, 0, st>>>(G, v->bits);
     ANL_LAUNCH_CHECK();
-    k_vox_fill<<<vox_blocks((int64_t)nx * ny * nz), VOX_T, 0, st>>>(G, v->bits, fill);
+    k_vox_fill<<<vox_blocks((int64_t)nx * ny * nz), VOX_T, 0, st>>>(G, v->bits, frac, fill);
     ANL_LAUNCH_CHECK();
     if (stats_h) {
         ANL_CUDA(cudaMemcpyAsync(v->host, v->sc + 2, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
