@@ -727,6 +727,11 @@ struct PcgScalars {
     double rr;      // ||r||^2
     double bb;      // ||b||^2
     double alpha;
+    // the next step's alpha and beta in both precisions, formed by the reductions' last thread (a
+    // division in every thread of a full grid is 6 us of FP64 on this part)
+    double step, beta;
+    float step_f, beta_f;
+    int step_bad;   // p.K p is not positive, or alpha no number
     double tol2;    // (rtol ||b||)^2
     double rr_true; // ||b - K x||^2 from the last residual replacement
     int done;       // 0 running, 1 converged, 2 maxiter, 3 non-finite, 4 breakdown; every
@@ -735,6 +740,20 @@ struct PcgScalars {
     int nonfinite;  // a non-finite scalar was seen
     int maxiter;
 };
+
+#ifdef __CUDACC__
+// after pq: alpha = r.z / p.K p (one thread)
+__device__ __forceinline__ void pcg_set_step(PcgScalars* sc) {
+    const double pq = sc->pq, v = sc->rz[sc->iters & 1] / pq;
+    sc->step = v;
+    sc->step_f = (float)v;
+    sc->step_bad = !(pq > 0.0) || !isfinite(v);
+}
+__device__ __forceinline__ float pcg_step(const PcgScalars* sc, float) { return sc->step_f; }
+__device__ __forceinline__ double pcg_step(const PcgScalars* sc, double) { return sc->step; }
+__device__ __forceinline__ float pcg_beta(const PcgScalars* sc, float) { return sc->beta_f; }
+__device__ __forceinline__ double pcg_beta(const PcgScalars* sc, double) { return sc->beta; }
+#endif
 
 inline int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 

@@ -66,6 +66,7 @@ struct KuArgs {
     unsigned* counter = nullptr;
     int partial_capacity = 0;
     double* red_out = nullptr;       // APPLY_DOT: u . K u
+    PcgScalars* sc = nullptr;        // APPLY_DOT in CG: the scalars whose pq red_out is (alpha follows)
     const int* done = nullptr;       // early-exit flag of the CG loop (may be null)
     // batch of right-hand sides (grid.y): slot r reads and writes its nodal vectors at
     // + r * vstride values, its done flag and dot at + r * sc_bytes bytes, its reduction scratch
@@ -98,6 +99,7 @@ __host__ __device__ __forceinline__ void ku_to_slot(KuArgs<T>& a, int r) {
     a.xout = slot_ptr(a.xout, r, a.vstride);
     a.done = slot_bytes(a.done, r, a.sc_bytes);
     a.red_out = slot_bytes(a.red_out, r, a.sc_bytes);
+    a.sc = slot_bytes(a.sc, r, a.sc_bytes);
     a.partials = slot_ptr(a.partials, r, a.part_stride);
     a.counter = slot_ptr(a.counter, r, (int64_t)1);
 }

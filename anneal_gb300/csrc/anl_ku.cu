@@ -511,12 +511,16 @@ __global__ void __launch_bounds__(KmCfg<T>::NT, KmCfg<T>::MINB) ku_kernel(KuArgs
         if constexpr (std::is_same<T, double>::value) {
             double v[1] = {dot.value()};
             block_sum<1, NT>(v, sred, tid);
-            finish_reduction<1, NT>(v, blockIdx.x, gridDim.x, a.partials, a.counter, a.red_out, tid, sred);
+            if (finish_reduction<1, NT>(v, blockIdx.x, gridDim.x, a.partials, a.counter, a.red_out, tid, sred) &&
+                tid == 0 && a.sc != nullptr)
+                pcg_set_step(a.sc);
         } else {
             float h[1] = {dot.a.s}, l[1] = {dot.a.c};
             float2* sp = reinterpret_cast<float2*>(sred);
             block_pair_sum<1, NT>(h, l, sp, tid);
-            finish_pair_reduction<1, NT>(h, l, blockIdx.x, gridDim.x, a.partials, a.counter, a.red_out, tid, sp);
+            if (finish_pair_reduction<1, NT>(h, l, blockIdx.x, gridDim.x, a.partials, a.counter, a.red_out, tid, sp) &&
+                tid == 0 && a.sc != nullptr)
+                pcg_set_step(a.sc);
         }
     }
 }

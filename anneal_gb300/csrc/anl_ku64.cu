@@ -116,7 +116,9 @@ __global__ void __launch_bounds__(NT64) k_ku64_nodes(KuArgs<double> a, const dou
     if (MODE == KU_APPLY_DOT) {
         double v[1] = {dot};
         block_sum<1, NT64>(v, sred, threadIdx.x);
-        finish_reduction<1, NT64>(v, blockIdx.x, gridDim.x, a.partials, a.counter, a.red_out, threadIdx.x, sred);
+        if (finish_reduction<1, NT64>(v, blockIdx.x, gridDim.x, a.partials, a.counter, a.red_out, threadIdx.x, sred) &&
+            threadIdx.x == 0 && a.sc != nullptr)
+            pcg_set_step(a.sc);
     }
 }
 

@@ -30,6 +30,10 @@ namespace anl {
 constexpr int VT = 256;  // threads of the 1D vector kernels
 
 static inline int vgrid(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>(kRedBlocks, (n + VT - 1) / VT)); }
+// The kernels that walk four values at a time: a group of four for every thread at most. (With vgrid,
+// three blocks of four had nothing to do but their part of the reduction: per CG iteration 286 us
+// instead of 249 with six load cases of 80x40x40, 198 instead of 188 at 96x48x48.)
+static inline int vgrid4(int64_t n) { return vgrid(n / 4); }
 
 // ------------------------------------------------------------------ accumulators
 
@@ -674,6 +678,9 @@ __global__ void k_init_scalars(PcgScalars* sc, double rtol, int maxiter, const d
     sc->maxiter = maxiter;
     sc->rz[0] = sc->rz[1] = 0.0;
     sc->alpha = 0.0;
+    sc->step = sc->beta = 0.0;
+    sc->step_f = sc->beta_f = 0.f;
+    sc->step_bad = 0;
     sc->zq = 0.0;
     sc->pq = 0.0;
 }
@@ -703,6 +710,16 @@ __device__ __forceinline__ void for_each4(int64_t n, F4 f4, F1 f1) {
     const int64_t n4 = n >> 2;
     for (int64_t g = t; g < n4; g += stride) f4(4 * g);
     for (int64_t i = 4 * n4 + t; i < n; i += stride) f1(i);
+}
+// the same from the end: each vector kernel of a CG iteration walks against the one before it, so that
+// it starts on the values that one left in the L2 (129 MB; the five vectors of 256x128x128 are 240 MB,
+// and an iteration there takes 853 us with k_pupdate and k_axpy backwards, 870 all forwards)
+template <class F4, class F1>
+__device__ __forceinline__ void for_each4_back(int64_t n, F4 f4, F1 f1) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t n4 = n >> 2;
+    for (int64_t i = 4 * n4 + t; i < n; i += stride) f1(i);
+    for (int64_t g = n4 - 1 - t; g >= 0; g -= stride) f4(4 * g);
 }
 
 template <class T>
@@ -749,6 +766,8 @@ __global__ void k_dots_rz_zq(int64_t n, const T* r, const T* z, const T* q, PcgS
             const int it = sc->iters;
             sc->rz[it & 1] = res[0];
             sc->zq = res[1];
+            sc->beta = -sc->alpha * res[1] / sc->rz[(it + 1) & 1];  // flexible; not read on a restart
+            sc->beta_f = (float)sc->beta;
             if (!isfinite(res[0]) || !isfinite(res[1])) {
                 sc->done = 3;
                 sc->nonfinite = 1;
@@ -766,9 +785,8 @@ __global__ void k_pupdate(int64_t n, const T* z, T* p, const PcgScalars* sc, con
     sc += blockIdx.y;
     restart += blockIdx.y;
     if (sc->done) return;
-    const int it = sc->iters;
     if (*restart) {  // p = z (not z + 0 p: p may hold non-finite values after a breakdown)
-        for_each4(
+        for_each4_back(
             n,
             [&](int64_t i) {
                 T zv[4];
@@ -778,8 +796,8 @@ __global__ void k_pupdate(int64_t n, const T* z, T* p, const PcgScalars* sc, con
             [&](int64_t i) { p[i] = z[i]; });
         return;
     }
-    const T bt = T(-sc->alpha * sc->zq / sc->rz[(it + 1) & 1]);
-    for_each4(
+    const T bt = pcg_beta(sc, T(0));
+    for_each4_back(
         n,
         [&](int64_t i) {
             T zv[4], pv[4];
@@ -811,14 +829,13 @@ __global__ void k_axpy(int64_t n, const T* p, const T* q, double* x, T* r, PcgSc
     }
     if (sc->done) return;
     const int it = sc->iters;
-    const double pq = sc->pq;
-    const double alpha = sc->rz[it & 1] / pq;
-    const bool bad = !(pq > 0.0) || !isfinite(alpha);
+    const double alpha = sc->step;
+    const bool bad = sc->step_bad != 0;
     Sum<T> rr1[1];
     Sum<T>& rr = rr1[0];
     if (!bad) {
-        const T at = T(alpha);
-        for_each4(
+        const T at = pcg_step(sc, T(0));
+        for_each4_back(
             n,
             [&](int64_t i) {
                 T pv[4], qv[4], rv[4];
@@ -851,7 +868,7 @@ __global__ void k_axpy(int64_t n, const T* p, const T* q, double* x, T* r, PcgSc
             sc->iters = it + 1;
             *restart = 0;
             if (bad) {
-                if (isfinite(pq) && isfinite(alpha)) sc->done = 4;
+                if (isfinite(sc->pq) && isfinite(alpha)) sc->done = 4;
                 else {
                     sc->done = 3;
                     sc->nonfinite = 1;
@@ -880,6 +897,8 @@ KeModal<float> modal_of<float>(const anl_ctx* c) { return c->kmf; }
 template <>
 KeModal<double> modal_of<double>(const anl_ctx* c) { return c->kmd; }
 
+__global__ void k_set_step(PcgScalars* sc) { pcg_set_step(sc); }
+
 // The K u passes of the finest level go to the tensor-core kernel (anl_kutc.cu) when the
 // context enables it (FP32 contexts); every other level and precision uses the SIMT kernel.
 template <class T>
@@ -888,7 +907,12 @@ static int ku_pass(anl_ctx* c, const Level& L, int mode, const KuArgs<T>& a, cud
         if (c->use_tc && c->rb == 1 && &L == &c->lev[0]) {
             KuArgs<float> t = a;
             t.diag = L.diag;
-            return launch_kutc(mode, t, c->kmf, s);
+            ANL_TRY(launch_kutc(mode, t, c->kmf, s));
+            if (mode == KU_APPLY_DOT && a.sc != nullptr) {
+                k_set_step<<<1, 1, 0, s>>>(a.sc);
+                ANL_LAUNCH_CHECK();
+            }
+            return ANL_OK;
         }
     }
     if constexpr (std::is_same<T, double>::value) {
@@ -946,6 +970,7 @@ static int apply_level(anl_ctx* c, const Level& L, const T* u, T* y, cudaStream_
     a.y = y;
     a.done = done;
     a.red_out = dot_out;
+    if (dot_out != nullptr && dot_out == &c->sc->pq) a.sc = c->sc;
     return ku_pass<T>(c, L, dot_out ? KU_APPLY_DOT : KU_APPLY, a, s);
 }
 
@@ -1277,7 +1302,7 @@ static int enqueue_chunk(anl_ctx* c, int chunk, cudaStream_t s) {
     int* restart = c->restart_d + c->slot;
     const int* done = &c->sc->done;
     const Bt bt = bt_of(c, L0);
-    const dim3 vg(vgrid(n), c->rb);
+    const dim3 vg(vgrid4(n), c->rb);
     for (int k = 0; k < chunk; ++k) {
         ANL_TRY(vcycle<T>(c, 0, done, s));
         const T* z = (const T*)L0.x;
