@@ -573,11 +573,15 @@ int launch_ku(int mode, const KuArgs<T>& args, const KeModal<T>& km, cudaStream_
         case KU_APPLY_RAW: resident = ku_resident<T, KU_APPLY_RAW>(); break;
         default: return ANL_ERR_BADARG;
     }
-    // one wave of CTAs per right-hand side. A segment costs one extra element layer, but a
-    // plane step is a ~1 us latency chain, so small (coarse-level) grids spread over many short
-    // segments. Every slot of a batch gets the partition a single solve gets, so its sums (the
-    // p.Kp reduction follows the CTAs) and its iterates are those of its own solve.
-    const int per_rhs = std::max(1, resident);
+    // One wave of CTAs. A segment costs one extra element layer and its ring prologue, and a plane
+    // step is a ~1 us latency chain, so small (coarse-level) grids spread over many short segments.
+    // Where the pass sums (the p.Kp reduction follows the CTAs) every slot of a batch gets the
+    // partition a single solve gets, so its iterates are those of its own solve. The other passes
+    // give a node the same value in any partition, so the slots share the wave (per CG iteration of
+    // six load cases of 80x40x40: 237 us, 249 with a wave each), unless the shares are so small that
+    // the remainder leaves more than an eighth of it idle.
+    const int nrhs = std::max(1, a.nrhs);
+    const int per_rhs = mode != KU_APPLY_DOT && nrhs <= resident / 8 ? resident / nrhs : std::max(1, resident);
     a.kz = (int)std::max<int64_t>(2, (total + per_rhs - 1) / per_rhs);
     const int blocks = (int)((total + a.kz - 1) / a.kz);
     dim3 block(32, KmCfg<T>::NW);
