@@ -270,6 +270,23 @@ static void free_ctx(anl_ctx* c) {
     delete c;
 }
 
+// the first level from which every level to the coarsest fits one cluster
+template <class T>
+static int find_tail(anl_ctx* c) {
+    const int nl = (int)c->lev.size();
+    ANL_TRY(vtail_prepare<T>(&c->tail_ctas));
+    for (int l = 0; l <= nl - 2 && c->tail_from < 0; ++l) {
+        if (nl - l > kTailMaxLevels) continue;
+        TailLevel<T> tl[kTailMaxLevels];
+        for (int q = l; q < nl; ++q) {
+            tl[q - l].d = c->lev[q].d;
+            tl[q - l].degree = c->degree(q);
+        }
+        if (vtail_fits<T>(tl, nl - l, c->tail_ctas)) c->tail_from = l;
+    }
+    return ANL_OK;
+}
+
 static int create(anl_ctx** out, int nx, int ny, int nz, double h, double nu, int flags) {
     if (!out || nx < 1 || ny < 1 || nz < 1 || !(h > 0) || !(nu > -1.0 && nu < 0.5)) {
         set_error("anl_ctx_create: bad arguments (grid %d x %d x %d, h %g, nu %g)", nx, ny, nz, h, nu);
@@ -435,25 +452,15 @@ static int create(anl_ctx** out, int nx, int ny, int nz, double h, double nu, in
         free_ctx(c);
         return ANL_ERR_CUDA;
     }
-    // the V-cycle tail: the first level from which every level to the coarsest fits one cluster
-    // (ANL_TAIL=0 turns it off)
+    // the V-cycle tail (ANL_TAIL=0 turns it off)
     {
         const char* e = std::getenv("ANL_TAIL");
         const bool tail_on = !(e && std::atoi(e) == 0);
         const int nl = (int)c->lev.size();
-        if (tail_on && !c->fp64 && c->dense_coarse && nl >= 2) {
-            if (vtail_prepare(&c->tail_ctas) != ANL_OK) {
+        if (tail_on && c->dense_coarse && nl >= 2) {
+            if ((c->fp64 ? find_tail<double>(c) : find_tail<float>(c)) != ANL_OK) {
                 free_ctx(c);
                 return ANL_ERR_CUDA;
-            }
-            for (int l = 0; l <= nl - 2 && c->tail_from < 0; ++l) {
-                if (nl - l > kTailMaxLevels) continue;
-                TailLevel tl[kTailMaxLevels];
-                for (int q = l; q < nl; ++q) {
-                    tl[q - l].d = c->lev[q].d;
-                    tl[q - l].degree = c->degree(q);
-                }
-                if (vtail_fits(tl, nl - l, c->tail_ctas)) c->tail_from = l;
             }
         }
     }

@@ -163,10 +163,11 @@ struct TailGeo {          // a level's slabs (anl_vtail.cu)
     int ns = 0, na = 0, nb = 0, es = 0, ea = 0, eb = 0;
     int p[3] = {0, 0, 0}; // node strides of the tail's own vectors along x, y, z
 };
-struct TailLayout {       // shared memory, in words
+struct TailLayout {       // shared memory, in values
     int xlen = 0, c = 0, words = 0;
     int f[kTailMaxLevels], flen[kTailMaxLevels], e[kTailMaxLevels];
 };
+template <class T>
 struct TailLevel {
     Dims d{};
     TailGeo g;
@@ -175,29 +176,34 @@ struct TailLevel {
     const float* diag = nullptr;
     const double* cheb = nullptr;  // (c1, c2) pairs of the level's sweep
     int degree = 0;
-    float* b = nullptr;            // the level's vectors, slots vs floats apart
-    float* r = nullptr;
-    float* x = nullptr;
-    float* xt = nullptr;
+    T* b = nullptr;                // the level's vectors, slots vs values apart
+    T* r = nullptr;
+    T* x = nullptr;
+    T* xt = nullptr;
     int64_t vs = 0;
 };
+template <class T>
 struct TailArgs {
     int nlev = 0, ctas = 0;
-    TailLevel lev[kTailMaxLevels];
+    TailLevel<T> lev[kTailMaxLevels];
     TailLayout lay;                // set by the launcher, as the levels' g
-    float* b0 = nullptr;
-    const float* ainv_hi = nullptr;
+    T* b0 = nullptr;
+    const float* ainv_hi = nullptr;  // the coarsest grid's inverse: FP32 contexts as float pairs
     const float* ainv_lo = nullptr;
+    const double* ainv = nullptr;    // FP64 contexts
     int nc = 0;
     const int* done = nullptr;
-    KeModal<float> km{};
+    KeModal<T> km{};
     // right-hand-side slots: cluster r works on slot r
     int nrhs = 1;
     int sc_bytes = 0;  // bytes between the slots' done flags
 };
+template <class T>
 int vtail_prepare(int* ctas);
-bool vtail_fits(TailLevel* lev, int nlev, int ctas);  // fills the levels' g
-int launch_vtail(const TailArgs& a, cudaStream_t s);
+template <class T>
+bool vtail_fits(TailLevel<T>* lev, int nlev, int ctas);  // fills the levels' g
+template <class T>
+int launch_vtail(const TailArgs<T>& a, cudaStream_t s);
 
 // ------------------------------------------------------------------ tensor-core K u (fine grid)
 

@@ -1167,8 +1167,9 @@ static int vcycle_box(anl_ctx* c, size_t l, int deg, const int* done, cudaStream
 
 // The levels from tail_from down in one cluster per right-hand-side slot: b of level l in, its
 // correction x out.
+template <class T>
 static int vcycle_tail(anl_ctx* c, size_t l, const int* done, cudaStream_t s) {
-    TailArgs a;
+    TailArgs<T> a;
     a.nlev = (int)(c->lev.size() - l);
     a.ctas = c->tail_ctas;
     for (int q = 0; q < a.nlev; ++q) {
@@ -1179,27 +1180,28 @@ static int vcycle_tail(anl_ctx* c, size_t l, const int* done, cudaStream_t s) {
         a.lev[q].diag = Lq.diag;
         a.lev[q].cheb = c->cheb_d + (l + q) * kChebStride + 1;
         a.lev[q].degree = c->degree(l + q);
-        a.lev[q].b = (float*)Lq.b;
-        a.lev[q].r = (float*)Lq.r;
-        a.lev[q].x = (float*)Lq.x;
-        a.lev[q].xt = (float*)Lq.xt;
+        a.lev[q].b = (T*)Lq.b;
+        a.lev[q].r = (T*)Lq.r;
+        a.lev[q].x = (T*)Lq.x;
+        a.lev[q].xt = (T*)Lq.xt;
         a.lev[q].vs = Lq.vs;
     }
-    a.b0 = (float*)c->lev[l].b;
+    a.b0 = (T*)c->lev[l].b;
     a.ainv_hi = c->ainv_hi;
     a.ainv_lo = c->ainv_lo;
     a.nc = c->nc;
     a.done = done;
-    a.km = c->kmf;
+    a.ainv = c->Ainv;
+    a.km = modal_of<T>(c);
     a.nrhs = c->rb;
     a.sc_bytes = (int)sizeof(PcgScalars);
-    return launch_vtail(a, s);
+    return launch_vtail<T>(a, s);
 }
 
 template <class T>
 static int vcycle(anl_ctx* c, size_t l, const int* done, cudaStream_t s) {
     Level& L = c->lev[l];
-    if (sizeof(T) == 4 && c->tail_from >= 0 && (int)l == c->tail_from) return vcycle_tail(c, l, done, s);
+    if (c->tail_from >= 0 && (int)l == c->tail_from) return vcycle_tail<T>(c, l, done, s);
     if (l + 1 == c->lev.size()) {
         if (c->dense_coarse) {
             const int n = c->nc;

@@ -37,18 +37,29 @@ namespace anl {
 
 namespace {
 
-constexpr int TT = 512;         // threads of a CTA
-constexpr int NPT = 2;          // owned nodes of a thread
+// TT: threads of a CTA, NPT: owned nodes of a thread. Levels of at most ALONE elements stay in one
+// CTA; levels with more than MOST elements in a CTA are left to launches of their own.
+template <class T>
+struct TailCfg;
+template <>
+struct TailCfg<float> {
+    // one CTA's step takes 0.9 us at 128 elements, shorter than a shared one, whose halo flight
+    // alone takes 0.7 us; at 432 it is not (2 us)
+    static constexpr int TT = 512, NPT = 2, ALONE = 256, MOST = 1 << 30;
+};
+template <>
+struct TailCfg<double> {
+    // A warp of elements holds the FP64 pipe for 1.6 us (176 instructions, 19 cycles each), so one
+    // CTA takes no more than one warp of them, and above five warps in each of 16 CTAs the 152 SMs
+    // of a launch are faster again.
+    static constexpr int TT = 256, NPT = 2, ALONE = 32, MOST = 160;
+};
 constexpr int FW = 25;          // words between two elements' forces (24 and one of padding)
 constexpr int kWaitTries = 1 << 20;  // bound of a halo wait
 constexpr int kTailMaxDegree = 16;  // Chebyshev steps per sweep there is room for
 
 // A level's slabs: A x B elements per layer, L layers along the tail's axis, `per` layers to a CTA.
-// Levels of at most kAloneElems elements stay in one CTA: its step (0.9 us at 128 elements)
-// is shorter than a shared one, whose halo flight alone takes 0.7 us; at 432 it is not (2 us).
-constexpr int kAloneElems = 256;
-
-TailGeo slab_geo(int axis, const Dims& d, int ctas) {
+TailGeo slab_geo(int axis, const Dims& d, int ctas, int alone) {
     const int n[3] = {d.nx, d.ny, d.nz};
     const int ax = axis == 0 ? 1 : 0, bx = axis == 2 ? 1 : 2;
     const int nstr[3] = {1, d.nx + 1, (d.nx + 1) * (d.ny + 1)}, estr[3] = {1, d.nx, d.nx * d.ny};
@@ -58,7 +69,7 @@ TailGeo slab_geo(int axis, const Dims& d, int ctas) {
     g.L = n[axis];
     g.ns = nstr[axis], g.na = nstr[ax], g.nb = nstr[bx];
     g.es = estr[axis], g.ea = estr[ax], g.eb = estr[bx];
-    const int use = d.ne() <= kAloneElems ? 1 : ctas;
+    const int use = d.ne() <= alone ? 1 : ctas;
     g.per = (g.L + use - 1) / use;
     g.active = (g.L + g.per - 1) / g.per;
     g.PA = g.A + 1;
@@ -74,16 +85,17 @@ int max_nodes(const TailGeo& g) { return (g.per + 1) * g.planeN; }
 int max_elems(const TailGeo& g) { return (g.per + (g.active > 1 ? 1 : 0)) * g.A * g.B; }
 int max_padded(const TailGeo& g) { return (g.per + 2) * g.planeN + g.A + 2; }
 
-// shared-memory carve-up in words: the iterate twice (own planes and two halo planes), the coarsest
+// shared-memory carve-up in values of the context's precision: the iterate twice (own planes and two halo planes), the coarsest
 // right-hand side, then per level the forces and the elements' (scale, packed indices) pairs
-TailLayout tail_layout(const TailLevel* lev, int nlev) {
+template <class T>
+TailLayout tail_layout(const TailLevel<T>* lev, int nlev) {
     TailLayout t{};
     for (int l = 0; l < nlev - 1; ++l) t.xlen = std::max(t.xlen, 3 * (max_nodes(lev[l].g) + 2 * lev[l].g.planeN));
     t.xlen = (t.xlen + 3) / 4 * 4;
     int o = 2 * t.xlen;
     for (int l = 0; l < nlev - 1; ++l) {
         t.e[l] = o;
-        o += (2 * max_elems(lev[l].g) + 3) / 4 * 4;
+        o += ((int)(sizeof(float2) / sizeof(T)) * max_elems(lev[l].g) + 3) / 4 * 4;
         t.f[l] = o;
         t.flen[l] = (FW * max_padded(lev[l].g) + 3) / 4 * 4;
         o += t.flen[l];
@@ -101,10 +113,14 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t addr, int rank) {
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
-// one word to another CTA of the cluster, counted on that CTA's barrier
+// one value to another CTA of the cluster, counted on that CTA's barrier
 __device__ __forceinline__ void st_async(uint32_t addr, float v, uint32_t bar) {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr),
                  "r"(__float_as_uint(v)), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void st_async(uint32_t addr, double v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+                 "l"(__double_as_longlong(v)), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void bar_expect(uint32_t bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -125,19 +141,18 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, unsigned parity) {
 // components c0 .. c0 + NC - 1 of (R r)(I, J, K): trilinear weights 1, 1/2, 1/4, 1/8 of the fine
 // residual r (slab-major, strides p); nodes outside the grid are read at its edge with weight 0, so
 // no load depends on a test and a plane's loads are in flight together
-template <int NC>
-__device__ __forceinline__ void restrict_at(const TailLevel& f, const float* r, int I, int J, int K, int c0,
-                                            float (&acc)[NC]) {
+template <int NC, class T>
+__device__ __forceinline__ void restrict_at(const TailLevel<T>& f, const T* r, int I, int J, int K, int c0, T (&acc)[NC]) {
     const Dims& d = f.d;
     const int px = 3 * f.g.p[0], py = 3 * f.g.p[1], pz = 3 * f.g.p[2];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) acc[c] = 0.f;
+    for (int c = 0; c < NC; ++c) acc[c] = T(0);
 #pragma unroll 1
     for (int dk = -1; dk <= 1; ++dk) {
         const int k = 2 * K + dk;
-        const float* p = r + pz * min(max(k, 0), d.nz) + c0;
-        const float wk = k < 0 || k > d.nz ? 0.f : dk ? 0.5f : 1.f;
-        float v[9][NC];
+        const T* p = r + pz * min(max(k, 0), d.nz) + c0;
+        const T wk = k < 0 || k > d.nz ? T(0) : dk ? T(0.5) : T(1);
+        T v[9][NC];
 #pragma unroll
         for (int q = 0; q < 9; ++q) {
             const int i = min(max(2 * I + q % 3 - 1, 0), d.nx), j = min(max(2 * J + q / 3 - 1, 0), d.ny);
@@ -148,28 +163,29 @@ __device__ __forceinline__ void restrict_at(const TailLevel& f, const float* r, 
         for (int q = 0; q < 9; ++q) {
             const int di = q % 3 - 1, dj = q / 3 - 1, i = 2 * I + di, j = 2 * J + dj;
             const bool in = i >= 0 && j >= 0 && i <= d.nx && j <= d.ny;
-            const float w = in ? (di ? 0.5f : 1.f) * (dj ? 0.5f : 1.f) * wk : 0.f;
+            const T w = in ? (di ? T(0.5) : T(1)) * (dj ? T(0.5) : T(1)) * wk : T(0);
 #pragma unroll
-            for (int c = 0; c < NC; ++c) acc[c] = fmaf(w, v[q][c], acc[c]);
+            for (int c = 0; c < NC; ++c) acc[c] = fma(w, v[q][c], acc[c]);
         }
     }
 }
 
 // (P xc)(i, j, k): the mean of the coarse nodes the fine node lies between (the unused ones of the
 // 8 are read at the node itself); xc has node strides p
-__device__ __forceinline__ void prolong_at(const int (&p)[3], const float* xc, int i, int j, int k, float (&acc)[3]) {
+template <class T>
+__device__ __forceinline__ void prolong_at(const int (&p)[3], const T* xc, int i, int j, int k, T (&acc)[3]) {
     const int di = i & 1, dj = j & 1, dk = k & 1;
     const int n0 = (i >> 1) * p[0] + (j >> 1) * p[1] + (k >> 1) * p[2];
-    float v[8][3];
+    T v[8][3];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const int n = n0 + (q & di) * p[0] + ((q >> 1) & dj) * p[1] + ((q >> 2) & dk) * p[2];
 #pragma unroll
         for (int c = 0; c < 3; ++c) v[q][c] = xc[3 * n + c];
     }
-    const float w = (di ? 0.5f : 1.f) * (dj ? 0.5f : 1.f) * (dk ? 0.5f : 1.f);
+    const T w = (di ? T(0.5) : T(1)) * (dj ? T(0.5) : T(1)) * (dk ? T(0.5) : T(1));
 #pragma unroll
-    for (int c = 0; c < 3; ++c) acc[c] = 0.f;
+    for (int c = 0; c < 3; ++c) acc[c] = T(0);
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         if (((q & 1) && !di) || ((q & 2) && !dj) || ((q & 4) && !dk)) continue;
@@ -181,31 +197,33 @@ __device__ __forceinline__ void prolong_at(const int (&p)[3], const float* xc, i
 }
 
 // an owned node of this thread on the current level
+template <class T>
 struct TailNode {
     int pn;         // node index in slab-major order, -1 for none
     int gn;         // node index on the level's grid
-    int nl;         // first word of the node in an iterate buffer
-    int nb;         // first word of the padded element above it in every direction
+    int nl;         // first value of the node in an iterate buffer
+    int nb;         // first value of the padded element above it in every direction
     int i, j, k;
     unsigned m;     // mask
-    float g;        // inverse diagonal
-    float b[3], d[3], x[3];
-    int down, up;   // words of its copies in the neighbours' halo planes, -1 for none
+    T g;            // inverse diagonal
+    T b[3], d[3], x[3];
+    int down, up;   // its copies in the neighbours' halo planes, -1 for none
 };
 
-template <int AXIS>
+template <class T, int AXIS>
 struct Tail {
-    const TailArgs& a;
-    float* sm;
+    static constexpr int TT = TailCfg<T>::TT, NPT = TailCfg<T>::NPT;
+    const TailArgs<T>& a;
+    T* sm;
     uint32_t bar;                 // this CTA's barriers: [direction][buffer], 8 bytes each
     uint32_t x_down, x_up, b_down, b_up;  // the neighbours' iterate buffers and barriers
     int tid, rank, ctas, slot;
     int cur = 0;                  // the buffer that holds the iterate
     unsigned phase = 0;           // next phase parity of barrier [direction][buffer], one bit each
     bool lost = false;            // a halo wait ran out
-    TailNode nd[NPT];
+    TailNode<T> nd[NPT];
 
-    __device__ float* vec(float* p, int l) const { return p + (int64_t)slot * a.lev[l].vs; }
+    __device__ T* vec(T* p, int l) const { return p + (int64_t)slot * a.lev[l].vs; }
 
     __device__ int own(const TailGeo& g) const { return rank < g.active ? min(g.per, g.L - rank * g.per) : 0; }
     // element layers the CTA computes: its own and, but for the first CTA, the one below
@@ -217,10 +235,10 @@ struct Tail {
 
     // the element table of level l and its zeroed forces (once per launch)
     __device__ void table(int l) {
-        const TailLevel& lv = a.lev[l];
+        const TailLevel<T>& lv = a.lev[l];
         const TailGeo& g = lv.g;
         float4* f = reinterpret_cast<float4*>(sm + a.lay.f[l]);
-        for (int t = tid; t < a.lay.flen[l] / 4; t += TT) f[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int t = tid; t < a.lay.flen[l] / (16 / (int)sizeof(T)); t += TT) f[t] = make_float4(0.f, 0.f, 0.f, 0.f);
         const int layer = g.A * g.B, ne = elems(g), first = first_layer(g), q0 = g.active > 1 ? 0 : 1;
         float2* et = reinterpret_cast<float2*>(sm + a.lay.e[l]);
         for (int e = tid; e < ne; e += TT) {
@@ -235,18 +253,18 @@ struct Tail {
 
     // this thread's nodes of level l
     __device__ void enter(int l) {
-        const TailLevel& lv = a.lev[l];
+        const TailLevel<T>& lv = a.lev[l];
         const TailGeo& g = lv.g;
         const int o = own(g), nown = o > 0 ? o + (rank == g.active - 1 ? 1 : 0) : 0;
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
-            TailNode& n = nd[r];
+            TailNode<T>& n = nd[r];
             const int t = tid + r * TT;
             n.pn = -1;
             n.m = 0;
-            n.g = 0.f;
+            n.g = T(0);
 #pragma unroll
-            for (int c = 0; c < 3; ++c) n.b[c] = n.d[c] = n.x[c] = 0.f;
+            for (int c = 0; c < 3; ++c) n.b[c] = n.d[c] = n.x[c] = T(0);
             if (t >= nown * g.planeN) continue;
             const int p = 1 + t / g.planeN, in = t - (p - 1) * g.planeN, b = in / g.PA, aa = in - b * g.PA;
             const int s = rank * g.per + p - 1;
@@ -259,7 +277,7 @@ struct Tail {
             n.j = AXIS == 1 ? s : AXIS == 0 ? aa : b;
             n.k = AXIS == 2 ? s : b;
             n.m = __ldg(lv.nmask + n.gn) & 7u;
-            n.g = __ldg(lv.diag + n.gn);
+            n.g = T(__ldg(lv.diag + n.gn));
             n.down = p == 1 && rank > 0 ? 3 * ((g.per + 1) * g.planeN + in) : -1;
             n.up = p == nown && rank + 1 < g.active ? 3 * in : -1;
         }
@@ -274,18 +292,18 @@ struct Tail {
         if (tid == 0) {
 #pragma unroll
             for (int q = 0; q < 2; ++q)
-                if (from[q]) bar_expect(bar + 8u * (2 * q + cur), 12u * (unsigned)g.planeN);
+                if (from[q]) bar_expect(bar + 8u * (2 * q + cur), 3u * (unsigned)sizeof(T) * (unsigned)g.planeN);
         }
         const int o = cur * a.lay.xlen;
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
-            const TailNode& n = nd[r];
+            const TailNode<T>& n = nd[r];
             if (n.pn < 0) continue;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 // this CTA lies above rank - 1 and below rank + 1
-                if (n.down >= 0) st_async(x_down + 4u * (unsigned)(o + n.down + c), n.x[c], b_down + 8u * (2 + cur));
-                if (n.up >= 0) st_async(x_up + 4u * (unsigned)(o + n.up + c), n.x[c], b_up + 8u * cur);
+                if (n.down >= 0) st_async(x_down + (unsigned)sizeof(T) * (unsigned)(o + n.down + c), n.x[c], b_down + 8u * (2 + cur));
+                if (n.up >= 0) st_async(x_up + (unsigned)sizeof(T) * (unsigned)(o + n.up + c), n.x[c], b_up + 8u * cur);
             }
 #pragma unroll
             for (int c = 0; c < 3; ++c) sm[o + n.nl + c] = n.x[c];
@@ -304,27 +322,28 @@ struct Tail {
     __device__ void elements(int l) const {
         const TailGeo& g = a.lev[l].g;
         const int ne = elems(g);
-        const float* x = sm + cur * a.lay.xlen;
+        const T* x = sm + cur * a.lay.xlen;
         const float2* et = reinterpret_cast<const float2*>(sm + a.lay.e[l]);
-        float* F = sm + a.lay.f[l];
+        T* F = sm + a.lay.f[l];
         const int sx = 3 * g.p[0], sy = 3 * g.p[1], sz = 3 * g.p[2];
         for (int e = tid; e < ne; e += TT) {
             const float2 te = et[e];
             if (te.x == 0.f) continue;  // its forces stay the zeros of table()
             const int tab = __float_as_int(te.y);
-            const float* p0 = x + 3 * (tab & 0xffff);
-            V3<float> u[2][2][2];
+            const T* p0 = x + 3 * (tab & 0xffff);
+            V3<T> u[2][2][2];
 #pragma unroll
             for (int pz = 0; pz < 2; ++pz)
 #pragma unroll
                 for (int py = 0; py < 2; ++py)
 #pragma unroll
                     for (int px = 0; px < 2; ++px) {
-                        const float* p = p0 + px * sx + py * sy + pz * sz;
-                        u[px][py][pz].xy = make_float2(p[0], p[1]);
+                        const T* p = p0 + px * sx + py * sy + pz * sz;
+                        u[px][py][pz].xy.x = p[0];
+                        u[px][py][pz].xy.y = p[1];
                         u[px][py][pz].z = p[2];
                     }
-            V3<float> dxb[2], dxt[2], dyb[2], dyt[2], dz[2][2], f[2][2][2];
+            V3<T> dxb[2], dxt[2], dyb[2], dyt[2], dz[2][2], f[2][2][2];
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 dxb[q] = u[1][q][0] - u[0][q][0];
@@ -336,8 +355,8 @@ struct Tail {
             for (int px = 0; px < 2; ++px)
 #pragma unroll
                 for (int py = 0; py < 2; ++py) dz[px][py] = u[px][py][1] - u[px][py][0];
-            modal_element<float>(a.km, te.x, dxb, dxt, dyb, dyt, dz, f);
-            float* fo = F + FW * (tab >> 16);
+            modal_element<T>(a.km, T(te.x), dxb, dxt, dyb, dyt, dz, f);
+            T* fo = F + FW * (tab >> 16);
 #pragma unroll
             for (int pz = 0; pz < 2; ++pz)
 #pragma unroll
@@ -356,31 +375,31 @@ struct Tail {
     }
 
     // (K x)(n): the 8 corners that meet at the node, in a fixed order
-    __device__ void force(int l, const TailNode& n, float (&y)[3]) const {
+    __device__ void force(int l, const TailNode<T>& n, T (&y)[3]) const {
         const TailGeo& g = a.lev[l].g;
-        const float* F = sm + a.lay.f[l] + n.nb;
-        y[0] = y[1] = y[2] = 0.f;
+        const T* F = sm + a.lay.f[l] + n.nb;
+        y[0] = y[1] = y[2] = T(0);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const float* p = F - FW * ((q & 1) + ((q >> 1) & 1) * g.PA + (q >> 2) * g.planeN) + 3 * q;
+            const T* p = F - FW * ((q & 1) + ((q >> 1) & 1) * g.PA + (q >> 2) * g.planeN) + 3 * q;
 #pragma unroll
             for (int c = 0; c < 3; ++c) y[c] += p[c];
         }
     }
 
     // one Chebyshev step
-    __device__ void step(int l, float c1, float c2) {
+    __device__ void step(int l, T c1, T c2) {
         elements(l);
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
-            TailNode& n = nd[r];
+            TailNode<T>& n = nd[r];
             if (n.m == 0) continue;
-            float y[3];
+            T y[3];
             force(l, n, y);
-            const float gn = c2 * n.g;
+            const T gn = c2 * n.g;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const float dn = (n.m >> c) & 1 ? c1 * n.d[c] + (n.b[c] - y[c]) * gn : 0.f;
+                const T dn = (n.m >> c) & 1 ? c1 * n.d[c] + (n.b[c] - y[c]) * gn : T(0);
                 n.d[c] = dn;
                 n.x[c] += dn;
             }
@@ -389,10 +408,12 @@ struct Tail {
     }
 };
 
-template <int AXIS>
-__global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArgs a) {
-    extern __shared__ __align__(16) float tail_smem[];
-    __shared__ float cf[kTailMaxLevels][2 * kTailMaxDegree];
+template <class T, int AXIS>
+__global__ void __launch_bounds__(TailCfg<T>::TT, 1) k_vtail(const __grid_constant__ TailArgs<T> a) {
+    constexpr int TT = TailCfg<T>::TT, NPT = TailCfg<T>::NPT;
+    extern __shared__ __align__(16) unsigned char tail_bytes[];
+    T* tail_smem = reinterpret_cast<T*>(tail_bytes);
+    __shared__ T cf[kTailMaxLevels][2 * kTailMaxDegree];
     __shared__ __align__(8) uint64_t bars[2][2];
     const int tid = threadIdx.x, ctas = a.ctas;
     const int rank = blockIdx.x % ctas, slot = blockIdx.x / ctas;
@@ -407,10 +428,10 @@ __global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArg
     }
     for (int q = tid; q < last * 2 * kTailMaxDegree; q += TT) {
         const int l = q / (2 * kTailMaxDegree), k = q - l * 2 * kTailMaxDegree;
-        if (k < 2 * a.lev[l].degree) cf[l][k] = (float)a.lev[l].cheb[k];
+        if (k < 2 * a.lev[l].degree) cf[l][k] = T(a.lev[l].cheb[k]);
     }
     __syncthreads();
-    Tail<AXIS> t{a, tail_smem, bar, 0, 0, 0, 0, tid, rank, ctas, slot};
+    Tail<T, AXIS> t{a, tail_smem, bar, 0, 0, 0, 0, tid, rank, ctas, slot};
     {
         const uint32_t xb = (uint32_t)__cvta_generic_to_shared(tail_smem);
         const int below = rank > 0 ? rank - 1 : 0, above = rank + 1 < ctas ? rank + 1 : rank;
@@ -427,19 +448,19 @@ __global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArg
         t.enter(l);
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
-            TailNode& n = t.nd[r];
+            TailNode<T>& n = t.nd[r];
             if (n.pn < 0) continue;
             if (l == 0) {
 #pragma unroll
                 for (int c = 0; c < 3; ++c) n.b[c] = __ldg(t.vec(a.b0, 0) + 3 * n.gn + c);
             } else {
-                restrict_at<3>(a.lev[l - 1], t.vec(a.lev[l - 1].r, l - 1), n.i, n.j, n.k, 0, n.b);
+                restrict_at<3, T>(a.lev[l - 1], t.vec(a.lev[l - 1].r, l - 1), n.i, n.j, n.k, 0, n.b);
             }
-            const float gn = cf[l][1] * n.g;  // step 0: x = d = c2_0 D^-1 b
-            float* save = t.vec(a.lev[l].b, l) + 3 * n.pn;
+            const T gn = cf[l][1] * n.g;  // step 0: x = d = c2_0 D^-1 b
+            T* save = t.vec(a.lev[l].b, l) + 3 * n.pn;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                if (!((n.m >> c) & 1)) n.b[c] = 0.f;
+                if (!((n.m >> c) & 1)) n.b[c] = T(0);
                 n.x[c] = n.d[c] = gn * n.b[c];
                 if (l > 0) save[c] = n.b[c];
             }
@@ -447,17 +468,17 @@ __global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArg
         t.exchange(l);
         for (int k = 1; k < deg; ++k) t.step(l, cf[l][2 * k], cf[l][2 * k + 1]);
         t.elements(l);
-        float* res = t.vec(a.lev[l].r, l);
-        float* save = t.vec(a.lev[l].xt, l);
+        T* res = t.vec(a.lev[l].r, l);
+        T* save = t.vec(a.lev[l].xt, l);
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
-            const TailNode& n = t.nd[r];
+            const TailNode<T>& n = t.nd[r];
             if (n.pn < 0) continue;
-            float y[3] = {0.f, 0.f, 0.f};
+            T y[3] = {T(0), T(0), T(0)};
             if (n.m) t.force(l, n, y);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                res[3 * n.pn + c] = (n.m >> c) & 1 ? n.b[c] - y[c] : 0.f;
+                res[3 * n.pn + c] = (n.m >> c) & 1 ? n.b[c] - y[c] : T(0);
                 save[3 * n.pn + c] = n.x[c];
             }
         }
@@ -466,40 +487,52 @@ __global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArg
 
     {  // the coarsest grid: its right-hand side in every CTA, the rows of the inverse shared out
         const Dims d = a.lev[last].d;
-        float* bc = tail_smem + a.lay.c;
-        const float* rf = t.vec(a.lev[last - 1].r, last - 1);
+        T* bc = tail_smem + a.lay.c;
+        const T* rf = t.vec(a.lev[last - 1].r, last - 1);
         for (int q = tid; q < 3 * (int)d.nn(); q += TT) {
             const int N = q / 3, c = q - 3 * N;
             const int K = N / ((d.nx + 1) * (d.ny + 1)), J = N / (d.nx + 1) % (d.ny + 1), I = N % (d.nx + 1);
             const unsigned m = __ldg(a.lev[last].nmask + N);
-            float v[1];
-            restrict_at<1>(a.lev[last - 1], rf, I, J, K, c, v);
-            bc[q] = (m >> c) & 1 ? v[0] : 0.f;
+            T v[1];
+            restrict_at<1, T>(a.lev[last - 1], rf, I, J, K, c, v);
+            bc[q] = (m >> c) & 1 ? v[0] : T(0);
         }
         __syncthreads();
         const int n = a.nc, lane = tid & 31;
-        float* xc = t.vec(a.lev[last].x, last);
+        T* xc = t.vec(a.lev[last].x, last);
         for (int row = rank * (TT / 32) + (tid >> 5); row < n; row += ctas * (TT / 32)) {
-            // one warp per row, compensated FP32 sums, the lanes' pairs added in a fixed tree
-            const float* hi = a.ainv_hi + (int64_t)row * n;
-            const float* lo = a.ainv_lo + (int64_t)row * n;
-            Acc2 acc;
+            // one warp per row; FP32: compensated sums of the inverse's float pairs, the lanes' pairs
+            // added in a fixed tree
+            T sum;
+            if constexpr (std::is_same<T, double>::value) {
+                const double* inv = a.ainv + (int64_t)row * n;
+                sum = 0.0;
 #pragma unroll 4
-            for (int c = lane; c < n; c += 32) {
-                const float h = __ldg(hi + c), q = __ldg(lo + c), b = bc[c];
-                acc.add_prod(h, b);
-                acc.add_prod(q, b);
-            }
-            float s = acc.s, e = acc.c;
+                for (int c = lane; c < n; c += 32) sum = fma(__ldg(inv + c), bc[c], sum);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float s2 = __shfl_down_sync(0xffffffffu, s, o), e2 = __shfl_down_sync(0xffffffffu, e, o);
-                float v, f;
-                two_sum(s, s2, v, f);
-                s = v;
-                e += e2 + f;
+                for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+            } else {
+                const float* hi = a.ainv_hi + (int64_t)row * n;
+                const float* lo = a.ainv_lo + (int64_t)row * n;
+                Acc2 acc;
+#pragma unroll 4
+                for (int c = lane; c < n; c += 32) {
+                    const float h = __ldg(hi + c), q = __ldg(lo + c), b = bc[c];
+                    acc.add_prod(h, b);
+                    acc.add_prod(q, b);
+                }
+                float s = acc.s, e = acc.c;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    const float s2 = __shfl_down_sync(0xffffffffu, s, o), e2 = __shfl_down_sync(0xffffffffu, e, o);
+                    float v, f;
+                    two_sum(s, s2, v, f);
+                    s = v;
+                    e += e2 + f;
+                }
+                sum = s + e;
             }
-            if (lane == 0) xc[row] = (__ldg(a.lev[last].nmask + row / 3) >> (row % 3)) & 1 ? s + e : 0.f;
+            if (lane == 0) xc[row] = (__ldg(a.lev[last].nmask + row / 3) >> (row % 3)) & 1 ? sum : T(0);
         }
         cluster_sync();
     }
@@ -507,32 +540,32 @@ __global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArg
     for (int l = last - 1; l >= 0; --l) {  // up: add the correction, smooth
         const int deg = a.lev[l].degree;
         t.enter(l);
-        const float* xc = t.vec(a.lev[l + 1].x, l + 1);
+        const T* xc = t.vec(a.lev[l + 1].x, l + 1);
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
-            TailNode& n = t.nd[r];
+            TailNode<T>& n = t.nd[r];
             if (n.pn < 0) continue;
             // the values this thread left on the way down
-            const float* b = l == 0 ? t.vec(a.b0, 0) + 3 * n.gn : t.vec(a.lev[l].b, l) + 3 * n.pn;
-            const float* x = t.vec(a.lev[l].xt, l) + 3 * n.pn;
-            float p[3];
+            const T* b = l == 0 ? t.vec(a.b0, 0) + 3 * n.gn : t.vec(a.lev[l].b, l) + 3 * n.pn;
+            const T* x = t.vec(a.lev[l].xt, l) + 3 * n.pn;
+            T p[3];
             prolong_at(a.lev[l + 1].g.p, xc, n.i, n.j, n.k, p);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                n.b[c] = (n.m >> c) & 1 ? b[c] : 0.f;
-                n.x[c] = x[c] + ((n.m >> c) & 1 ? p[c] : 0.f);
+                n.b[c] = (n.m >> c) & 1 ? b[c] : T(0);
+                n.x[c] = x[c] + ((n.m >> c) & 1 ? p[c] : T(0));
             }
         }
         t.exchange(l);
-        for (int k = 0; k < deg; ++k) t.step(l, k == 0 ? 0.f : cf[l][2 * k], cf[l][2 * k + 1]);
-        float* xo = t.vec(a.lev[l].x, l);
+        for (int k = 0; k < deg; ++k) t.step(l, k == 0 ? T(0) : cf[l][2 * k], cf[l][2 * k + 1]);
+        T* xo = t.vec(a.lev[l].x, l);
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
-            const TailNode& n = t.nd[r];
+            const TailNode<T>& n = t.nd[r];
             if (n.pn < 0) continue;
 #pragma unroll
             for (int c = 0; c < 3; ++c)  // a lost halo fails the solve
-                xo[3 * (l == 0 ? n.gn : n.pn) + c] = t.lost ? NAN : n.x[c];
+                xo[3 * (l == 0 ? n.gn : n.pn) + c] = t.lost ? T(NAN) : n.x[c];
         }
         cluster_sync();  // the correction is written; at the end no CTA leaves before its neighbours' stores
     }
@@ -541,7 +574,8 @@ __global__ void __launch_bounds__(TT, 1) k_vtail(const __grid_constant__ TailArg
 int tail_axis(const Dims& d) { return d.nx >= d.ny && d.nx >= d.nz ? 0 : d.ny >= d.nz ? 1 : 2; }
 
 // fills the levels' geometry and the layout; false where they exceed a cluster
-bool tail_plan(TailLevel* lev, int nlev, int ctas, int axis, TailLayout* lay) {
+template <class T>
+bool tail_plan(TailLevel<T>* lev, int nlev, int ctas, int axis, TailLayout* lay) {
     for (int l = 0; l < nlev; ++l) {
         TailGeo& g = lev[l].g;
         if (lev[l].d.nn() > 0xffff) return false;
@@ -551,21 +585,22 @@ bool tail_plan(TailLevel* lev, int nlev, int ctas, int axis, TailLayout* lay) {
             g.p[2] = g.p[1] * (lev[l].d.ny + 1);
             continue;
         }
-        g = slab_geo(axis, lev[l].d, ctas);
+        g = slab_geo(axis, lev[l].d, ctas, TailCfg<T>::ALONE);
         if (lev[l].degree < 1 || lev[l].degree > kTailMaxDegree) return false;
-        if (max_nodes(g) > TT * NPT || max_padded(g) > 0x7fff || max_nodes(g) + 2 * g.planeN > 0xffff) return false;
+        if (max_elems(g) > TailCfg<T>::MOST) return false;
+        if (max_nodes(g) > TailCfg<T>::TT * TailCfg<T>::NPT || max_padded(g) > 0x7fff || max_nodes(g) + 2 * g.planeN > 0xffff) return false;
     }
-    *lay = tail_layout(lev, nlev);
-    return sizeof(float) * (size_t)lay->words <= (size_t)kTailMaxSmem;
+    *lay = tail_layout<T>(lev, nlev);
+    return sizeof(T) * (size_t)lay->words <= (size_t)kTailMaxSmem;
 }
 
-cudaLaunchConfig_t tail_config(int ctas, int nrhs, size_t bytes, cudaStream_t s, cudaLaunchAttribute* attr) {
+cudaLaunchConfig_t tail_config(int ctas, int threads, int nrhs, size_t bytes, cudaStream_t s, cudaLaunchAttribute* attr) {
     attr->id = cudaLaunchAttributeClusterDimension;
     attr->val.clusterDim.x = (unsigned)ctas;
     attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(ctas * nrhs));
-    cfg.blockDim = dim3(TT);
+    cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = bytes;
     cfg.stream = s;
     cfg.attrs = attr;
@@ -573,10 +608,10 @@ cudaLaunchConfig_t tail_config(int ctas, int nrhs, size_t bytes, cudaStream_t s,
     return cfg;
 }
 
-template <int AXIS>
+template <class T, int AXIS>
 int tail_prepare_axis() {
-    ANL_CUDA(cudaFuncSetAttribute(k_vtail<AXIS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailMaxSmem));
-    ANL_CUDA(cudaFuncSetAttribute(k_vtail<AXIS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    ANL_CUDA(cudaFuncSetAttribute(k_vtail<T, AXIS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailMaxSmem));
+    ANL_CUDA(cudaFuncSetAttribute(k_vtail<T, AXIS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     return ANL_OK;
 }
 
@@ -584,16 +619,17 @@ int tail_prepare_axis() {
 
 // CTAs of the tail's cluster: 16 where the device can place such a cluster with the largest
 // shared memory, else 8 (the portable size).
+template <class T>
 int vtail_prepare(int* ctas) {
     static int n = 0;
     if (n == 0) {
-        ANL_TRY(tail_prepare_axis<0>());
-        ANL_TRY(tail_prepare_axis<1>());
-        ANL_TRY(tail_prepare_axis<2>());
+        ANL_TRY((tail_prepare_axis<T, 0>()));
+        ANL_TRY((tail_prepare_axis<T, 1>()));
+        ANL_TRY((tail_prepare_axis<T, 2>()));
         cudaLaunchAttribute attr;
-        cudaLaunchConfig_t cfg = tail_config(16, 1, kTailMaxSmem, nullptr, &attr);
+        cudaLaunchConfig_t cfg = tail_config(16, TailCfg<T>::TT, 1, kTailMaxSmem, nullptr, &attr);
         int fit = 0;
-        if (cudaOccupancyMaxActiveClusters(&fit, k_vtail<0>, &cfg) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveClusters(&fit, k_vtail<T, 0>, &cfg) != cudaSuccess) {
             cudaGetLastError();
             fit = 0;
         }
@@ -603,29 +639,38 @@ int vtail_prepare(int* ctas) {
     return ANL_OK;
 }
 
-bool vtail_fits(TailLevel* lev, int nlev, int ctas) {
+template <class T>
+bool vtail_fits(TailLevel<T>* lev, int nlev, int ctas) {
     TailLayout lay;
-    return tail_plan(lev, nlev, ctas, tail_axis(lev[0].d), &lay);
+    return tail_plan<T>(lev, nlev, ctas, tail_axis(lev[0].d), &lay);
 }
 
-int launch_vtail(const TailArgs& args, cudaStream_t s) {
-    TailArgs a = args;
+template <class T>
+int launch_vtail(const TailArgs<T>& args, cudaStream_t s) {
+    TailArgs<T> a = args;
     const int axis = tail_axis(a.lev[0].d);
-    if (a.nlev < 2 || a.nlev > kTailMaxLevels || !tail_plan(a.lev, a.nlev, a.ctas, axis, &a.lay)) {
+    if (a.nlev < 2 || a.nlev > kTailMaxLevels || !tail_plan<T>(a.lev, a.nlev, a.ctas, axis, &a.lay)) {
         set_error("V-cycle tail: the levels exceed one cluster of %d CTAs", a.ctas);
         return ANL_ERR_BADARG;
     }
-    const size_t bytes = sizeof(float) * (size_t)a.lay.words;
+    const size_t bytes = sizeof(T) * (size_t)a.lay.words;
     cudaLaunchAttribute attr;
-    cudaLaunchConfig_t cfg = tail_config(a.ctas, std::max(1, a.nrhs), bytes, s, &attr);
+    cudaLaunchConfig_t cfg = tail_config(a.ctas, TailCfg<T>::TT, std::max(1, a.nrhs), bytes, s, &attr);
     switch (axis) {
-        case 0: ANL_CUDA(cudaLaunchKernelEx(&cfg, k_vtail<0>, a)); break;
-        case 1: ANL_CUDA(cudaLaunchKernelEx(&cfg, k_vtail<1>, a)); break;
-        default: ANL_CUDA(cudaLaunchKernelEx(&cfg, k_vtail<2>, a)); break;
+        case 0: ANL_CUDA(cudaLaunchKernelEx(&cfg, k_vtail<T, 0>, a)); break;
+        case 1: ANL_CUDA(cudaLaunchKernelEx(&cfg, k_vtail<T, 1>, a)); break;
+        default: ANL_CUDA(cudaLaunchKernelEx(&cfg, k_vtail<T, 2>, a)); break;
     }
     ANL_LAUNCH_CHECK();
     return ANL_OK;
 }
+
+template int vtail_prepare<float>(int*);
+template int vtail_prepare<double>(int*);
+template bool vtail_fits<float>(TailLevel<float>*, int, int);
+template bool vtail_fits<double>(TailLevel<double>*, int, int);
+template int launch_vtail<float>(const TailArgs<float>&, cudaStream_t);
+template int launch_vtail<double>(const TailArgs<double>&, cudaStream_t);
 
 ANL_DEBUG_UNIT(vtail)
 
