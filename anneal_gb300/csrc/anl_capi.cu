@@ -300,6 +300,10 @@ static int create(anl_ctx** out, int nx, int ny, int nz, double h, double nu, in
     c->nu = nu;
     c->flags = flags;
     c->fp64 = (flags & ANL_FLAG_FP64) != 0;
+    if (c->fp64) {
+        c->mg_degree_coarse = ANL_MG_DEGREE_COARSE64;
+        c->cheb_lo_coarse = ANL_CHEB_LO_COARSE64;
+    }
     c->rmax = std::max(1, (flags >> 8) & 0xFF);
     c->tsize = c->fp64 ? 8 : 4;
     hex8_ke(nu, 1.0, c->ke);

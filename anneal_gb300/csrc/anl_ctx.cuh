@@ -80,8 +80,16 @@ struct anl_ctx {
     // coarse degree: CG iterations per solve, SIMP iterations/s):
     //   0.05 / 0.05, 2: 48.3, 21.4     0.05 / 0.05, 6: 32.6, 25.3    0.03 / 0.01, 6: 28.8, 28.2
     //   0.03 / 0.002, 6: 27.7, 29.2    0.03 / 0.002, 8: 24.1, 30.4   0.03 / 0.0005, 8: 24.5, 30.0
+    // FP64 contexts take 5 steps from 0.006: there a step on these levels costs 3-10 us of FP64 issue
+    // (an as-built solve at 64x32x32, low end and degree: ms, CG iterations)
+    //   0.002, 8: 56.4, 96   0.004, 6: 50.7, 97   0.006, 5: 47.0, 96   0.01, 4: 45.9, 101   0.03, 3: 47.0, 112
+    // and at 96x48x48
+    //   0.002, 8: 94.3, 90   0.004, 6: 85.0, 88   0.006, 5: 81.3, 88   0.01, 4: 83.0, 94    0.03, 3: 89.5, 107
 #ifndef ANL_MG_DEGREE_COARSE
 #define ANL_MG_DEGREE_COARSE 8
+#endif
+#ifndef ANL_MG_DEGREE_COARSE64
+#define ANL_MG_DEGREE_COARSE64 5
 #endif
     int mg_degree_coarse = ANL_MG_DEGREE_COARSE;
     int degree(size_t l) const { return l >= 2 ? mg_degree_coarse : mg_degree; }
@@ -125,6 +133,9 @@ struct anl_ctx {
 #endif
 #ifndef ANL_CHEB_LO_COARSE
 #define ANL_CHEB_LO_COARSE 0.002
+#endif
+#ifndef ANL_CHEB_LO_COARSE64
+#define ANL_CHEB_LO_COARSE64 0.006
 #endif
     // Lower ends of the smoothed intervals, as fractions of their upper end (levels 0-1, 2+). With
     // two steps 0.1 damps what the next level cannot represent and leaves the rest to it; CG

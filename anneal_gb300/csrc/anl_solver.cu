@@ -7,8 +7,8 @@
 //    coarse element scale = (sum of the 8 children)/4 (their mean at Ke(2h) = 2 Ke(h)),
 //    trilinear prolongation P and restriction P^T, Chebyshev smoothing on D^-1 K below the
 //    element bound lambda_max(Ke) / Ke_00 (an upper bound of the spectrum for every design):
-//    2 steps over [0.1, 1] x bound on levels 0-1, 8 steps over [0.002, 1] x bound on the
-//    latency-bound levels below; a dense inverse on the coarsest grid, formed
+//    2 steps over [0.1, 1] x bound on levels 0-1, 8 steps over [0.002, 1] x bound (FP64: 5 over
+//    [0.006, 1]) on the latency-bound levels below; a dense inverse on the coarsest grid, formed
 //    anew every solve (a high-degree Chebyshev sweep if that grid is too large for a dense factor);
 //  * the CG iterate x and right-hand side stay in FP64; the CG scalars come from FP64
 //    reductions (compensated FP32 partials); the residual is replaced by the true residual
