@@ -448,10 +448,8 @@ static int create(anl_ctx** out, int nx, int ny, int nz, double h, double nu, in
         return ANL_ERR_CUDA;
     }
     c->use_graph = std::getenv("ANL_NO_GRAPH") == nullptr;
-    if (const char* e = std::getenv("ANL_BOX_FROM")) c->box_from = std::atoi(e);
     if (const char* e = std::getenv("ANL_TC")) c->use_tc = !c->fp64 && std::atoi(e) != 0;
     ku_prepare();
-    kbox_prepare();
     if (c->use_tc && kutc_prepare(c->ke) != ANL_OK) {
         free_ctx(c);
         return ANL_ERR_CUDA;
@@ -519,7 +517,6 @@ int anl_debug_oob(long long* count_h, long long* first_h) {
     unsigned long long n = 0;
     ANL_TRY(anl::debug_take_ku(&n, first_h));
     ANL_TRY(anl::debug_take_ku64(&n, first_h));
-    ANL_TRY(anl::debug_take_kbox(&n, first_h));
     ANL_TRY(anl::debug_take_solver(&n, first_h));
     ANL_TRY(anl::debug_take_design(&n, first_h));
     ANL_TRY(anl::debug_take_vtail(&n, first_h));

@@ -93,9 +93,6 @@ struct anl_ctx {
 #endif
     int mg_degree_coarse = ANL_MG_DEGREE_COARSE;
     int degree(size_t l) const { return l >= 2 ? mg_degree_coarse : mg_degree; }
-    // first level smoothed by the box kernels (anl_kbox.cu; FP32 contexts): on the levels below
-    // 128 x 64 x 64 elements a z-marching K u launch is a chain of latencies
-    int box_from = 2;
     // the finest level's K u passes on the tensor cores (anl_kutc.cu; FP32 contexts)
     bool use_tc = false;
     // first level of the V-cycle tail (anl_vtail.cu; FP32 contexts), -1 for none, and the CTAs of

@@ -1093,78 +1093,6 @@ static int smooth(anl_ctx* c, Level& L, int degree, bool x_is_zero, const int* d
 template <class T>
 static int vcycle(anl_ctx* c, size_t l, const int* done, cudaStream_t s);
 
-// One V-cycle step on a level the box kernels (anl_kbox.cu) smooth: the pre-smoothing sweep
-// from x = 0 (its first two steps fused), the residual, the restriction, the coarser levels,
-// then the post-smoothing sweep whose first step also adds the coarse-grid correction.
-static int vcycle_box(anl_ctx* c, size_t l, int deg, const int* done, cudaStream_t s) {
-    Level& L = c->lev[l];
-    Level& C = c->lev[l + 1];
-    const double* cf = c->cheb_d + l * kChebStride + 1;  // (c1, c2) pairs
-    KbArgs base;
-    base.d = L.d;
-    base.E = L.E;
-    base.nmask = L.nmask;
-    base.diag = L.diag;
-    base.b = (const float*)L.b;
-    base.done = done;
-    base.nrhs = c->rb;
-    base.vstride = L.vs;
-    base.cstride = C.vs;
-    base.sc_bytes = (int)sizeof(PcgScalars);
-    int k0 = 0;
-    if (deg >= 2) {
-        KbArgs a = base;
-        a.cheb0 = cf;
-        a.cheb = cf + 2;
-        a.dv = (float*)L.dv;
-        a.xout = (float*)L.x;
-        a.dv_keep = deg > 2;
-        ANL_TRY(launch_kbox(KB_CHEB0, a, c->kmf, s));
-        k0 = 2;
-    } else {
-        k_cheb_first<float><<<dim3(vgrid(L.d.nn()), c->rb), VT, 0, s>>>(L.d.nn(), (const float*)L.b, L.diag, L.nmask, cf + 1,
-                                                            (float*)L.x, (float*)L.dv, done, bt_of(c, L));
-        ANL_LAUNCH_CHECK();
-        k0 = 1;
-    }
-    for (int k = k0; k < deg; ++k) {
-        KbArgs a = base;
-        a.u = (const float*)L.x;
-        a.dv = (float*)L.dv;
-        a.xout = (float*)L.xt;
-        a.cheb = cf + 2 * k;
-        a.dv_keep = k + 1 < deg;
-        ANL_TRY(launch_kbox(KB_CHEB, a, c->kmf, s));
-        std::swap(L.x, L.xt);
-    }
-    {
-        KbArgs a = base;
-        a.u = (const float*)L.x;
-        a.y = (float*)L.r;
-        ANL_TRY(launch_kbox(KB_RESID, a, c->kmf, s));
-    }
-    k_restrict<float><<<transfer_grid(C.d, c->rb), dim3(TR_X, TR_Y), 0, s>>>(L.d, C.d, (const float*)L.r, C.nmask,
-                                                                            (float*)C.b, done, bt_of(c, L, &C));
-    ANL_LAUNCH_CHECK();
-    ANL_TRY(vcycle<float>(c, l + 1, done, s));
-    for (int k = 0; k < deg; ++k) {
-        KbArgs a = base;
-        a.u = (const float*)L.x;
-        a.dv = (float*)L.dv;
-        a.xout = (float*)L.xt;
-        a.cheb = cf + 2 * k;
-        a.c1_zero = k == 0;
-        a.dv_keep = k + 1 < deg;
-        if (k == 0) {
-            a.dc = C.d;
-            a.xc = (const float*)C.x;
-        }
-        ANL_TRY(launch_kbox(k == 0 ? KB_PCHEB : KB_CHEB, a, c->kmf, s));
-        std::swap(L.x, L.xt);
-    }
-    return ANL_OK;
-}
-
 // The levels from tail_from down in one cluster per right-hand-side slot: b of level l in, its
 // correction x out.
 template <class T>
@@ -1214,7 +1142,6 @@ static int vcycle(anl_ctx* c, size_t l, const int* done, cudaStream_t s) {
     }
     Level& C = c->lev[l + 1];
     const int deg = c->degree(l);
-    if (sizeof(T) == 4 && (int)l >= c->box_from) return vcycle_box(c, l, deg, done, s);
     ANL_TRY(smooth<T>(c, L, deg, true, done, s));
     KuArgs<T> a = ku_args<T>(c, L);
     a.u = (const T*)L.x;
