@@ -574,7 +574,9 @@ int launch_ku(int mode, const KuArgs<T>& args, const KeModal<T>& km, cudaStream_
         default: return ANL_ERR_BADARG;
     }
     // One wave of CTAs. A segment costs one extra element layer and its ring prologue, and a plane
-    // step is a ~1 us latency chain, so small (coarse-level) grids spread over many short segments.
+    // step is a ~1 us latency chain, so small (coarse-level) grids spread over many short segments,
+    // of one plane where that fits the wave (per CG iteration, against two planes at least: 48x24x24
+    // 107.5 -> 104.4 us, 96x48x48 188.1 -> 185.2).
     // Where the pass sums (the p.Kp reduction follows the CTAs) every slot of a batch gets the
     // partition a single solve gets, so its iterates are those of its own solve. The other passes
     // give a node the same value in any partition, so the slots share the wave (per CG iteration of
@@ -582,7 +584,7 @@ int launch_ku(int mode, const KuArgs<T>& args, const KeModal<T>& km, cudaStream_
     // the remainder leaves more than an eighth of it idle.
     const int nrhs = std::max(1, a.nrhs);
     const int per_rhs = mode != KU_APPLY_DOT && nrhs <= resident / 8 ? resident / nrhs : std::max(1, resident);
-    a.kz = (int)std::max<int64_t>(2, (total + per_rhs - 1) / per_rhs);
+    a.kz = (int)((total + per_rhs - 1) / per_rhs);
     const int blocks = (int)((total + a.kz - 1) / a.kz);
     dim3 block(32, KmCfg<T>::NW);
     const dim3 grid(blocks, std::max(1, a.nrhs));
@@ -612,7 +614,7 @@ int launch_ku_resid_df(const KuArgs<DF>& args, const KeModal<DF>& km, cudaStream
     const int NXn = d.nx + 1, NYn = d.ny + 1, NZn = d.nz + 1;
     const int64_t total = (int64_t)ceil_div(NXn, KmCfg<DF>::OX) * ceil_div(NYn, KmCfg<DF>::OY) * NZn;
     const int resident = ku_resident<DF, KU_RESID>();
-    a.kz = (int)std::max<int64_t>(2, (total + resident - 1) / resident);
+    a.kz = (int)((total + resident - 1) / resident);
     const int blocks = (int)((total + a.kz - 1) / a.kz);
     if (blocks > a.partial_capacity) {
         set_error("accurate residual: %d blocks exceed the reduction scratch (%d)", blocks, a.partial_capacity);
