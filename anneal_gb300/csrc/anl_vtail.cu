@@ -17,7 +17,8 @@
 //      its Chebyshev update and writes its new value to its own copy of the iterate and, from a
 //      boundary plane, to the neighbour's halo plane: st.async into distributed shared memory,
 //      counted by the neighbour's mbarrier;
-//   3. the CTA waits for its own two halo planes only. The iterate is double-buffered and there is
+//   3. the CTA waits for its own two halo planes only (FP32: only the elements at them do, the
+//      others are computed meanwhile). The iterate is double-buffered and there is
 //      a barrier per direction and buffer: a neighbour can be one step ahead, never two, since it
 //      needs this CTA's plane of every step. (A cluster barrier a step costs 0.9 us: its release
 //      drains the remote stores first.)
@@ -46,6 +47,10 @@ struct TailCfg<float> {
     // one CTA's step takes 0.9 us at 128 elements, shorter than a shared one, whose halo flight
     // alone takes 0.7 us; at 432 it is not (2 us)
     static constexpr int TT = 512, NPT = 2, ALONE = 256, MOST = 1 << 30;
+    // EARLY: only the elements that need a halo plane wait for it, the others work meanwhile (per CG
+    // iteration 96x48x48 185.2 -> 181.8 us, 256x128x128 850.9 -> 841.0; in FP64, where a CTA has one
+    // layer of its own and so no such element, the test costs 1 %)
+    static constexpr bool EARLY = true;
 };
 template <>
 struct TailCfg<double> {
@@ -53,6 +58,7 @@ struct TailCfg<double> {
     // CTA takes no more than one warp of them, and above five warps in each of 16 CTAs the 152 SMs
     // of a launch are faster again.
     static constexpr int TT = 256, NPT = 2, ALONE = 32, MOST = 160;
+    static constexpr bool EARLY = false;
 };
 constexpr int FW = 25;          // words between two elements' forces (24 and one of padding)
 constexpr int kWaitTries = 1 << 20;  // bound of a halo wait
@@ -220,6 +226,7 @@ struct Tail {
     int tid, rank, ctas, slot;
     int cur = 0;                  // the buffer that holds the iterate
     unsigned phase = 0;           // next phase parity of barrier [direction][buffer], one bit each
+    unsigned due = 0;             // per direction: 1 + the parity the last exchange's halo plane completes, or 0
     bool lost = false;            // a halo wait ran out
     TailNode<T> nd[NPT];
 
@@ -247,7 +254,9 @@ struct Tail {
             const float Ee = first + q >= 0 && ANL_IN_RANGE(ge, lv.d.ne()) ? __ldg(lv.E + ge) : 0.f;
             // node plane 0 is the halo below; a level in one CTA starts at plane 1
             const int n0 = (q + q0) * g.planeN + aa + g.PA * b, pe = ((q + q0) * (g.B + 1) + b + 1) * g.PA + aa + 1;
-            et[e] = make_float2(Ee, __int_as_float(n0 | (pe << 16)));
+            // the top bit: the element has nodes of a halo plane
+            const bool halo = g.active > 1 && ((q == 0 && rank > 0) || (first + q + 1 == (rank + 1) * g.per && rank + 1 < g.active));
+            et[e] = make_float2(Ee, __int_as_float(n0 | (pe << 16) | (halo ? 0x80000000 : 0)));
         }
     }
 
@@ -283,8 +292,8 @@ struct Tail {
         }
     }
 
-    // the nodes' x into the other buffer and the neighbours' halo planes; then the wait for the own
-    // halo planes
+    // the nodes' x into the other buffer and the neighbours' halo planes; with EARLY the threads whose
+    // elements need the own halo planes wait for them there (wait_halo), otherwise every thread here
     __device__ void exchange(int l) {
         const TailGeo& g = a.lev[l].g;
         cur ^= 1;
@@ -308,28 +317,46 @@ struct Tail {
 #pragma unroll
             for (int c = 0; c < 3; ++c) sm[o + n.nl + c] = n.x[c];
         }
+        due = 0;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             if (!from[q]) continue;
             const unsigned bit = 2 * q + cur;
-            if (!lost) lost = !bar_wait(bar + 8u * bit, (phase >> bit) & 1u);
+            due |= (1u + ((phase >> bit) & 1u)) << (2 * q);
             phase ^= 1u << bit;
         }
+        if (!TailCfg<T>::EARLY) wait_halo();
         __syncthreads();
     }
 
+    // This thread's wait for the halo planes of the last exchange. Some thread of the CTA waits in every
+    // step (each side's halo plane has elements at it), and all pass a barrier after that, so the
+    // next use of an mbarrier finds this phase complete.
+    __device__ void wait_halo() {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const unsigned w = (due >> (2 * q)) & 3u;
+            if (w != 0 && !lost) lost = !bar_wait(bar + 8u * (2 * q + cur), w - 1u);
+        }
+    }
+
     // the corner forces of the CTA's elements (corner pa + 2 pb + 4 ps in slab directions)
-    __device__ void elements(int l) const {
+    __device__ void elements(int l) {
         const TailGeo& g = a.lev[l].g;
         const int ne = elems(g);
         const T* x = sm + cur * a.lay.xlen;
         const float2* et = reinterpret_cast<const float2*>(sm + a.lay.e[l]);
         T* F = sm + a.lay.f[l];
         const int sx = 3 * g.p[0], sy = 3 * g.p[1], sz = 3 * g.p[2];
+        bool waited = false;
         for (int e = tid; e < ne; e += TT) {
             const float2 te = et[e];
-            if (te.x == 0.f) continue;  // its forces stay the zeros of table()
             const int tab = __float_as_int(te.y);
+            if (TailCfg<T>::EARLY && tab < 0 && !waited) {
+                wait_halo();
+                waited = true;
+            }
+            if (te.x == 0.f) continue;  // its forces stay the zeros of table()
             const T* p0 = x + 3 * (tab & 0xffff);
             V3<T> u[2][2][2];
 #pragma unroll
@@ -356,7 +383,7 @@ struct Tail {
 #pragma unroll
                 for (int py = 0; py < 2; ++py) dz[px][py] = u[px][py][1] - u[px][py][0];
             modal_element<T>(a.km, T(te.x), dxb, dxt, dyb, dyt, dz, f);
-            T* fo = F + FW * (tab >> 16);
+            T* fo = F + FW * ((tab >> 16) & 0x7fff);
 #pragma unroll
             for (int pz = 0; pz < 2; ++pz)
 #pragma unroll
@@ -558,6 +585,7 @@ __global__ void __launch_bounds__(TailCfg<T>::TT, 1) k_vtail(const __grid_consta
         }
         t.exchange(l);
         for (int k = 0; k < deg; ++k) t.step(l, k == 0 ? T(0) : cf[l][2 * k], cf[l][2 * k + 1]);
+        if (TailCfg<T>::EARLY) t.wait_halo();  // (nothing reads the last halo planes, but their stores have to be in)
         T* xo = t.vec(a.lev[l].x, l);
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
