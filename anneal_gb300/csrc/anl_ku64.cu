@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(NT64) k_ku64_nodes(KuArgs<double> a, const dou
 bool ku64_split(const Dims& d, int sms, int march_ox, int march_oy, int march_warps) {
     if (d.ne() > (1 << 20)) return false;  // 200 MB of forces
     const int64_t planes = (int64_t)ceil_div(d.nx + 1, march_ox) * ceil_div(d.ny + 1, march_oy) * (d.nz + 1);
-    const int64_t march = (std::max<int64_t>(2, (planes + sms - 1) / sms) + 1) * march_warps * 150;
+    const int64_t march = ((planes + sms - 1) / sms + 1) * march_warps * 150;
     const int64_t split = ceil_div(ceil_div(d.ne(), 32), sms) * (int64_t)190 + ceil_div(ceil_div(d.nn(), 32), sms) * (int64_t)35;
     return 16 * split + 8000 < 16 * march;
 }
