@@ -572,7 +572,8 @@ struct OcState {
     int tlo, thi;        // bits of the largest lambda known above the target volume and of the smallest
                          // one not above it; next to the bisection's bracket while not known
     int width;           // the interval before the last pass (0: a side was not known)
-    double flo, fhi;     // their volumes (NaN: not known)
+    int known;           // bit 0: tlo is such a lambda, bit 1: thi is
+    double flo, fhi;     // their volumes
     OcBank bank;         // the lambdas of the next pass
 };
 
@@ -581,6 +582,7 @@ struct OcState {
 __device__ void oc_advance(OcState* st, const double* vols, int nmax, int lane) {
     int tlo = st->tlo, thi = st->thi;
     const int n = st->bank.n, width = st->width;
+    int known = st->known;
     double flo = st->flo, fhi = st->fhi;
     const double target = st->vtarget;
     // a lane per lambda: the largest above the target, then the smallest not above it beyond that
@@ -590,12 +592,14 @@ __device__ void oc_advance(OcState* st, const double* vols, int nmax, int lane) 
     const int up = __reduce_max_sync(0xffffffffu, lane < n && above ? pj : -1);
     if (up > tlo) {
         tlo = up;
+        known |= 1;
         flo = __shfl_sync(0xffffffffu, vj, __ffs(__ballot_sync(0xffffffffu, lane < n && above && pj == up)) - 1);
     }
     const bool low = lane < n && !above && pj > tlo;
     const int dn = __reduce_min_sync(0xffffffffu, low ? pj : INT_MAX);
     if (dn < thi) {
         thi = dn;
+        known |= 2;
         fhi = __shfl_sync(0xffffffffu, vj, __ffs(__ballot_sync(0xffffffffu, low && pj == dn)) - 1);
     }
     const int gap = thi - tlo - 1;
@@ -617,17 +621,17 @@ __device__ void oc_advance(OcState* st, const double* vols, int nmax, int lane) 
     }
     // Next: from a known side towards the other end in octaves 2, 8, 32, ...; every float while they
     // fit the bank; around the zero of the line through the two ends (its error shrinks with the
-    // square of the interval) at doubling distances; or, where that did not halve the interval, at
-    // even distances
+    // square of the interval) at doubling distances; or, where that did not halve the interval or a
+    // volume is not finite, at even distances
     const int m = min(nmax, gap), h = (m - 1) / 2;
-    const bool known = !isnan(flo) && !isnan(fhi);
+    const bool both = known == 3, line = isfinite(flo) && isfinite(fhi);
     int p;
     if (gap <= nmax) {
         p = tlo + 1 + lane;
-    } else if (!known) {
+    } else if (!both) {
         const long long d = 2ll << (23 + 2 * min(lane, 8));
-        p = isnan(fhi) ? (int)min(tlo + d, (long long)thi - 1) : (int)max(thi - d, (long long)tlo + 1);
-    } else if (width > 0 && thi - tlo > width / 2) {
+        p = known == 1 ? (int)min(tlo + d, (long long)thi - 1) : (int)max(thi - d, (long long)tlo + 1);
+    } else if (!line || (width > 0 && thi - tlo > width / 2)) {
         p = tlo + (int)((int64_t)(thi - tlo) * (lane + 1) / (m + 1));
     } else {
         const double d = thi - tlo;
@@ -643,7 +647,8 @@ __device__ void oc_advance(OcState* st, const double* vols, int nmax, int lane) 
         st->bank.n = m;
         st->tlo = tlo;
         st->thi = thi;
-        st->width = known ? thi - tlo : 0;
+        st->known = known;
+        st->width = both ? thi - tlo : 0;
         st->flo = flo;
         st->fhi = fhi;
     }
@@ -677,6 +682,7 @@ __global__ void k_oc_begin(OcState* st, const double* sums, const double* vfroze
         st->tlo = a - 1;
         st->thi = b + 1;
         st->width = 0;
+        st->known = 0;
         st->flo = st->fhi = NAN;
         st->bank.n = n;
     }
