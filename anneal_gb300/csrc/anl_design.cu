@@ -735,7 +735,7 @@ __global__ void __launch_bounds__(OCB_T, 1) k_oc_vol_bank(int64_t ne, const floa
 }
 
 // One pass with projection: the volume sum phi physical(xn(lambda)) of each lambda of the bank,
-// xn filtered as in k_filter; phi xp is summed exactly as float pairs.
+// xn filtered as in k_filter; phi xp is formed (exactly) and summed in FP64.
 struct OcProjArgs {
     FilterArgs f;
     const float4* el;
@@ -749,8 +749,7 @@ template <int R>
 __global__ void __launch_bounds__(FT_N) k_oc_vol_proj(OcProjArgs a) {
     if (a.st->stop) return;  // the same for every block
     using Tile = FilterTile<R>;
-    __shared__ float pl[2][OC_PROJ][Tile::PL];
-    __shared__ float2 sm[OC_PROJ * FT_N / 32];
+    __shared__ __align__(8) float pl[2][OC_PROJ][Tile::PL];
     const Dims d = a.f.d;
     const int n = a.st->bank.n;
     float lam[OC_PROJ], rl[OC_PROJ];
@@ -779,11 +778,13 @@ __global__ void __launch_bounds__(FT_N) k_oc_vol_proj(OcProjArgs a) {
     const int i = i0 + tx, j = j0 + ty;
     const bool in_xy = i < d.nx && j < d.ny;
     float acc[OC_PROJ][2 * R + 1];
-    PairSum vol[OC_PROJ];
+    double vol[OC_PROJ];
 #pragma unroll
-    for (int m = 0; m < OC_PROJ; ++m)
+    for (int m = 0; m < OC_PROJ; ++m) {
+        vol[m] = 0.0;
 #pragma unroll
         for (int q = 0; q < 2 * R + 1; ++q) acc[m][q] = 0.f;
+    }
     for (int gk = kb - R; gk < kend + R; ++gk) {
         float(&buf)[OC_PROJ][Tile::PL] = pl[gk & 1];
 #pragma unroll
@@ -812,25 +813,17 @@ __global__ void __launch_bounds__(FT_N) k_oc_vol_proj(OcProjArgs a) {
             if (in_e) {
                 const float th = tanhf(a.f.beta * (acc[m][0] / hs - a.f.eta));
                 const float xp = fzn ? 1.f : (a.f.t0 + th) / (a.f.t0 + a.f.t1);
-                float pv, pr;
-                two_prod(ph, xp, pv, pr);
-                vol[m].add(pv);
-                vol[m].l += pr;
+                vol[m] = fma((double)ph, (double)xp, vol[m]);
             }
 #pragma unroll
             for (int q = 0; q < 2 * R; ++q) acc[m][q] = acc[m][q + 1];
             acc[m][2 * R] = 0.f;
         }
     }
-    float h[OC_PROJ], l[OC_PROJ];
-#pragma unroll
-    for (int m = 0; m < OC_PROJ; ++m) {
-        h[m] = vol[m].h;
-        l[m] = vol[m].l;
-    }
+    static_assert(sizeof(pl) >= OC_PROJ * FT_N * sizeof(double), "the threads' sums in place of the planes");
     const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    if (reduce_pairs_wide<OC_PROJ, FT_N>(h, l, bid, gridDim.x * gridDim.y * gridDim.z, a.partials, a.counter, a.out, tid,
-                                         sm) && tid < 32)
+    if (reduce_doubles_wide<OC_PROJ, FT_N>(vol, bid, gridDim.x * gridDim.y * gridDim.z, a.partials, a.counter, a.out, tid,
+                                           reinterpret_cast<double*>(&pl[0][0][0])) && tid < 32)
         oc_advance(a.st, a.out, OC_PROJ, tid);
 }
 
