@@ -246,6 +246,7 @@ int filter_init(anl_ctx* c, double r, cudaStream_t s) {
     FilterArgs a = filter_args(c);
     a.out = c->filt.Hs;
     ANL_TRY(launch_filter<F_HS>(c, a, s));
+    ANL_CUDA(cudaStreamSynchronize(s));  // Hs is read by calls on any stream from here on
     c->filt.ready = true;
     return ANL_OK;
 }

@@ -122,7 +122,8 @@ int anl_stiffness_scale(anl_ctx* ctx, const float* xphys, const float* phi, doub
 /* ---------------------------------------------------------------- density filter */
 
 /* Filter.__init__ (optimize.py:25-34): cone weights max(0, r - |d|) on a (2R+1)^3 box,
-   R = max(ceil(r) - 1, 1) (R <= 5), Hs = conv(active) with zeros set to 1. */
+   R = max(ceil(r) - 1, 1) (R <= 5), Hs = conv(active) with zeros set to 1. Synchronises the
+   stream: the filter can be used on any stream afterwards. */
 int anl_filter_init(anl_ctx* ctx, double r_vox, anl_stream_t stream);
 /* Filter.forward (optimize.py:41-43): out = conv(in * active) / Hs on active elements. */
 int anl_filter_fwd(anl_ctx* ctx, const float* in, float* out, anl_stream_t stream);
