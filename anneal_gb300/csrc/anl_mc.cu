@@ -398,7 +398,8 @@ struct PruneState {
     unsigned long long vmax;  // bits of the largest |volume|
     long long hi, lo;         // the kept components' volume
     int coord;                // bits of the largest |coordinate|
-    int dropped, bad;
+    int dropped, bad;         // bad: a face's volume is no number
+    int ncomp;
 };
 
 __global__ void k_pr_extent(int64_t n, const float* v, PruneState* st) {
@@ -464,7 +465,10 @@ __device__ __forceinline__ double prune_volume(longlong2 a) {  // in units of 1 
 }
 __global__ void k_pr_max(int64_t nv, const longlong2* acc, const int* has, PruneState* st) {
     for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < nv; l += (int64_t)gridDim.x * blockDim.x)
-        if (has[l]) atomicMax(&st->vmax, (unsigned long long)__double_as_longlong(prune_volume(acc[l])));
+        if (has[l]) {
+            atomicMax(&st->vmax, (unsigned long long)__double_as_longlong(prune_volume(acc[l])));
+            atomicAdd(&st->ncomp, 1);
+        }
 }
 // keep[l] of every label: 1 kept, 0 dropped; the labels dropped and the kept volume
 __global__ void k_pr_label(int64_t nv, const longlong2* acc, const int* has, double fraction, int* keep, PruneState* st) {
@@ -472,7 +476,8 @@ __global__ void k_pr_label(int64_t nv, const longlong2* acc, const int* has, dou
     for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < nv; l += (int64_t)gridDim.x * blockDim.x) {
         bool k = false;
         if (has[l]) {
-            k = !st->bad && prune_volume(acc[l]) >= least;  // a volume that is no number keeps nothing
+            // a volume that is no number compares with no other: only a component by itself stays
+            k = st->bad ? st->ncomp == 1 : prune_volume(acc[l]) >= least;
             if (k) add_fixed(&st->hi, &st->lo, acc[l].x, acc[l].y);
             else atomicAdd(&st->dropped, 1);
         }
@@ -800,8 +805,8 @@ int anl_mc_prune(anl_mc* m, double fraction, int64_t* nverts_h, int64_t* nfaces_
     float coord;
     std::memcpy(&coord, &st->coord, sizeof(coord));
     const double unit = std::ldexp(1.0, 3 * (std::ilogb(std::max(coord, 1e-12f)) + 1) - 30);  // 1 / prune_scale
-    *volume_h = ((double)st->hi + (double)st->lo / 1073741824.0) * unit;
     *dropped_h = st->dropped;
+    *volume_h = st->bad && st->dropped == 0 ? std::nan("") : ((double)st->hi + (double)st->lo / 1073741824.0) * unit;
     if (st->dropped == 0) return ANL_OK;
     // the kept vertices and faces, in their order
     ANL_TRY(grow(m->fflag, m->fflag_cap, nf, sizeof(int)));

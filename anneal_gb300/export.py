@@ -161,7 +161,7 @@ def surface(grid, f, level, upsample=2, smooth=10, log=print):
         faces = fc.long().cpu().numpy()
     finally:
         mc.close()
-    mesh = Mesh(verts, faces if volume >= 0 else faces[:, ::-1])   # export.py:145-146
+    mesh = Mesh(verts, faces[:, ::-1] if volume < 0 else faces)   # export.py:145-146
     try:
         import trimesh
         return trimesh.Trimesh(mesh.vertices, mesh.faces, process=False)

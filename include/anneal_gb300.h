@@ -207,7 +207,8 @@ int anl_mc_components(anl_mc* mc, int32_t* face_label, int* rounds_h, anl_stream
    |signed volume| is below `fraction` of the largest one's. The current mesh becomes the kept
    components, vertices and faces in their order (as numpy's unique and boolean indexing give
    them; untouched when nothing is dropped); writes its counts, the number of components dropped
-   and its signed volume (host). A volume that is no number drops everything. */
+   and its signed volume (host). A volume that is no number (of NaN vertices) drops everything,
+   but a mesh of one component, whose volume is then NaN. */
 int anl_mc_prune(anl_mc* mc, double fraction, int64_t* nverts_h, int64_t* nfaces_h, int64_t* dropped_h, double* volume_h,
                  anl_stream_t stream);
 
