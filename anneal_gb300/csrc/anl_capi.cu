@@ -458,6 +458,7 @@ static int create(anl_ctx** out, int nx, int ny, int nz, double h, double nu, in
     {
         const char* e = std::getenv("ANL_TAIL");
         const bool tail_on = !(e && std::atoi(e) == 0);
+        if (const char* lf = std::getenv("ANL_TAIL_LOSE_FROM")) c->tail_lose_from = std::atoi(lf);
         const int nl = (int)c->lev.size();
         if (tail_on && c->dense_coarse && nl >= 2) {
             if ((c->fp64 ? find_tail<double>(c) : find_tail<float>(c)) != ANL_OK) {

@@ -98,6 +98,7 @@ struct anl_ctx {
     // first level of the V-cycle tail (anl_vtail.cu; FP32 contexts), -1 for none, and the CTAs of
     // its cluster
     int tail_from = -1, tail_ctas = 0;
+    int tail_lose_from = 1 << 30;  // TailArgs::lose_from (ANL_TAIL_LOSE_FROM)
     // right-hand-side slots (ANL_FLAG_RHS): the solve's per-vector state (the hierarchy's
     // vectors, p, q, the FP64 solution and right-hand side, its float-pair split, the PCG
     // scalars, the restart flags, the reduction scratch) exists once per slot; a batched solve

@@ -156,6 +156,8 @@ struct TailArgs {
     int nc = 0;
     const int* done = nullptr;
     KeModal<T> km{};
+    // a check of the error path: the early halo waits of the threads from this one on count as run out
+    int lose_from = 1 << 30;
     // right-hand-side slots: cluster r works on slot r
     int nrhs = 1;
     int sc_bytes = 0;  // bytes between the slots' done flags

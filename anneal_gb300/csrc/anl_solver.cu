@@ -1100,6 +1100,7 @@ static int vcycle_tail(anl_ctx* c, size_t l, const int* done, cudaStream_t s) {
     TailArgs<T> a;
     a.nlev = (int)(c->lev.size() - l);
     a.ctas = c->tail_ctas;
+    a.lose_from = c->tail_lose_from;
     for (int q = 0; q < a.nlev; ++q) {
         const Level& Lq = c->lev[l + q];
         a.lev[q].d = Lq.d;

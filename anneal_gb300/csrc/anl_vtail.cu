@@ -227,7 +227,8 @@ struct Tail {
     int cur = 0;                  // the buffer that holds the iterate
     unsigned phase = 0;           // next phase parity of barrier [direction][buffer], one bit each
     unsigned due = 0;             // per direction: 1 + the parity the last exchange's halo plane completes, or 0
-    bool lost = false;            // a halo wait ran out
+    bool lost = false;            // a halo wait of this thread ran out
+    volatile int* cta_lost;       // (shared) 2: one of any thread of the CTA has; 1: one counts as run out
     TailNode<T> nd[NPT];
 
     __device__ T* vec(T* p, int l) const { return p + (int64_t)slot * a.lev[l].vs; }
@@ -298,7 +299,7 @@ struct Tail {
         const TailGeo& g = a.lev[l].g;
         cur ^= 1;
         const bool from[2] = {rank > 0 && rank < g.active, rank + 1 < g.active};
-        if (tid == 0) {
+        if (tid == 0 && *cta_lost < 2) {  // (a phase that a lost wait left open takes no second arrival)
 #pragma unroll
             for (int q = 0; q < 2; ++q)
                 if (from[q]) bar_expect(bar + 8u * (2 * q + cur), 3u * (unsigned)sizeof(T) * (unsigned)g.planeN);
@@ -336,7 +337,10 @@ struct Tail {
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const unsigned w = (due >> (2 * q)) & 3u;
-            if (w != 0 && !lost) lost = !bar_wait(bar + 8u * (2 * q + cur), w - 1u);
+            if (w != 0 && !lost && !bar_wait(bar + 8u * (2 * q + cur), w - 1u)) {
+                lost = true;
+                *cta_lost = 2;
+            }
         }
     }
 
@@ -354,6 +358,7 @@ struct Tail {
             const int tab = __float_as_int(te.y);
             if (TailCfg<T>::EARLY && tab < 0 && !waited) {
                 wait_halo();
+                if (tid >= a.lose_from) *cta_lost = 1;
                 waited = true;
             }
             if (te.x == 0.f) continue;  // its forces stay the zeros of table()
@@ -442,6 +447,7 @@ __global__ void __launch_bounds__(TailCfg<T>::TT, 1) k_vtail(const __grid_consta
     T* tail_smem = reinterpret_cast<T*>(tail_bytes);
     __shared__ T cf[kTailMaxLevels][2 * kTailMaxDegree];
     __shared__ __align__(8) uint64_t bars[2][2];
+    __shared__ int cta_lost;
     const int tid = threadIdx.x, ctas = a.ctas;
     const int rank = blockIdx.x % ctas, slot = blockIdx.x / ctas;
     const int* done = slot_bytes(a.done, slot, a.sc_bytes);
@@ -452,6 +458,7 @@ __global__ void __launch_bounds__(TailCfg<T>::TT, 1) k_vtail(const __grid_consta
 #pragma unroll
         for (int q = 0; q < 4; ++q) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8u * q) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        cta_lost = 0;
     }
     for (int q = tid; q < last * 2 * kTailMaxDegree; q += TT) {
         const int l = q / (2 * kTailMaxDegree), k = q - l * 2 * kTailMaxDegree;
@@ -459,6 +466,7 @@ __global__ void __launch_bounds__(TailCfg<T>::TT, 1) k_vtail(const __grid_consta
     }
     __syncthreads();
     Tail<T, AXIS> t{a, tail_smem, bar, 0, 0, 0, 0, tid, rank, ctas, slot};
+    t.cta_lost = &cta_lost;
     {
         const uint32_t xb = (uint32_t)__cvta_generic_to_shared(tail_smem);
         const int below = rank > 0 ? rank - 1 : 0, above = rank + 1 < ctas ? rank + 1 : rank;
@@ -585,18 +593,23 @@ __global__ void __launch_bounds__(TailCfg<T>::TT, 1) k_vtail(const __grid_consta
         }
         t.exchange(l);
         for (int k = 0; k < deg; ++k) t.step(l, k == 0 ? T(0) : cf[l][2 * k], cf[l][2 * k + 1]);
-        if (TailCfg<T>::EARLY) t.wait_halo();  // (nothing reads the last halo planes, but their stores have to be in)
+        if (TailCfg<T>::EARLY) {  // (nothing reads the last halo planes, but their stores have to be in)
+            t.wait_halo();
+            __syncthreads();
+        }
+        // a lost halo fails the solve, whichever thread waited for it
+        const bool lost = cta_lost != 0;
         T* xo = t.vec(a.lev[l].x, l);
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
             const TailNode<T>& n = t.nd[r];
             if (n.pn < 0) continue;
 #pragma unroll
-            for (int c = 0; c < 3; ++c)  // a lost halo fails the solve
-                xo[3 * (l == 0 ? n.gn : n.pn) + c] = t.lost ? T(NAN) : n.x[c];
+            for (int c = 0; c < 3; ++c) xo[3 * (l == 0 ? n.gn : n.pn) + c] = lost ? T(NAN) : n.x[c];
         }
         cluster_sync();  // the correction is written; at the end no CTA leaves before its neighbours' stores
     }
+    if (cta_lost == 2) __nanosleep(1000000);  // ... which it has not seen arrive if a wait ran out
 }
 
 int tail_axis(const Dims& d) { return d.nx >= d.ny && d.nx >= d.nz ? 0 : d.ny >= d.nz ? 1 : 2; }
