@@ -172,6 +172,7 @@ int solver_apply(anl_ctx* c, const float* escale, const void* u, void* y, cudaSt
 int solver_solve(anl_ctx* c, const float* escale, const double* f, double* x, int nrhs, double rtol, int maxiter,
                  int rebuild, int* iters, double* relres, cudaStream_t s);
 int solver_dot(anl_ctx* c, const double* a, const double* b, double* out, cudaStream_t s);
+int filter_blocks(const Dims& d);
 int filter_init(anl_ctx* c, double r, cudaStream_t s);
 int element_stress(anl_ctx* c, const double* u, const double* Emat, double Escalar, double* sig, double* vm,
                    cudaStream_t s);
@@ -429,11 +430,7 @@ static int create(anl_ctx** out, int nx, int ny, int nz, double h, double nu, in
     ALLOC(c->sc, R * sizeof(PcgScalars));
     c->part_cap = std::max(ku_grid_blocks(c->d), kRedBlocks);
     if (c->fp64 && c->lev[0].split) c->part_cap = std::max(c->part_cap, ceil_div(nn, 128));  // its p.Kp partials
-    {
-        // the filter reduction grid (32 x 8 columns of 16 layers) can exceed both
-        const int fb = ceil_div(c->d.nx, 32) * ceil_div(c->d.ny, 8) * ceil_div(c->d.nz, 16);
-        c->part_cap = std::max(c->part_cap, fb);
-    }
+    c->part_cap = std::max(c->part_cap, filter_blocks(c->d));  // the projected volumes of the OC update
     c->part_stride = (int64_t)c->part_cap * kMaxRedVals;
     ALLOC(c->partials, R * c->part_stride * sizeof(double));
     ALLOC(c->counter, (16 + R) * sizeof(unsigned));

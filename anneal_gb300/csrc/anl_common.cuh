@@ -387,11 +387,7 @@ __device__ __forceinline__ void block_sum(double (&val)[NV], double* smem /* NV*
     }
 }
 
-// The same block sum for values given as unevaluated float pairs (s + c) per thread: the warp
-// tree adds pairs with TwoSum on the FP32 pipes (FP64 arithmetic on this part runs at a small
-// fraction of FP32, and a tree of FP64 adds over every thread of a full grid costs microseconds),
-// each warp's pair becomes one double, and thread 0 adds the warps' doubles in order. About 48
-// significant bits; deterministic. Result valid in the thread with flat index 0.
+// s + e = a + b exactly (TwoSum)
 __device__ __forceinline__ void two_sum_f(float a, float b, float& s, float& e) {
     s = a + b;
     const float bb = s - a;
@@ -400,7 +396,8 @@ __device__ __forceinline__ void two_sum_f(float a, float b, float& s, float& e) 
 // Block sum of NV float pairs (hi + lo per thread), entirely on the FP32 pipes: the warp tree
 // adds pairs with TwoSum, then thread 0 adds the warps' pairs in order. FP64 arithmetic on this
 // part runs at a small fraction of the FP32 rate: even a few FP64 instructions per warp, in every
-// block of a 1,216-block reduction, cost several microseconds. Result in thread 0 (in place).
+// block of a 1,216-block reduction, cost several microseconds. About 48 significant bits; deterministic.
+// Result in thread 0 (in place).
 template <int NV, int NT>
 __device__ __forceinline__ void block_pair_sum(float (&hi)[NV], float (&lo)[NV], float2* smem /* NV*NT/32 */,
                                                int tid) {
@@ -432,23 +429,6 @@ __device__ __forceinline__ void block_pair_sum(float (&hi)[NV], float (&lo)[NV],
             hi[v] = a.x;
             lo[v] = a.y;
         }
-    }
-}
-
-// The same block sum with the result as doubles (thread 0), for finish_reduction.
-template <int NV, int NT>
-__device__ __forceinline__ void block_sum_f2(const float (&s)[NV], const float (&c)[NV], double (&val)[NV],
-                                             double* smem /* NV*NT/32 */, int tid) {
-    float h[NV], l[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        h[v] = s[v];
-        l[v] = c[v];
-    }
-    block_pair_sum<NV, NT>(h, l, reinterpret_cast<float2*>(smem), tid);
-    if (tid == 0) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) val[v] = (double)h[v] + (double)l[v];
     }
 }
 

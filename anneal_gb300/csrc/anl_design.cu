@@ -38,6 +38,13 @@ static inline int filter_chunk(const Dims& d) {
     const int columns = ceil_div(d.nx, FT_X) * ceil_div(d.ny, FT_Y);
     return std::max(4, std::min(FT_ZC, ceil_div(d.nz, ceil_div(3 * 152, columns))));
 }
+static inline dim3 filter_grid(const Dims& d) {
+    return dim3(ceil_div(d.nx, FT_X), ceil_div(d.ny, FT_Y), ceil_div(d.nz, filter_chunk(d)));
+}
+int filter_blocks(const Dims& d) {
+    const dim3 g = filter_grid(d);
+    return (int)(g.x * g.y * g.z);
+}
 
 struct FilterArgs {
     Dims d;
@@ -210,13 +217,10 @@ static FilterArgs filter_args(const anl_ctx* c) {
     a.zc = filter_chunk(a.d);
     return a;
 }
-static dim3 filter_grid(const FilterArgs& a) {
-    return dim3(ceil_div(a.d.nx, FT_X), ceil_div(a.d.ny, FT_Y), ceil_div(a.d.nz, a.zc));
-}
 
 template <int MODE>
 static int launch_filter(anl_ctx* c, const FilterArgs& a, cudaStream_t s) {
-    const dim3 grid = filter_grid(a), block(FT_X, FT_Y);
+    const dim3 grid = filter_grid(a.d), block(FT_X, FT_Y);
     switch (c->filt.R) {
         case 1: k_filter<MODE, 1><<<grid, block, 0, s>>>(a); break;
         case 2: k_filter<MODE, 2><<<grid, block, 0, s>>>(a); break;
@@ -899,7 +903,7 @@ int oc_update(anl_ctx* c, const float* x, const float* dcx, const float* dvx, co
         pa.partials = c->partials;
         pa.counter = c->counter;
         pa.out = c->red_out;
-        pgrid = filter_grid(pa.f);
+        pgrid = filter_grid(pa.f.d);
         if ((int64_t)pgrid.x * pgrid.y * pgrid.z > c->part_cap) {
             set_error("filter reduction needs %d blocks, scratch holds %d", pgrid.x * pgrid.y * pgrid.z, c->part_cap);
             return ANL_ERR_BADARG;
