@@ -156,7 +156,7 @@ struct TailArgs {
     int nc = 0;
     const int* done = nullptr;
     KeModal<T> km{};
-    // a check of the error path: the early halo waits of the threads from this one on count as run out
+    // a check of the error path: the first CTA's threads from this one on count as having lost a halo wait
     int lose_from = 1 << 30;
     // right-hand-side slots: cluster r works on slot r
     int nrhs = 1;

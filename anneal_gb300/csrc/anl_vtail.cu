@@ -228,7 +228,6 @@ struct Tail {
     unsigned phase = 0;           // next phase parity of barrier [direction][buffer], one bit each
     unsigned due = 0;             // per direction: 1 + the parity the last exchange's halo plane completes, or 0
     bool lost = false;            // a halo wait of this thread ran out
-    volatile int* cta_lost;       // (shared) 2: one of any thread of the CTA has; 1: one counts as run out
     TailNode<T> nd[NPT];
 
     __device__ T* vec(T* p, int l) const { return p + (int64_t)slot * a.lev[l].vs; }
@@ -299,7 +298,7 @@ struct Tail {
         const TailGeo& g = a.lev[l].g;
         cur ^= 1;
         const bool from[2] = {rank > 0 && rank < g.active, rank + 1 < g.active};
-        if (tid == 0 && *cta_lost < 2) {  // (a phase that a lost wait left open takes no second arrival)
+        if (tid == 0) {
 #pragma unroll
             for (int q = 0; q < 2; ++q)
                 if (from[q]) bar_expect(bar + 8u * (2 * q + cur), 3u * (unsigned)sizeof(T) * (unsigned)g.planeN);
@@ -337,10 +336,7 @@ struct Tail {
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const unsigned w = (due >> (2 * q)) & 3u;
-            if (w != 0 && !lost && !bar_wait(bar + 8u * (2 * q + cur), w - 1u)) {
-                lost = true;
-                *cta_lost = 2;
-            }
+            if (w != 0 && !lost) lost = !bar_wait(bar + 8u * (2 * q + cur), w - 1u);
         }
     }
 
@@ -358,7 +354,6 @@ struct Tail {
             const int tab = __float_as_int(te.y);
             if (TailCfg<T>::EARLY && tab < 0 && !waited) {
                 wait_halo();
-                if (tid >= a.lose_from) *cta_lost = 1;
                 waited = true;
             }
             if (te.x == 0.f) continue;  // its forces stay the zeros of table()
@@ -466,7 +461,6 @@ __global__ void __launch_bounds__(TailCfg<T>::TT, 1) k_vtail(const __grid_consta
     }
     __syncthreads();
     Tail<T, AXIS> t{a, tail_smem, bar, 0, 0, 0, 0, tid, rank, ctas, slot};
-    t.cta_lost = &cta_lost;
     {
         const uint32_t xb = (uint32_t)__cvta_generic_to_shared(tail_smem);
         const int below = rank > 0 ? rank - 1 : 0, above = rank + 1 < ctas ? rank + 1 : rank;
@@ -593,12 +587,10 @@ __global__ void __launch_bounds__(TailCfg<T>::TT, 1) k_vtail(const __grid_consta
         }
         t.exchange(l);
         for (int k = 0; k < deg; ++k) t.step(l, k == 0 ? T(0) : cf[l][2 * k], cf[l][2 * k + 1]);
-        if (TailCfg<T>::EARLY) {  // (nothing reads the last halo planes, but their stores have to be in)
-            t.wait_halo();
-            __syncthreads();
-        }
-        // a lost halo fails the solve, whichever thread waited for it
-        const bool lost = cta_lost != 0;
+        if (TailCfg<T>::EARLY) t.wait_halo();  // (nothing reads the last halo planes, but their stores have to be in)
+        if (t.lost || (rank == 0 && tid >= a.lose_from)) cta_lost = 1;
+        __syncthreads();
+        const bool lost = cta_lost != 0;  // a lost halo fails the solve, whichever thread waited for it
         T* xo = t.vec(a.lev[l].x, l);
 #pragma unroll
         for (int r = 0; r < NPT; ++r) {
@@ -609,7 +601,7 @@ __global__ void __launch_bounds__(TailCfg<T>::TT, 1) k_vtail(const __grid_consta
         }
         cluster_sync();  // the correction is written; at the end no CTA leaves before its neighbours' stores
     }
-    if (cta_lost == 2) __nanosleep(1000000);  // ... which it has not seen arrive if a wait ran out
+    if (t.lost) __nanosleep(1000000);  // ... which it has not seen arrive if a wait ran out
 }
 
 int tail_axis(const Dims& d) { return d.nx >= d.ny && d.nx >= d.nz ? 0 : d.ny >= d.nz ? 1 : 2; }

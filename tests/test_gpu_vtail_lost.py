@@ -1,7 +1,7 @@
 """A halo wait of the cluster tail that runs out fails the solve, whichever thread waited. The waits are
-only counted as run out here (ANL_TAIL_LOSE_FROM, on the threads from that one on): on 16 x 16 x 16 a CTA
-computes two layers of 256 elements, one to a thread, and but for the last owns one plane of 17 x 17
-nodes, so its threads from 289 on wait for halo planes and own no node."""
+only counted as run out here (ANL_TAIL_LOSE_FROM, in the first CTA's threads from that one on): on
+16 x 16 x 16 a CTA computes two layers of 256 elements, one to a thread, and but for the last owns one
+plane of 17 x 17 nodes, so its threads from 289 on can wait for a halo plane and own no node."""
 import numpy as np
 import pytest
 import torch
