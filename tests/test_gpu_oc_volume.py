@@ -29,7 +29,7 @@ def _case(oracle, shape, r, seed):
 # a volume that is no number is not above the target in the bisection, whatever the multiplier: it ends
 # at the lower end of its bracket; an infinite one is above it, and it ends at the upper end. (With no
 # projection an infinite phi is no number either: the filter's zero weights meet it.)
-@pytest.mark.parametrize("shape,r", [((9, 4, 3), 1.5), ((33, 17, 9), 2.6)])
+@pytest.mark.parametrize("shape,r", [((9, 4, 3), 1.5), ((33, 17, 9), 2.6), ((33, 17, 9), 3.4)])
 @pytest.mark.parametrize("beta,bad", [(0.0, np.nan), (1.0, np.nan), (4.0, np.nan), (1.0, np.inf), (4.0, np.inf)])
 def test_volume_that_is_no_number_ends_as_the_bisection(oracle, shape, r, beta, bad):
     c, F, x, dcx, dvx, phi, frozen = _case(oracle, shape, r, 5)
@@ -46,7 +46,7 @@ def test_volume_that_is_no_number_ends_as_the_bisection(oracle, shape, r, beta, 
     c.close()
 
 
-@pytest.mark.parametrize("r", [1.5, 2.6])
+@pytest.mark.parametrize("r", [1.5, 2.6, 3.4])
 def test_projected_volume_is_summed_in_double_precision(r):
     """One design element beside many frozen ones, whose phi add up to 2^17.6 and are multiples of
     2^-34: FP64 holds their sum exactly in any order. The target leaves the design element, of phi
