@@ -741,9 +741,9 @@ __global__ void __launch_bounds__(OCB_T, 1) k_oc_vol_bank(int64_t ne, const floa
 }
 
 // The double of a float without the FP64 pipe, which converts a warp in some 19 cycles per SM. In
-// k_oc_vol_proj it pays where the filter's registers leave few warps to hide that: an update takes 763
+// k_oc_vol_proj it pays where the filter's registers leave few warps to hide that: an update takes 760
 // instead of 805 us at 192x90x90, R = 3, 251 either way at 97x50x41, R = 2, but 479 instead of 472 at
-// 160x80x80, R = 1.
+// 160x80x80, R = 1 (before reduce_doubles_wide added in trees).
 __device__ __forceinline__ double widen(float v) {
     const unsigned b = __float_as_uint(v), e = (b >> 23) & 0xffu;
     if (e - 1u >= 254u) return (double)v;  // zero, denormal, infinite, no number
