@@ -423,6 +423,7 @@ static int create(anl_ctx** out, int nx, int ny, int nz, double h, double nu, in
             L.split = ku_prefers_split(L.d);
             if (L.split) most = std::max(most, L.d.ne());
         }
+        // 192 bytes to an element of the largest such level: up to 200 MB a context
         if (most > 0) ALLOC(c->f64, 24 * most * sizeof(double));
     }
     ALLOC(c->xbuf, R * vs0 * sizeof(double));

@@ -95,7 +95,7 @@ struct anl_ctx {
     int degree(size_t l) const { return l >= 2 ? mg_degree_coarse : mg_degree; }
     // the finest level's K u passes on the tensor cores (anl_kutc.cu; FP32 contexts)
     bool use_tc = false;
-    // first level of the V-cycle tail (anl_vtail.cu; FP32 contexts), -1 for none, and the CTAs of
+    // first level of the V-cycle tail (anl_vtail.cu), -1 for none, and the CTAs of
     // its cluster
     int tail_from = -1, tail_ctas = 0;
     int tail_lose_from = 1 << 30;  // TailArgs::lose_from (ANL_TAIL_LOSE_FROM)

@@ -21,8 +21,9 @@
 // The caller's K u (KU_APPLY_RAW) takes the y and z edges of both sides and adds the two layers of a
 // node by z mode: rounding errors that are large beside what is left of neighbouring forces then cancel
 // first. Its error against FP64 (root mean square, relative; smooth displacements, 14 grids of 1k to
-// 1.8M elements) is 1.03e-7, 1.09e-7 with the solver passes' order and 1.08e-7 with 8 corner forces to an
-// element.
+// 1.8M elements) is 1.03e-7, 1.09e-7 in the solver passes' order and 1.08e-7 with 8 corner forces to an
+// element; of white noise, where nothing cancels, 6.3e-8, 6.7e-8 and 6.0e-8. It takes 36.8 us at
+// 192x96x96, 36.6 in the solver passes' order.
 // HBM traffic is u once, y once, E once and the node mask once (halo re-reads hit L2).
 //
 // The same kernel in double-float arithmetic (T = DF, residual mode only) evaluates the FP64

@@ -72,7 +72,8 @@ __global__ void __launch_bounds__(NT64) k_ku64_nodes(KuArgs<double> a, const dou
         const int NX = d.nx + 1, NY = d.ny + 1;
         const int i = n % NX, j = n / NX % NY, k = n / (NX * NY);
         const uint8_t nm = a.nmask[n];
-        // all loads in flight together; corners outside the grid are read at an element inside
+        // no load waits for a test: corners outside the grid are read at an element inside. (Not all 24
+        // values are in flight at once: the kernel has 32 registers, so they come in groups.)
         double f[8][3];
         bool in[8];
 #pragma unroll
@@ -125,7 +126,8 @@ __global__ void __launch_bounds__(NT64) k_ku64_nodes(KuArgs<double> a, const dou
 }  // namespace
 
 // Whether a level's FP64 passes take the two kernels: the FP64 instructions of the busiest SM
-// (16 cycles each), march against elements and nodes, and 8,000 cycles for the second launch.
+// (counted at the nominal 16 cycles; with the 19 measured the choice differs for 0.2 % of grids of 4 to
+// 256 elements a side), march against elements and nodes, and 8,000 cycles for the second launch.
 // One pass, two kernels against the march: 64x32x32 34.9 against 60.2 us, 128x64x64 216 against 252;
 // at 256x128x128 the forces alone would be 800 MB and the march takes 1.6 ms.
 bool ku64_split(const Dims& d, int sms, int march_ox, int march_oy, int march_warps) {

@@ -458,7 +458,10 @@ constexpr int GJ_B = 16, GJ_T = 32, GJ_NT = 256;
 
 __device__ __forceinline__ double gj_recip(double a) {
     // the FP32 reciprocal refined by two Newton steps (each doubles the correct bits): a chain of
-    // four FP64 operations, where a division is several times longer on this part's FP64 pipe
+    // four FP64 operations, where a division is several times longer on this part's FP64 pipe. After the
+    // first step the remainder 1 - a r is below 2^-45, so the second is off by its own rounding alone
+    // (2e8 random a: always the rounded quotient). Pivots are not so small that (float)a loses bits:
+    // they are at least 1e-12 of the largest diagonal entry, which is 1 or more with a fixed unknown.
     const float r0 = 1.f / (float)a;
     if (!(r0 > 0.f && r0 < INFINITY)) return 1.0 / a;
     double r = r0;

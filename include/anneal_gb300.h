@@ -32,7 +32,8 @@ enum {
     ANL_ERR_CUDA = 5,
     ANL_ERR_SINGULAR = 6, /* reserved (tiny coarse-grid pivots are regularised, not reported) */
     ANL_ERR_NOMEM = 7,
-    ANL_ERR_STATE = 8, /* a call that needs anl_set_domain / anl_filter_init came first */
+    ANL_ERR_STATE = 8, /* a call that needs anl_set_domain / anl_filter_init came first, or an OC
+                          multiplier search that did not end */
     ANL_ERR_STAGNATION = 9 /* an FP32 solve stopped improving above rtol: finish it in FP64 */
 };
 
